@@ -154,7 +154,7 @@ int sbwt_search_reads(const sbwt_index_t *index, const char *chars,
  *     is implied); the caller allocates inputs and outputs.  n_results (host,
  *     may be NULL) receives the k-mer count; the call returns when the results
  *     are written (it synchronizes `stream`).
- *   - Scratch is one fixed array of about 9 MiB in the library's device
+ *   - Scratch is one fixed array of about 11 MiB in the library's device
  *     memory, present on every GPU that loads the library until the process
  *     exits.  At most 8 Mi chars (8388608) and 256 Ki reads (262144) per call;
  *     larger calls fail with SBWT_E_INVALID.

@@ -199,8 +199,7 @@ int sbwt_index_set_kmer_table(sbwt_index_t *index, int enable, uint64_t *table_b
     } else if (!x.view.kmer_table) {
       x.build_kmer_table();
     }
-    x.device_bytes = x.presearch.size() + x.hot.size() + x.key_buf.size() + x.l0_all.size() +
-                     x.kmer_table.size() + x.kmer_filter.size();
+    x.device_bytes = x.held_bytes();
     if (table_bytes) *table_bytes = x.kmer_table.size();
   });
 }

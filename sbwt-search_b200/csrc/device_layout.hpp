@@ -34,6 +34,15 @@ struct Block {
   unsigned long long w0, w1, w2, w3;
 };
 
+// 32 positions of the path cover (path_cover.cu): their chars (2 bits, first
+// on top), break bits (bit i: position i does not follow position i - 1) and
+// branch bits (bit i: the k-mer at position i - 1 has another edge); or 32
+// chars of a read batch and their invalid bits (in brk).
+struct alignas(16) PathEntry {
+  unsigned long long chars;
+  uint32_t brk, branch;
+};
+
 // Device view of the SBWT used by the search kernels.
 struct SbwtView {
   const Block *blocks[4];
@@ -52,6 +61,14 @@ struct SbwtView {
   uint64_t kmer_table_mask;    // slots - 1
   const uint64_t *kmer_filter; // blocked Bloom filter of the table's keys, or nullptr
   uint64_t filter_words;       // 64-bit words of kmer_filter
+  // the value of a table slot is the node, with the k-mer's position in the
+  // path cover in its high half when there is one (node_mask: the node's bits)
+  uint64_t node_mask;
+  const uint32_t *path_node;    // node at each position of the path cover, or nullptr
+  const PathEntry *path_entry;  // chars and breaks of the positions
+  const uint64_t *lmer_filter;  // Bloom filter of the k-mers' L-mers, or nullptr
+  uint32_t lmer_words;          // 64-bit words of lmer_filter
+  uint32_t lmer_len;            // L (0: no filter)
   uint64_t num_bits;
   uint32_t k;
   uint32_t p;      // presearch depth used by this call

@@ -169,6 +169,53 @@ __global__ void pack16_kernel(const char *__restrict__ chars, uint64_t n,
   }
 }
 
+// Packing into interleaved entries (32 chars and their invalid bits in 16
+// bytes; two empty entries past the end).  A lane packs 16 consecutive chars
+// and stores half an entry, so loads and stores are whole lines: 2-bit codes
+// and bits of 16 chars come from one 16-byte load.  ALIGNED: chars are 16-byte
+// aligned, else they are read byte by byte.
+template <bool ALIGNED>
+__global__ void pack_entries_kernel(const char *__restrict__ chars, uint64_t n,
+                                    uint2 *__restrict__ halves, uint64_t n_words) {
+  const uint64_t step = (uint64_t)gridDim.x * blockDim.x, n_half = 2 * (n_words + 2);
+  constexpr int U = 4;  // loads in flight per thread
+  for (uint64_t h0 = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; h0 < ((n_half + 31) & ~31ULL);
+       h0 += U * step) {
+    uint4 x[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const uint64_t h = h0 + u * step, i0 = 16 * h;
+      x[u] = make_uint4(0x41414141u, 0x41414141u, 0x41414141u, 0x41414141u);  // past n: 'A'
+      if (ALIGNED && i0 + 16 <= n) {
+        x[u] = __ldcs(reinterpret_cast<const uint4 *>(chars + i0));
+      } else if (i0 < n) {
+        uint32_t *w = &x[u].x;
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+          if (i0 + i < n)
+            w[i >> 2] = (w[i >> 2] & ~(0xFFu << (8 * (i & 3)))) |
+                        (uint32_t)(uint8_t)chars[i0 + i] << (8 * (i & 3));
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const uint64_t h = h0 + u * step;
+      uint32_t c[4], b[4];
+      pack_4chars(x[u].x, c[0], b[0]);
+      pack_4chars(x[u].y, c[1], b[1]);
+      pack_4chars(x[u].z, c[2], b[2]);
+      pack_4chars(x[u].w, c[3], b[3]);
+      const uint32_t codes = c[0] << 24 | c[1] << 16 | c[2] << 8 | c[3];
+      const uint32_t bits = b[0] | b[1] << 4 | b[2] << 8 | b[3] << 12;
+      // even lane: the entry's 64 code bits; odd lane: its 32 invalid bits
+      const uint32_t codes2 = __shfl_xor_sync(0xFFFFFFFFu, codes, 1);
+      const uint32_t bits2 = __shfl_xor_sync(0xFFFFFFFFu, bits, 1);
+      if (h < n_half)
+        halves[h] = h & 1 ? make_uint2(bits2 | bits << 16, 0) : make_uint2(codes2, codes);
+    }
+  }
+}
+
 // --- exclusive scan of per-read k-mer counts -> kmer_off[0..n_reads] ---------
 constexpr int kScanThreads = 256;
 constexpr int kScanItems = 16;
@@ -400,6 +447,7 @@ __global__ void __launch_bounds__(256) search_positions_kernel(
 struct ReadsView {
   const uint64_t *packed;   // chunk chars, 2-bit packed (+1 pad word)
   const uint32_t *invalid;  // invalid-char bits, 32 per word
+  const PathEntry *entries; // both interleaved (+2 pad entries), for search_paths_kernel
   const uint64_t *ends;     // exclusive read ends (absolute)
   const uint64_t *kmer_off; // n_reads + 1
   uint64_t base;            // absolute char offset of chunk char 0
@@ -466,13 +514,35 @@ __global__ void ends_upper_bound_kernel(const uint64_t *ends, uint64_t r0, uint6
 }
 
 // First read of every work tile: tile_read[t] = the read holding k-mer slot
-// t * tile.  One thread per read; reads without k-mers own no tile.
-__global__ void tile_reads_kernel(const uint64_t *kmer_off, uint64_t n_reads, uint64_t tile,
+// t * tile, with the char of that k-mer in the high half when with_pos.  One
+// thread per read (a read of more than a few tiles is shared by its warp);
+// reads without k-mers own no tile.
+__global__ void tile_reads_kernel(const uint64_t *kmer_off, const uint64_t *ends, uint64_t base,
+                                  uint64_t n_reads, uint64_t tile, uint32_t with_pos,
                                   uint64_t *tile_read) {
-  for (uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; r < n_reads;
-       r += (uint64_t)gridDim.x * blockDim.x) {
-    const uint64_t a = kmer_off[r], b = kmer_off[r + 1];
-    for (uint64_t t = (a + tile - 1) / tile; t * tile < b; ++t) tile_read[t] = r;
+  const uint32_t lane = threadIdx.x & 31;
+  const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
+  for (uint64_t r0 = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) & ~31ULL; r0 < n_reads;
+       r0 += step) {
+    const uint64_t r = r0 + lane;
+    uint64_t t = 0, t_end = 0, entry = 0;
+    if (r < n_reads) {
+      const uint64_t a = kmer_off[r], b = kmer_off[r + 1];
+      t = (a + tile - 1) / tile;
+      t_end = (b + tile - 1) / tile;
+      entry = r;
+      if (with_pos && t < t_end)  // the char at slot 0, modulo 2^32
+        entry |= ((r ? ends[r - 1] : base) - base - a) << 32;
+    }
+    const uint64_t up = with_pos ? tile << 32 : 0;
+    for (uint32_t i = 0; i < 32 && t < t_end; ++i, ++t) tile_read[t] = entry + t * up;
+    for (unsigned m = __ballot_sync(0xFFFFFFFFu, t < t_end); m; m &= m - 1) {
+      const int q = __ffs(m) - 1;
+      const uint64_t q_end = __shfl_sync(0xFFFFFFFFu, t_end, q);
+      const uint64_t q_entry = __shfl_sync(0xFFFFFFFFu, entry, q);
+      for (uint64_t x = __shfl_sync(0xFFFFFFFFu, t, q) + lane; x < q_end; x += 32)
+        tile_read[x] = q_entry + x * up;
+    }
   }
 }
 
@@ -939,10 +1009,10 @@ __global__ void __launch_bounds__(256, SBWT_SEARCH_MIN_BLOCKS)
     } else if (kind == K_HASH) {  // slots u, u + 1: (key, node) each
       const uint64_t key = SMALLK ? cw.prefix(pos, k) : 0;
       if (A.w0 == key) {
-        emit = (I)A.w1;
+        emit = (I)(A.w1 & s.node_mask);
         emitted = true;
       } else if (A.w2 == key) {
-        emit = (I)A.w3;
+        emit = (I)(A.w3 & s.node_mask);
         emitted = true;
       } else if (A.w0 == ~0ULL || A.w2 == ~0ULL) {  // an empty slot: absent
         emit = NONE;
@@ -1284,6 +1354,12 @@ __device__ __forceinline__ uint64_t load_u64_nc(const uint64_t *p) {
   return v;
 }
 
+__device__ __forceinline__ uint32_t load_u32_nc(const uint32_t *p) {
+  uint32_t v;
+  asm("ld.global.nc.L1::no_allocate.u32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
+
 // load_u64_nc with an L2 eviction policy.
 __device__ __forceinline__ uint64_t load_u64_hint(const uint64_t *p, uint64_t policy) {
   uint64_t v;
@@ -1291,6 +1367,11 @@ __device__ __forceinline__ uint64_t load_u64_hint(const uint64_t *p, uint64_t po
       : "=l"(v)
       : "l"(p), "l"(policy));
   return v;
+}
+
+__device__ __forceinline__ uint2 load_uint2_hint(const uint64_t *p, uint64_t policy) {
+  const uint64_t v = load_u64_hint(p, policy);
+  return make_uint2((uint32_t)v, (uint32_t)(v >> 32));
 }
 
 __device__ __forceinline__ void store_u32x4_cs(uint32_t *p, uint32_t a, uint32_t b,
@@ -1925,10 +2006,10 @@ __global__ void __launch_bounds__(256)
         if (!look[t]) continue;
         if (COUNT) ++n_table;
         if (A[t].w0 == key[t]) {
-          res[t] = A[t].w1;
+          res[t] = (uint32_t)A[t].w1;
           look[t] = false;
         } else if (A[t].w2 == key[t]) {
-          res[t] = A[t].w3;
+          res[t] = (uint32_t)A[t].w3;
           look[t] = false;
         } else if (A[t].w0 == ~0ULL || A[t].w2 == ~0ULL) {
           look[t] = false;  // an empty slot: absent
@@ -1954,6 +2035,10 @@ __global__ void __launch_bounds__(256)
     atomicAdd(counters + 12, (unsigned long long)n_table);   // table lookups
   }
 }
+
+}  // namespace sbwt
+#include "search_paths.cuh"
+namespace sbwt {
 
 template <int PER, bool COUNT>
 __global__ void __launch_bounds__(256)
@@ -2130,10 +2215,10 @@ __global__ void __launch_bounds__(256)
         if (!look[t]) continue;
         if (COUNT) ++n_table;
         if (A[t].w0 == key[t]) {
-          res[t] = A[t].w1;
+          res[t] = (uint32_t)A[t].w1;
           look[t] = false;
         } else if (A[t].w2 == key[t]) {
-          res[t] = A[t].w3;
+          res[t] = (uint32_t)A[t].w3;
           look[t] = false;
         } else if (A[t].w0 == ~0ULL || A[t].w2 == ~0ULL) {
           look[t] = false;  // an empty slot: absent
@@ -2274,8 +2359,12 @@ static bool walks_kernel_applies(const SbwtView &sv, const ReadsView &rv, bool s
          sv.k <= 31 && mtk == 0 && sv.suffix_group_starts;
 }
 
+// Mode 7 (automatic, the default) runs search_paths_kernel on an index with a
+// path cover (every narrow index with suffix groups whose cover fits the
+// device: it is faster than the two below at every size measured, see its
+// comment), else the k-mers kernel or the walks kernel.
 // The k-mers kernel (modes 6, 11) has the walks kernel's conditions.  Mode 7
-// (automatic, the default) picks it, with 2 k-mers per lane (mode 11: 51
+// picks it (without a cover), with 2 k-mers per lane (mode 11: 51
 // registers, 5 blocks per SM; faster than 4 per lane at 3 blocks), when the
 // table and filter fit kKmersKernelMaxBytes (they then stay in L2 and inside
 // the translation reach, and independent lookups beat the chained stream
@@ -2287,8 +2376,10 @@ static bool walks_kernel_applies(const SbwtView &sv, const ReadsView &rv, bool s
 // kernel's 8-byte stores).  Where the walks kernel does not apply, mode 17
 // runs the table kernel.
 constexpr u64 kKmersKernelMaxBytes = 256ULL << 20;
+constexpr uint32_t kPathsKernel = 100;  // what mode 7 resolves to, not a mode of its own
 static uint32_t resolve_kernel_mode(const SbwtView &sv, uint32_t kernel_mode) {
   if (kernel_mode != 7) return kernel_mode;
+  if (sv.path_node) return kPathsKernel;
   const u64 bytes = (sv.kmer_table_mask + 1) * 16 + sv.filter_words * 8;
   return sv.kmer_table && sv.kmer_filter && bytes <= kKmersKernelMaxBytes ? 11u : 17u;
 }
@@ -2373,7 +2464,20 @@ static void launch_search_kernel(bool stream, const SbwtView &sv, const ReadsVie
       launch_ex(search_walks_kernel<W_, B_, false>, grid, threads, st, la, sv, rv, tile_read, \
                 ctr);                                                                      \
   } while (0)
-    if (kernel_mode == 2) SBWT_WALKS(1, 5);
+#define SBWT_PATHS(C_, K_, O_)                                                           \
+  launch_one_wave(search_paths_kernel<C_, K_, O_>, grid, threads, st, la, sv, rv, tile_read, \
+                  ctr)
+#define SBWT_PATHS_K(C_, K_)      \
+  do {                            \
+    if (rv.out32)                 \
+      SBWT_PATHS(C_, K_, true);   \
+    else                          \
+      SBWT_PATHS(C_, K_, false);  \
+  } while (0)
+    if (kernel_mode == kPathsKernel && ctr) SBWT_PATHS_K(true, 0);
+    else if (kernel_mode == kPathsKernel && sv.k == 31) SBWT_PATHS_K(false, 31);
+    else if (kernel_mode == kPathsKernel) SBWT_PATHS_K(false, 0);
+    else if (kernel_mode == 2) SBWT_WALKS(1, 5);
     else if (kernel_mode == 3) SBWT_WALKS(2, 4);
     else if (kernel_mode == 4) SBWT_WALKS(2, 3);
     else if (kernel_mode == 5) SBWT_WALKS(4, 2);
@@ -2427,6 +2531,8 @@ static void launch_search_kernel(bool stream, const SbwtView &sv, const ReadsVie
     else
       launch_one_wave(search_kmers_kernel<4, false>,
                       grid, threads, st, la, sv, rv, tile_read, ctr);
+#undef SBWT_PATHS
+#undef SBWT_PATHS_K
 #undef SBWT_WALKS
 #undef SBWT_LEAN
 #undef SBWT_LEANS
@@ -2614,8 +2720,7 @@ IndexImpl::IndexImpl(const u64 *const acgt[4], u64 num_bits_, u32 k_,
   }
   SBWT_CUDA(cudaDeviceSynchronize());
   build_kmer_table();
-  device_bytes = presearch.size() + hot.size() + key_buf.size() + l0_all.size() +
-                 kmer_table.size() + kmer_filter.size();
+  device_bytes = held_bytes();
 }
 
 SbwtView IndexImpl::view_for(u32 p) const {
@@ -2750,8 +2855,30 @@ static uint32_t probe_length(u64 num_bits, u32 k, const LaunchConfig &cfg) {
   return L < k ? L : 0;
 }
 
-static u64 tile_size(int device, u64 n_kmers, const LaunchConfig &cfg) {
+// More than every chunk position, slot and read number of a batch.
+static u64 reads_bound(u64 n_chars, u64 n_reads) { return std::max<u64>(n_chars, n_reads) + 64; }
+
+// Whether a read search of this index runs search_paths_kernel.
+static bool paths_kernel_applies(const IndexImpl &ix, u64 n_kmers_bound, u32 flags,
+                                 const LaunchConfig &cfg) {
+  ReadsView rv{};
+  rv.n_kmers_bound = n_kmers_bound;
+  const bool stream = !(flags & SBWT_PER_KMER_WALK) && ix.view.suffix_group_starts;
+  const u32 mtk = (flags & SBWT_MOVE_TO_KEY_KMER) ? 1u : 0u;
+  return resolve_kernel_mode(ix.view, cfg.table_kernel) == kPathsKernel &&
+         walks_kernel_applies(ix.view, rv, stream, mtk, kPathsKernel);
+}
+
+// paths: for search_paths_kernel, where a tile costs its lane a table lookup
+// at its start: four tiles per resident lane, at most 64 slots.  Kernel time
+// with tiles of 16 / 32 / 64 / 128 slots: 63 / 74 / 90 / 124 us on 2.4 M
+// k-mers, - / 92 / 95 / 96 us on 12 M, - / 2.93 / 2.83 / 2.97 ms on 420 M.
+static u64 tile_size(int device, u64 n_kmers, const LaunchConfig &cfg, bool paths) {
   if (cfg.tile) return cfg.tile;
+  if (paths) {
+    const u64 tile = n_kmers / ((u64)sm_count(device) * 4096);
+    return (std::min<u64>(std::max<u64>(tile, 16), 64) + 15) & ~15ULL;
+  }
   const u64 resident = (u64)sm_count(device) * cfg.blocks_per_sm * cfg.block_threads;
   u64 tile = n_kmers / (resident * 8);
   // at most 128 slots: the tiles in flight then span less of the chars and
@@ -2763,9 +2890,10 @@ static u64 tile_size(int device, u64 n_kmers, const LaunchConfig &cfg) {
 
 // Scan of per-read k-mer counts and the packing of the chars (device-resident
 // inputs).  The k-mer total lands in *sc.total.
+// entries: packed as interleaved entries, for search_paths_kernel.
 static void launch_prepare(int device, u32 k, const char *d_chars, u64 n_chars,
                            const u64 *d_ends, u64 n_reads, u64 base,
-                           const ReadsScratch &sc, cudaStream_t st) {
+                           const ReadsScratch &sc, bool entries, cudaStream_t st) {
   const u64 n_words = (n_chars + 31) / 32;
   const u64 n_scan_blocks = (n_reads + kScanTile - 1) / kScanTile;
   scan_reduce_kernel<<<(unsigned)n_scan_blocks, kScanThreads, 0, st>>>(
@@ -2774,6 +2902,18 @@ static void launch_prepare(int device, u32 k, const char *d_chars, u64 n_chars,
                                                sc.err);
   scan_write_kernel<<<(unsigned)n_scan_blocks, kScanThreads, 0, st>>>(
       d_ends, n_reads, base, k, sc.block_sums, sc.kmer_off, sc.err);
+  if (entries) {
+    const int grid = grid_for(device, (2 * (n_words + 2) + 3) / 4, 256, 8);
+    if (((uintptr_t)d_chars & 15) == 0)
+      pack_entries_kernel<true><<<grid, 256, 0, st>>>(
+          d_chars, n_chars, reinterpret_cast<uint2 *>(sc.packed), n_words);
+    else
+      pack_entries_kernel<false><<<grid, 256, 0, st>>>(
+          d_chars, n_chars, reinterpret_cast<uint2 *>(sc.packed), n_words);
+    SBWT_CUDA(cudaGetLastError());
+    note_launches(4);
+    return;
+  }
   SBWT_CUDA(cudaMemsetAsync(sc.packed + n_words, 0, 16, st));
   SBWT_CUDA(cudaMemsetAsync(sc.invalid + n_words, 0, 8, st));
   if (n_words && ((uintptr_t)d_chars & 15) == 0)
@@ -2798,15 +2938,17 @@ static void launch_search(const IndexImpl &ix, u64 n_chars, const u64 *d_ends, u
   if (n_reads == 0 || n_kmers == 0) return;
   ReadsView rv{};
   rv.out32 = d_out32;
-  rv.n_kmers_bound = std::max<u64>(n_chars, n_reads) + 64;
+  rv.n_kmers_bound = reads_bound(n_chars, n_reads);
   rv.packed = sc.packed;
+  rv.entries = reinterpret_cast<const PathEntry *>(sc.packed);
   rv.invalid = sc.invalid;
   rv.ends = d_ends;
   rv.kmer_off = sc.kmer_off;
   rv.base = base;
   rv.n_reads = n_reads;
   rv.n_kmers = n_kmers;
-  rv.tile = tile_size(ix.device, n_kmers, cfg);
+  const bool paths = paths_kernel_applies(ix, rv.n_kmers_bound, flags, cfg);
+  rv.tile = tile_size(ix.device, n_kmers, cfg, paths);
   rv.n_tiles = (n_kmers + rv.tile - 1) / rv.tile;
   rv.out = d_out;
   rv.out_capacity = out_capacity;
@@ -2815,7 +2957,7 @@ static void launch_search(const IndexImpl &ix, u64 n_chars, const u64 *d_ends, u
   rv.queue = sc.queue;
   SBWT_CUDA(cudaMemsetAsync(sc.queue, 0, 8, st));
   tile_reads_kernel<<<grid_for(ix.device, n_reads, 256, 16), 256, 0, st>>>(
-      sc.kmer_off, n_reads, rv.tile, sc.tile_read);
+      sc.kmer_off, d_ends, rv.base, n_reads, rv.tile, paths, sc.tile_read);
   SBWT_CUDA(cudaGetLastError());
   note_launches(1);
   const int threads = (int)cfg.block_threads;
@@ -2856,10 +2998,13 @@ void enqueue_index_step(const IndexImpl &ix, const char *d_chars, u64 n_chars,
     SBWT_CUDA(cudaMemsetAsync(sc.total, 0, 8, st));
     return;
   }
-  launch_prepare(ix.device, ix.k, d_chars, n_chars, d_ends, n_reads, 0, sc, st);
+  const u64 bound = reads_bound(n_chars, n_reads);
+  const bool paths = paths_kernel_applies(ix, bound, flags, cfg);
+  launch_prepare(ix.device, ix.k, d_chars, n_chars, d_ends, n_reads, 0, sc, paths, st);
   ReadsView rv{};
-  rv.n_kmers_bound = std::max<u64>(n_chars, n_reads) + 64;
+  rv.n_kmers_bound = bound;
   rv.packed = sc.packed;
+  rv.entries = reinterpret_cast<const PathEntry *>(sc.packed);
   rv.invalid = sc.invalid;
   rv.ends = d_ends;
   rv.kmer_off = sc.kmer_off;
@@ -2867,14 +3012,14 @@ void enqueue_index_step(const IndexImpl &ix, const char *d_chars, u64 n_chars,
   rv.n_reads = n_reads;
   rv.n_kmers = 0;
   rv.n_kmers_dev = sc.total;
-  rv.tile = tile_size(ix.device, std::max<u64>(max_kmers, 1), cfg);
+  rv.tile = tile_size(ix.device, std::max<u64>(max_kmers, 1), cfg, paths);
   rv.n_tiles = 0;  // computed on the device from the total
   rv.out = d_out;
   rv.out_capacity = out_capacity;
   rv.probe_len = probe_length(ix.num_bits, ix.k, cfg);
   rv.queue = sc.queue;
   tile_reads_kernel<<<grid_for(ix.device, n_reads, 256, 16), 256, 0, st>>>(
-      sc.kmer_off, n_reads, rv.tile, sc.tile_read);
+      sc.kmer_off, d_ends, rv.base, n_reads, rv.tile, paths, sc.tile_read);
   const int grid = (int)((u64)sm_count(ix.device) * cfg.blocks_per_sm);
   const SbwtView sv = ix.view_for(cfg.presearch_letters);
   const bool stream = !(flags & SBWT_PER_KMER_WALK) && ix.view.suffix_group_starts;
@@ -2884,16 +3029,22 @@ void enqueue_index_step(const IndexImpl &ix, const char *d_chars, u64 n_chars,
   note_launches(1);
 }
 
+// Smallest tile any search of such a batch uses (the tile table's size).
 u64 index_tile_size(const IndexImpl &ix, u64 max_kmers, const LaunchConfig &cfg) {
-  return tile_size(ix.device, std::max<u64>(max_kmers, 1), cfg);
+  return std::min(tile_size(ix.device, std::max<u64>(max_kmers, 1), cfg, false),
+                  tile_size(ix.device, std::max<u64>(max_kmers, 1), cfg, true));
 }
+
+// Smallest tile a launch may use: what a tile table sized before the k-mer
+// count is known has to hold.
+static u64 tile_min(const LaunchConfig &cfg) { return cfg.tile ? std::min<u64>(cfg.tile, 16) : 16; }
 
 // Grows the workspace buffers of slot b for a batch and returns raw pointers.
 static ReadsScratch scratch_for(Workspace &ws, int b, u64 n_chars, u64 n_reads,
                                 u64 n_kmers_max, u64 tile_min) {
   const u64 n_words = (n_chars + 31) / 32;
   ws.kmer_off[b].ensure((n_reads + 1) * 8);
-  ws.packed[b].ensure((n_words + 2) * 8);
+  ws.packed[b].ensure((n_words + 2) * 16);  // words, or interleaved entries
   ws.invalid[b].ensure((n_words + 2) * 4);
   ws.block_sums[b].ensure(((n_reads + kScanTile - 1) / kScanTile + 1) * 8);
   ws.total[b].ensure(8);
@@ -2943,8 +3094,9 @@ void IndexImpl::search_reads_device_pieces(const char *chars, u64 n_chars,
     if (c1 < c0 || c1 > n_chars)
       throw Error(SBWT_E_INVALID, "read_ends are not non-decreasing within n_chars");
     const u64 nc = c1 - c0, nr = r1 - r0;
-    const ReadsScratch sc = scratch_for(ws, 0, nc, nr, nc, 16);
-    launch_prepare(device, k, chars + c0, nc, read_ends + r0, nr, c0, sc, st);
+    const ReadsScratch sc = scratch_for(ws, 0, nc, nr, nc, tile_min(cfg));
+    launch_prepare(device, k, chars + c0, nc, read_ends + r0, nr, c0, sc,
+                   paths_kernel_applies(*this, reads_bound(nc, nr), flags, cfg), st);
     u64 n_k = 0;
     SBWT_CUDA(cudaMemcpyAsync(&n_k, sc.total, 8, cudaMemcpyDeviceToHost, st));
     SBWT_CUDA(cudaStreamSynchronize(st));
@@ -2993,13 +3145,15 @@ void IndexImpl::search_reads(const char *chars, u64 n_chars, const u64 *read_end
     u64 n_k = 0;
     if (n_reads) {
       // k-mers <= chars, so a tile table sized for n_chars is always enough
-      const ReadsScratch sc = scratch_for(ws, 0, n_chars, n_reads, n_chars, 16);
+      const ReadsScratch sc = scratch_for(ws, 0, n_chars, n_reads, n_chars, tile_min(cfg));
       // scan, packing, tile table and search queued back to back: the search
       // reads the k-mer count from the scan's total (a batch with bad read
       // ends has a total of 0), tiles are sized for n_chars (>= the count),
       // and no kernel writes at or past `capacity`.  The count and the error
       // word come back under one synchronisation (check_err_word's).
-      launch_prepare(device, k, chars, n_chars, read_ends, n_reads, 0, sc, user_stream);
+      launch_prepare(device, k, chars, n_chars, read_ends, n_reads, 0, sc,
+                     paths_kernel_applies(*this, reads_bound(n_chars, n_reads), flags, cfg),
+                     user_stream);
       launch_search(*this, n_chars, read_ends, n_reads, 0, n_chars, results, capacity, flags,
                     cfg, sc, user_stream, nullptr, sc.total);
       u64 *const total_host = reinterpret_cast<u64 *>(ws.err_host + 2);
@@ -3063,7 +3217,7 @@ void IndexImpl::search_reads(const char *chars, u64 n_chars, const u64 *read_end
     cudaStream_t st = ws.streams[b];
     const u64 nc = prev - c0, nr = r1 - r0;
     ReadsView probe{};
-    probe.n_kmers_bound = std::max<u64>(nc, nr) + 64;
+    probe.n_kmers_bound = reads_bound(nc, nr);
     const bool narrow = !pinned && walks_kernel_applies(sv_host, probe, stream_host, mtk_host,
                                                         resolve_kernel_mode(sv_host,
                                                                             cfg.table_kernel));
@@ -3073,12 +3227,12 @@ void IndexImpl::search_reads(const char *chars, u64 n_chars, const u64 *read_end
       ws.results32[b].ensure(std::max<u64>(nk, 1) * 4);
     else
       ws.results[b].ensure(std::max<u64>(nk, 1) * 8);
-    const ReadsScratch sc = scratch_for(ws, b, nc, nr, nk, tile_size(device, nk, cfg));
+    const ReadsScratch sc = scratch_for(ws, b, nc, nr, nk, index_tile_size(*this, nk, cfg));
     SBWT_CUDA(cudaMemcpyAsync(ws.chars[b].get(), chars + c0, nc, cudaMemcpyHostToDevice, st));
     SBWT_CUDA(cudaMemcpyAsync(ws.ends[b].get(), read_ends + r0, nr * 8,
                               cudaMemcpyHostToDevice, st));
     launch_prepare(device, k, ws.chars[b].get<char>(), nc, ws.ends[b].get<u64>(), nr, c0, sc,
-                   st);
+                   paths_kernel_applies(*this, reads_bound(nc, nr), flags, cfg), st);
     if (narrow) {
       uint32_t *stage = ws.staging(b, std::max<u64>(nk, 1));
       launch_search(*this, nc, ws.ends[b].get<u64>(), nr, c0, nk, nullptr, nk, flags, cfg, sc,
@@ -3165,15 +3319,15 @@ void IndexImpl::search_positions(const u64 *bit_seqs, u64 n_words, const u64 *po
 // table, search kernel) with all its scratch in this fixed device array.
 //
 // Limits: at most kNoAllocMaxChars chars and kNoAllocMaxReads reads per call.
-// The array (about 9 MiB) lives on every GPU that loads this library until
+// The array (about 11 MiB) lives on every GPU that loads this library until
 // the process exits.  All calls share it, so calls that overlap on the GPU
 // (from several host threads or streams) race: serialize them.
 constexpr u64 kNoAllocMaxChars = 8ULL << 20;
 constexpr u64 kNoAllocMaxReads = 1ULL << 18;
 constexpr u64 kNoAllocWords = kNoAllocMaxChars / 32;
 constexpr u64 kNoAllocOffKmerOff = 0;
-constexpr u64 kNoAllocOffPacked = kNoAllocOffKmerOff + (kNoAllocMaxReads + 1) * 8;
-constexpr u64 kNoAllocOffInvalid = kNoAllocOffPacked + (kNoAllocWords + 2) * 8;
+constexpr u64 kNoAllocOffPacked = ((kNoAllocOffKmerOff + (kNoAllocMaxReads + 1) * 8 + 255) / 256) * 256;
+constexpr u64 kNoAllocOffInvalid = kNoAllocOffPacked + (kNoAllocWords + 2) * 16;
 constexpr u64 kNoAllocOffBlockSums =
     ((kNoAllocOffInvalid + (kNoAllocWords + 2) * 4 + 255) / 256) * 256;
 constexpr u64 kNoAllocOffTotal =
@@ -3244,10 +3398,11 @@ void IndexImpl::search_reads_noalloc(const char *d_chars, u64 n_chars, const u64
   // clear them first
   SBWT_CUDA(cudaMemsetAsync(sc.err, 0, 4, st));
   SBWT_CUDA(cudaMemsetAsync(sc.queue, 0, 8, st));
+  const bool paths = paths_kernel_applies(*this, reads_bound(n_chars, n_reads), flags, cfg_in);
   u64 n_k = 0;
   uint32_t err = 0;
   if (n_reads) {
-    launch_prepare(device, k, d_chars, n_chars, d_ends, n_reads, 0, sc, st);
+    launch_prepare(device, k, d_chars, n_chars, d_ends, n_reads, 0, sc, paths, st);
     SBWT_CUDA(cudaMemcpyAsync(&n_k, sc.total, 8, cudaMemcpyDeviceToHost, st));
     SBWT_CUDA(cudaMemcpyAsync(&err, sc.err, 4, cudaMemcpyDeviceToHost, st));
     SBWT_CUDA(cudaStreamSynchronize(st));
@@ -3260,22 +3415,23 @@ void IndexImpl::search_reads_noalloc(const char *d_chars, u64 n_chars, const u64
   LaunchConfig cfg = cfg_in;  // the tile table is sized for tiles of >= 16
   if (cfg.tile && cfg.tile < kNoAllocTileMin) cfg.tile = kNoAllocTileMin;
   ReadsView rv{};
-  rv.n_kmers_bound = std::max<u64>(n_chars, n_reads) + 64;
+  rv.n_kmers_bound = reads_bound(n_chars, n_reads);
   rv.packed = sc.packed;
+  rv.entries = reinterpret_cast<const PathEntry *>(sc.packed);
   rv.invalid = sc.invalid;
   rv.ends = d_ends;
   rv.kmer_off = sc.kmer_off;
   rv.base = 0;
   rv.n_reads = n_reads;
   rv.n_kmers = n_k;
-  rv.tile = tile_size(device, n_k, cfg);
+  rv.tile = tile_size(device, n_k, cfg, paths);
   rv.n_tiles = (n_k + rv.tile - 1) / rv.tile;
   rv.out = d_results;
   rv.out_capacity = capacity;
   rv.probe_len = probe_length(num_bits, k, cfg);
   rv.queue = sc.queue;
-  tile_reads_kernel<<<grid_for(device, n_reads, 256, 16), 256, 0, st>>>(sc.kmer_off, n_reads,
-                                                                        rv.tile, sc.tile_read);
+  tile_reads_kernel<<<grid_for(device, n_reads, 256, 16), 256, 0, st>>>(
+      sc.kmer_off, d_ends, 0, n_reads, rv.tile, paths, sc.tile_read);
   const int grid = grid_for(device, rv.n_tiles, (int)cfg.block_threads, cfg.blocks_per_sm);
   const SbwtView sv = view_for(cfg.presearch_letters);
   const u32 mtk = (flags & SBWT_MOVE_TO_KEY_KMER) ? 1u : 0u;

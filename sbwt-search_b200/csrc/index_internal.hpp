@@ -16,6 +16,9 @@ constexpr uint32_t kPresearchMaxLetters = 14;
 constexpr u64 kKmerTableMaxBytes = 32ULL << 30;
 // Bits per k-mer of the k-mer filter built with the table.
 constexpr u64 kFilterBitsPerKmer = 10;
+// Bits per k-mer of the L-mer filter built with the path cover (about one
+// distinct L-mer per k-mer: 2.5 % false positives).
+constexpr u64 kLmerFilterBits = 8;
 
 // Read search kernel of an index with a k-mer table by default
 // (LaunchConfig::table_kernel): automatic (the k-mers kernel for small
@@ -44,6 +47,13 @@ struct IndexImpl {
   // built
   bool build_kmer_table();
   void drop_kmer_table();
+  // path cover and L-mer filter of a table under construction
+  bool build_path_cover(const u64 *key, const u8 *alive, u64 n_kmers, DeviceBuffer &pos);
+  void drop_path_cover();
+  u64 held_bytes() const {  // device memory of the handle
+    return presearch.size() + hot.size() + key_buf.size() + l0_all.size() + kmer_table.size() +
+           kmer_filter.size() + path_nodes.size() + path_entries.size() + lmer_filter.size();
+  }
 
   void search_positions(const u64 *bit_seqs, u64 n_words, const u64 *positions,
                         u64 n, u64 *results, u32 flags, cudaStream_t st,
@@ -76,6 +86,7 @@ struct IndexImpl {
   SbwtView view{};
   DeviceBuffer hot;  // rank blocks of A/C/G/T + suffix-group words, contiguous
   DeviceBuffer l0_all, presearch, key_buf, kmer_table, kmer_filter;
+  DeviceBuffer path_nodes, path_entries, lmer_filter;
   u64 table_kmers = 0;
   u64 window_bytes = 0;   // L2 access-policy window over `hot`
 };

@@ -15,8 +15,10 @@
 // over all nodes spell every label; a node whose chain reaches the root
 // within k chars is a dummy ($-padded) and is not a k-mer.
 //
-// Table: 2^m slots of 16 bytes (key, node), key = the k chars with the first
-// char on top (2 bits each), empty = ~0; a key's probe sequence starts at an
+// Table: 2^m slots of 16 bytes (key, value), value = the node, with the k-mer's
+// position in the path cover (path_cover.cu) in the high half when the index
+// has one; key = the k chars with the first char on top (2 bits each), empty
+// = ~0; a key's probe sequence starts at an
 // even slot (so a 32-byte sector holds the first two slots it probes) and
 // moves one slot at a time; at most half of the slots are used.
 //
@@ -103,8 +105,11 @@ __global__ void count_alive_kernel(const uint8_t *alive, uint64_t n, unsigned lo
   if ((threadIdx.x & 31) == 0 && c) atomicAdd(out, c);
 }
 
+// pos: the k-mers' positions in the path cover (the high half of a slot's
+// value), or nullptr.
 __global__ void table_insert_kernel(const uint64_t *key, const uint8_t *alive, uint64_t n,
-                                    uint64_t *table, uint64_t mask, uint32_t *err) {
+                                    const uint32_t *pos, uint64_t *table, uint64_t mask,
+                                    uint32_t *err) {
   const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < n; v += step) {
     if (!alive[v]) continue;
@@ -114,7 +119,7 @@ __global__ void table_insert_kernel(const uint64_t *key, const uint8_t *alive, u
       const unsigned long long old =
           atomicCAS((unsigned long long *)(table + 2 * s), ~0ULL, kk);
       if (old == ~0ULL) {
-        table[2 * s + 1] = v;
+        table[2 * s + 1] = pos ? v | (uint64_t)pos[v] << 32 : v;
         break;
       }
       if (old == kk) {  // a k-mer twice: the SBWT is malformed
@@ -196,18 +201,30 @@ bool IndexImpl::build_kmer_table() {
   if (slots > (1ULL << 32) || slots * 16 > kKmerTableMaxBytes ||
       slots * 16 + filter_words * 8 > free_b / 4)
     return false;
+  // the path cover first: the table's values hold its positions.  An index
+  // that cannot have it (or no memory for it) keeps the table alone.
+  DeviceBuffer pos;
+  try {
+    if (!build_path_cover(key.get<u64>(), alive.get<u8>(), n_kmers, pos)) pos.release();
+  } catch (const Error &e) {
+    if (e.code != SBWT_E_OOM) throw;
+    cudaGetLastError();
+    pos.release();
+    drop_path_cover();
+  }
   kmer_table.resize(slots * 16);
   SBWT_CUDA(cudaMemset(kmer_table.get(), 0xFF, slots * 16));
   DeviceBuffer d_err(4);
   SBWT_CUDA(cudaMemset(d_err.get(), 0, 4));
   table_insert_kernel<<<grid_of(n), 256>>>(key.get<u64>(), alive.get<uint8_t>(), n,
-                                           kmer_table.get<u64>(), slots - 1,
+                                           pos.get<u32>(), kmer_table.get<u64>(), slots - 1,
                                            d_err.get<uint32_t>());
   SBWT_CUDA(cudaGetLastError());
   uint32_t e = 0;
   SBWT_CUDA(cudaMemcpy(&e, d_err.get(), 4, cudaMemcpyDeviceToHost));
   if (e) {
     kmer_table.release();
+    drop_path_cover();
     throw Error(SBWT_E_FORMAT, "an SBWT k-mer occurs twice");
   }
   kmer_filter.resize(filter_words * 8);
@@ -218,6 +235,7 @@ bool IndexImpl::build_kmer_table() {
   SBWT_CUDA(cudaGetLastError());
   view.kmer_table = kmer_table.get<u64>();
   view.kmer_table_mask = slots - 1;
+  view.node_mask = view.path_node ? 0xFFFFFFFFULL : ~0ULL;
   view.kmer_filter = kmer_filter.get<u64>();
   view.filter_words = filter_words;
   table_kmers = n_kmers;
@@ -228,6 +246,7 @@ void IndexImpl::drop_kmer_table() {
   DeviceGuard g(device);
   kmer_table.release();
   kmer_filter.release();
+  drop_path_cover();
   view.kmer_table = nullptr;
   view.kmer_table_mask = 0;
   view.kmer_filter = nullptr;

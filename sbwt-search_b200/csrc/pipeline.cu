@@ -66,7 +66,7 @@ struct PipelineImpl {
     d_ends.resize(max_reads * 8);
     d_results.resize(max_chars * 8);
     kmer_off.resize((max_reads + 1) * 8);
-    packed.resize((n_words + 2) * 8);
+    packed.resize((n_words + 2) * 16);  // words, or interleaved entries
     invalid.resize((n_words + 2) * 4);
     block_sums.resize(((max_reads + 4095) / 4096 + 1) * 8);
     total.resize(8);

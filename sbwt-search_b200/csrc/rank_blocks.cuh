@@ -108,6 +108,25 @@ __device__ __forceinline__ uint64_t kmer_filter_bits(uint64_t z) {
          (1ULL << ((z >> 18) & 63));
 }
 
+// L-mer filter: a blocked Bloom filter with one 64-bit word per L-mer, two of
+// its bits in either half, from a 32-bit hash (the MurmurHash3 finalizer,
+// Appleby 2011, of the L-mer folded to 32 bits): a third of the instructions
+// that kmer_mix and the k-mer filter's bits take.
+__device__ __forceinline__ uint32_t lmer_hash(uint64_t lmer) {
+  uint32_t z = (uint32_t)lmer ^ ((uint32_t)(lmer >> 32) * 0x9e3779b1u);
+  z = (z ^ (z >> 16)) * 0x85ebca6bu;
+  z = (z ^ (z >> 13)) * 0xc2b2ae35u;
+  return z ^ (z >> 16);
+}
+__device__ __forceinline__ uint32_t lmer_word(uint32_t z, uint32_t n_words) {
+  return __umulhi(z, n_words);
+}
+__device__ __forceinline__ uint2 lmer_bits(uint32_t z) {
+  const uint32_t g = z * 0x9e3779b1u;
+  return make_uint2((1u << (g >> 27)) | (1u << ((g >> 22) & 31)),
+                    (1u << ((g >> 17) & 31)) | (1u << ((g >> 12) & 31)));
+}
+
 // rank_c(i): ones of vector c in [0, i), i in [0, N].
 __device__ __forceinline__ uint64_t rank_full(const SbwtView &s, uint32_t c,
                                               uint64_t i) {

@@ -1,0 +1,53 @@
+"""Read search over the path cover (the automatic kernel of an index with its
+k-mer table): equal to the oracle on the graphs and reads where runs end."""
+import numpy as np
+import pytest
+
+import sbwt_b200 as S
+import sbwt_tools as T
+from helpers import TMP, mixed_reads, oracle_index, oracle_results
+
+pytestmark = pytest.mark.gpu
+
+
+def genomes_of(kind: str, k: int) -> T.Genomes:
+    if kind == "strains":  # branches every few k-mers
+        return T.gen_genomes(5, 12, 4000, 2, 0.03, 0.03, 0.0)
+    rng = np.random.default_rng(9)
+    base = np.frombuffer(b"ACGT", np.uint8)
+    if kind == "circular":  # one long cycle (each sequence repeats its first k - 1 chars)
+        seqs = [base[rng.integers(0, 4, 3000)]]
+        seqs = [np.concatenate([s, s[:k - 1]]) for s in seqs]
+    else:  # short cycles: tandem repeats of 1 to 90 chars
+        seqs = [np.tile(base[rng.integers(0, 4, u)], 1 + 200 // u) for u in (1, 2, 7, 40, 90)]
+    return T.Genomes(np.concatenate(seqs), np.array([len(s) for s in seqs], np.uint64))
+
+
+@pytest.mark.parametrize("kind", ["strains", "circular", "tandem"])
+@pytest.mark.parametrize("k", [31, 30, 21, 13, 6])
+def test_path_cover_matches_oracle(kind, k):
+    import torch
+    g = genomes_of(kind, k)
+    path = TMP / f"cover_{kind}_{k}.sbwt"
+    T.build_sbwt(g, k, str(path))
+    idx = S.SbwtIndex.open(path)
+    oracle = oracle_index(str(path), min(k, 6))
+    src = g if kind != "tandem" else T.Genomes(np.concatenate([g.chars, g.chars, g.chars]),
+                                               np.array([3 * len(g.chars)], np.uint64))
+    for sub, n_rate in ((0.0, 0.0), (0.01, 0.005), (0.1, 0.03)):
+        chars, ends = mixed_reads(src, 17, 700, median=90, sigma=0.8, sub=sub, n_rate=n_rate,
+                                  frac=0.8, len_min=0, len_max=500)
+        exp = oracle_results(oracle, chars, ends)
+        d_chars = torch.from_numpy(chars.copy()).cuda()
+        d_ends = torch.from_numpy(ends.view(np.int64).copy()).cuda()
+        try:
+            for tile in (0, 1, 31, 32, 33, 129):
+                S.set_launch_config(tile=tile)
+                out = torch.full((len(exp) + 4,), -7, dtype=torch.int64, device="cuda")
+                assert idx.search_reads(d_chars, d_ends, out=out) == len(exp)
+                got = out.cpu().numpy()
+                assert np.array_equal(got[:len(exp)].view(np.uint64), exp)
+                assert (got[len(exp):] == -7).all()
+        finally:
+            S.set_launch_config()
+        assert np.array_equal(idx.search_reads(chars, ends), exp)  # 32-bit codes, widened
