@@ -49,8 +49,7 @@ struct ColorsView {
   const uint32_t *sparse;   // sparse color ids
   uint32_t num_colors;
   uint32_t row_words;       // ceil(num_colors / 64)
-  uint32_t words_per_lane;  // row words per lane in one color tile (<= 4)
-  uint32_t tiles;           // color tiles per read: ceil(row_words / (32 * words_per_lane))
+  uint32_t tiles;           // color tiles per read: ceil(row_words / 32)
   uint32_t sparse_sorted;   // 1 when every sparse list is strictly ascending
 };
 
@@ -64,17 +63,16 @@ struct ColorsImpl {
                    u64 n_reads, double tau, u32 flags, uint32_t *ids, u64 capacity,
                    u64 *ids_offsets, cudaStream_t st) const;
   void launch(const u64 *d_vals, const u64 *d_offs, const u64 *d_nf, const u64 *d_inv,
-              u64 n_reads, u64 max_kmers, double tau, u32 flags, int mode,
-              u64 *d_pass_bits, uint32_t *d_pass_count, uint32_t *d_counts,
+              u64 n_reads, int planes, double tau, u32 flags, int mode, u64 *d_pass_bits,
+              uint32_t *d_word_mask, uint32_t *d_pass_count, uint32_t *d_counts,
               uint32_t *d_err, cudaStream_t st) const;
+  void emit_ids(const u64 *d_pass_bits, const uint32_t *d_word_mask, const u64 *d_ids_off,
+                u64 n_reads, uint32_t *d_ids, u64 capacity, cudaStream_t st) const;
 
   void enqueue_pseudoalign(const u64 *d_vals, const u64 *d_offs, u64 n_reads, u64 max_kmers,
                            double tau, u32 flags, u64 *d_pass_bits, uint32_t *d_pass_count,
                            u64 *d_ids_off, uint32_t *d_ids, u64 ids_capacity,
                            uint32_t *d_err, cudaStream_t st) const;
-  // sets the shared-memory attribute for batches of up to max_kmers k-mers per
-  // read (must precede a stream capture)
-  void prepare_launch(u64 max_kmers) const;
   // builds (or drops) the per-node set record table; false when not built
   bool set_node_table(bool enable);
   u64 device_footprint() const;

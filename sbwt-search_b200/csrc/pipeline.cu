@@ -81,7 +81,7 @@ struct PipelineImpl {
       const u64 rw = (ci->num_colors + 63) / 64;
       ids_capacity = max_reads * 64;
       pass_bits.resize(max_reads * rw * 8);
-      pass_count.resize(max_reads * 4);
+      pass_count.resize(max_reads * 4 * (1 + (u64)ci->view.tiles));  // counts, word masks
       ids_off.resize((max_reads + 1) * 8);
       ids.resize(ids_capacity * 4);
       SBWT_CUDA(cudaMallocHost(&h_ids_off, (max_reads + 1) * 8));
@@ -156,7 +156,6 @@ struct PipelineImpl {
   // launches it; completion is signalled by `done`.
   void launch() {
     DeviceGuard g(device);
-    if (ci) ci->prepare_launch(std::max<u64>(max_read_kmers, 1));
     SBWT_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeRelaxed));
     try {
       enqueue();
@@ -203,10 +202,10 @@ struct PipelineImpl {
       throw Error(SBWT_E_INVALID, "an SBWT index is not a key k-mer of this color index");
     if (*h_total != n_kmers) throw Error(SBWT_E_CUDA, "k-mer count mismatch");
     if (ci) {
+      big_ids.clear();  // of an earlier batch
       const u64 n_ids = h_ids_off[n_reads];
       if (n_ids > ids_capacity) {  // rare: more ids than the staging holds
-        std::vector<uint32_t> tmp;
-        expand_from_bits(tmp);
+        expand_from_bits();
         return;
       }
       if (n_ids)
@@ -216,21 +215,22 @@ struct PipelineImpl {
   }
 
   // Fallback when a batch passes more ids than ids_capacity: the ids are
-  // expanded on the host from the per-read pass bitmasks.
+  // expanded on the host from the reads' passing words.
   std::vector<uint32_t> big_ids;
-  void expand_from_bits(std::vector<uint32_t> &) {
-    const u64 rw = (ci->num_colors + 63) / 64;
+  void expand_from_bits() {
+    const u64 rw = ci->view.row_words, T = ci->view.tiles;
     std::vector<u64> bits(n_reads * rw);
+    std::vector<uint32_t> mask(n_reads * T);
     SBWT_CUDA(cudaMemcpy(bits.data(), pass_bits.get(), bits.size() * 8, cudaMemcpyDeviceToHost));
-    big_ids.clear();
+    SBWT_CUDA(cudaMemcpy(mask.data(), pass_count.get<uint32_t>() + n_reads, mask.size() * 4,
+                         cudaMemcpyDeviceToHost));
     h_ids_off[0] = 0;
     for (u64 r = 0; r < n_reads; ++r) {
-      for (u64 w = 0; w < rw; ++w) {
-        u64 m = bits[r * rw + w];
-        while (m) {
-          big_ids.push_back((uint32_t)(w * 64 + __builtin_ctzll(m)));
-          m &= m - 1;
-        }
+      for (u64 t = 0; t < T; ++t) {
+        const u64 *w = bits.data() + r * rw + 32 * t;
+        for (uint32_t k = mask[r * T + t]; k; k &= k - 1, ++w)
+          for (u64 m = *w; m; m &= m - 1)
+            big_ids.push_back((uint32_t)((32 * t + __builtin_ctz(k)) * 64 + __builtin_ctzll(m)));
       }
       h_ids_off[r + 1] = big_ids.size();
     }
