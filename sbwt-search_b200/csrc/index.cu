@@ -3281,10 +3281,13 @@ void IndexImpl::search_positions(const u64 *bit_seqs, u64 n_words, const u64 *po
     throw Error(SBWT_E_INVALID, "SBWT_MOVE_TO_KEY_KMER needs key k-mer marks");
   const SbwtView sv = view_for(cfg.presearch_letters);
   const u32 mtk = (flags & SBWT_MOVE_TO_KEY_KMER) ? 1u : 0u;
-  const int grid = grid_for(device, n, 256, cfg.blocks_per_sm);
+  const int grid = grid_for(device, n, 256, 4 * cfg.blocks_per_sm);
+  // table kernel mode 0 keeps the presearch and steps
+  const auto kernel = sv.kmer_table && cfg.table_kernel != 0 ? search_positions_table_kernel
+                                                             : search_positions_kernel;
   if (flags & SBWT_DEVICE_POINTERS) {
-    search_positions_kernel<<<grid, 256, 0, st>>>(sv, bit_seqs, n_words * 32, positions,
-                                                   n, results, mtk, ws.err_dev.get<u32>());
+    kernel<<<grid, 256, 0, st>>>(sv, bit_seqs, n_words * 32, positions, n, results, mtk,
+                                 ws.err_dev.get<u32>());
     note_launches(1);
     SBWT_CUDA(cudaGetLastError());
     check_err_word(ws, st);
@@ -3297,10 +3300,8 @@ void IndexImpl::search_positions(const u64 *bit_seqs, u64 n_words, const u64 *po
   SBWT_CUDA(cudaMemsetAsync(ws.bits.get<u64>() + n_words, 0, 16, s0));
   SBWT_CUDA(cudaMemcpyAsync(ws.bits.get(), bit_seqs, n_words * 8, cudaMemcpyHostToDevice, s0));
   SBWT_CUDA(cudaMemcpyAsync(ws.positions.get(), positions, n * 8, cudaMemcpyHostToDevice, s0));
-  search_positions_kernel<<<grid, 256, 0, s0>>>(sv, ws.bits.get<u64>(), n_words * 32,
-                                                 ws.positions.get<u64>(), n,
-                                                 ws.results[0].get<u64>(), mtk,
-                                                 ws.err_dev.get<u32>());
+  kernel<<<grid, 256, 0, s0>>>(sv, ws.bits.get<u64>(), n_words * 32, ws.positions.get<u64>(), n,
+                               ws.results[0].get<u64>(), mtk, ws.err_dev.get<u32>());
   note_launches(1);
   SBWT_CUDA(cudaGetLastError());
   SBWT_CUDA(cudaMemcpyAsync(results, ws.results[0].get(), n * 8, cudaMemcpyDeviceToHost, s0));

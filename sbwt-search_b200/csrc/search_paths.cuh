@@ -360,4 +360,99 @@ __global__ void __launch_bounds__(256, kPathsBlocksPerSm)
   }
 }
 
+// The reference seam of an index with its k-mer table (k <= 31): a k-mer is a
+// table lookup (32 bytes) instead of a presearch entry and k - p steps.
+// Positions usually come from reads, so consecutive entries are consecutive
+// positions: a warp takes 32 entries, and in kLeadRounds rounds the first
+// unresolved entry of every stretch of consecutive positions is looked up and
+// the entries behind it follow the path cover as far as their chars agree
+// with it; what is left is looked up entry by entry, all together.
+// What bounds it: the lookups' random DRAM sectors and the round trips of a
+// round.  4 M positions on a 20 M-node index, a third of them absent: whole
+// call 392 us with presearch and steps, 98 us here (two leading rounds 105 us,
+// none 115 us; one round is the best or near it with no and with many absent
+// k-mers).  32 registers, so that 64 warps per SM hide the round trips: 100 us
+// against 107 us at 40.
+constexpr int kLeadRounds = 1;
+__global__ void __launch_bounds__(256, 8) search_positions_table_kernel(
+    SbwtView s, const uint64_t *__restrict__ packed, uint64_t n_chars_cap,
+    const uint64_t *__restrict__ positions, uint64_t n, uint64_t *__restrict__ out,
+    uint32_t move_to_key, uint32_t *err) {
+  constexpr uint32_t FULL = 0xFFFFFFFFu;
+  const uint32_t k = s.k, lane = threadIdx.x & 31;
+  const uint64_t pol_first = l2_policy_evict_first();
+  const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
+  for (uint64_t t0 = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) & ~31ULL; t0 < n;
+       t0 += step) {
+    const uint64_t t = t0 + lane;
+    const uint64_t pos = t < n ? __ldg(positions + t) : 0;
+    uint64_t v = SBWT_NOT_FOUND;
+    const bool in = t < n && pos <= n_chars_cap && n_chars_cap - pos >= k;
+    if (t < n && !in) atomicOr(err, 2u);  // a k-mer past bit_seqs
+    bool open = in;
+    const uint64_t before = __shfl_up_sync(FULL, pos, 1);
+    const bool joined = lane > 0 && pos == before + 1;
+    for (int round = s.path_node ? 0 : kLeadRounds; round <= kLeadRounds; ++round) {
+      const unsigned om = __ballot_sync(FULL, open);
+      if (!om) break;
+      const bool last_round = round == kLeadRounds;
+      // a leader: an open entry that does not continue an open one
+      const bool lead = open && (last_round || !joined || !((om >> (lane - 1)) & 1u));
+      const unsigned lm = __ballot_sync(FULL, lead);
+      // open entries that join on behind this leader
+      const unsigned stop = ~(om & ~lm) & ~((2u << lane) - 1u);
+      const uint32_t behind = lead ? (stop ? (uint32_t)__ffs(stop) - 1u : 32u) - lane - 1 : 0;
+      uint32_t at = ~0u, follow = 0;
+      if (lead) {
+        const uint64_t w = pos >> 5;
+        const uint32_t off = (uint32_t)(pos & 31);
+        uint64_t key = __ldg(packed + w) << (2 * off);
+        if (off + k > 32) key |= __ldg(packed + w + 1) >> (64 - 2 * off);
+        key >>= 64 - 2 * k;
+        uint64_t hs = kmer_table_bucket(key, s.kmer_table_mask);
+        while (true) {
+          const Block A =
+              load_block_hint(reinterpret_cast<const Block *>(s.kmer_table + 2 * hs), pol_first);
+          if (A.w0 == key || A.w2 == key) {
+            const uint64_t value = A.w0 == key ? A.w1 : A.w3;
+            v = value & s.node_mask;
+            at = (uint32_t)(value >> 32);
+            break;
+          }
+          if (A.w0 == ~0ULL || A.w2 == ~0ULL) break;  // an empty slot: absent
+          hs = (hs + 2) & s.kmer_table_mask;
+        }
+        open = false;
+        if (behind && v != SBWT_NOT_FOUND) {
+          // the chars of the entries behind (their words are inside bit_seqs)
+          const uint64_t c = pos + k, cw = c >> 5;
+          const uint32_t co = (uint32_t)(c & 31);
+          uint64_t x = __ldg(packed + cw) << (2 * co);
+          if (co + behind > 32) x |= __ldg(packed + cw + 1) >> (64 - 2 * co);
+          const uint32_t b = at + 1, bo = b & 31;
+          const PathEntry e0 = load_path_entry(s.path_entry + (b >> 5));
+          const PathEntry e1 = load_path_entry(s.path_entry + (b >> 5) + 1);
+          x ^= window_at(e0.chars, e1.chars, bo);
+          const uint64_t mm = (x | (x >> 1)) & 0x5555555555555555ULL;
+          const uint32_t brk = __funnelshift_r(e0.brk, e1.brk, bo);
+          follow = min(min((uint32_t)__clzll(mm) >> 1, (uint32_t)__clz(__brev(brk))), behind);
+        }
+      }
+      if (last_round) break;
+      // entries behind a leader take its next positions
+      const unsigned mine = lm & ((2u << lane) - 1u);
+      const int q = mine ? 31 - __clz(mine) : 0;
+      const uint32_t q_at = __shfl_sync(FULL, at, q), q_follow = __shfl_sync(FULL, follow, q);
+      if (open && mine && lane - q <= q_follow) {
+        v = __ldg(s.path_node + q_at + (lane - q));
+        open = false;
+      }
+    }
+    if (t < n) {
+      if (move_to_key && v != SBWT_NOT_FOUND) v = key_walk(s, v, err);
+      __stcs(out + t, (unsigned long long)v);
+    }
+  }
+}
+
 }  // namespace sbwt

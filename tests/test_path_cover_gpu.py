@@ -3,6 +3,7 @@ k-mer table): equal to the oracle on the graphs and reads where runs end."""
 import numpy as np
 import pytest
 
+import oracle as O
 import sbwt_b200 as S
 import sbwt_tools as T
 from helpers import TMP, mixed_reads, oracle_index, oracle_results
@@ -51,3 +52,42 @@ def test_path_cover_matches_oracle(kind, k):
         finally:
             S.set_launch_config()
         assert np.array_equal(idx.search_reads(chars, ends), exp)  # 32-bit codes, widened
+
+
+@pytest.mark.parametrize("kind", ["strains", "circular", "tandem"])
+@pytest.mark.parametrize("k", [31, 21, 6])
+def test_positions_over_the_cover_match_oracle(kind, k):
+    """The positions seam with its k-mer table: stretches of consecutive
+    positions of every length, steps back, repeats and scattered positions, up
+    to the last k-mer of bit_seqs; one past it is an error."""
+    import torch
+    g = genomes_of(kind, k)
+    path = TMP / f"cover_{kind}_{k}.sbwt"
+    T.build_sbwt(g, k, str(path))
+    idx = S.SbwtIndex.open(path)
+    chars, ends = mixed_reads(g, 19, 200, median=60, sigma=0.5, sub=0.01, n_rate=0.01, frac=0.9,
+                              len_min=0, len_max=200)
+    chars = np.concatenate([chars, g.chars])[:len(chars) + (-len(chars)) % 32 + 32 * 4]
+    bits, _ = O.seq_to_bits(chars.tobytes())
+    bits = bits[:len(chars) // 32]  # no word past the last char
+    last = len(chars) - k
+    rng = np.random.default_rng(k)
+    parts = [np.arange(last + 1), np.arange(last, -1, -1), rng.integers(0, last + 1, 500),
+             np.full(40, last), np.arange(last - 40, last + 1)]
+    for n in range(1, 70):
+        a = int(rng.integers(0, last + 1 - n))
+        parts.append(np.arange(a, a + n))
+    pos = np.concatenate(parts).astype(np.uint64)
+    exp = oracle_index(str(path), min(k, 6)).search_positions(bits, pos)
+    assert np.array_equal(idx.search(bits, pos), exp)
+    d_bits, d_pos = (torch.from_numpy(x.view(np.int64).copy()).cuda() for x in (bits, pos))
+    for table in (True, False):
+        idx.set_kmer_table(table)
+        out = torch.full((len(pos) + 1,), -7, dtype=torch.int64, device="cuda")
+        idx.search(d_bits, d_pos, out=out)
+        got = out.cpu().numpy()
+        assert np.array_equal(got[:-1].view(np.uint64), exp) and got[-1] == -7
+    idx.set_kmer_table(True)
+    with pytest.raises(S.SbwtError) as e:
+        idx.search(bits, np.array([0, last + 1], np.uint64))
+    assert e.value.code == S.E_INVALID
