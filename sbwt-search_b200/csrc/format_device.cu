@@ -12,10 +12,12 @@
 // color separated by ',' and ended by '\n'.  Headers (and the csv title row)
 // are written once per file by the host writers, not here.
 //
-// Ascii needs the byte length of every read before anything is written: one
-// warp per read sums its token lengths, a multi-block scan turns the lengths
-// into offsets, and one warp per read writes its tokens at warp-scanned
-// positions.  The other formats have closed-form offsets.
+// Ascii is written in tiles of kTile tokens, whatever the reads' lengths: a
+// pass over the tokens sums each tile's bytes, a scan turns them into offsets,
+// and one block per tile composes its bytes in shared memory and stores them
+// 16 at a time.  Every token is followed by one ' ' or '\n', so the first pass
+// needs nothing of the reads but the empty ones ('\n' each) of a tile.  The
+// other formats have closed-form offsets.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -31,45 +33,49 @@ namespace {
 constexpr uint32_t FULL = 0xFFFFFFFFu;
 constexpr uint32_t kScanThreads = 1024, kScanPer = 4, kScanSpan = kScanThreads * kScanPer;
 
-__device__ __forceinline__ uint32_t dec_len(uint64_t v) {
-  uint32_t n = 1;
-  uint64_t p = 10;
-  while (n < 20 && v >= p) {
-    ++n;
-    p *= 10;
+// Decimal digits of v, v < 2^32: entry log2(v) of `table` holds, in its high
+// half, the digits of 2^log2(v) plus a carry-in that adds one from the next
+// power of ten on (Lemire, "Computing the number of digits of an integer even
+// faster", 2021).
+__device__ __forceinline__ uint32_t dec_len32(const uint64_t *table, uint32_t v) {
+  return (uint32_t)((v + table[31 - __clz(v | 1)]) >> 32);
+}
+struct DecLenTable {
+  uint64_t entry[32];
+  constexpr DecLenTable() : entry() {
+    for (int log2 = 0; log2 < 32; ++log2) {
+      uint64_t n = 1, p = 10;  // digits of 2^log2, the first power of ten above it
+      while (p <= (1ULL << log2)) {
+        p *= 10;
+        ++n;
+      }
+      entry[log2] = p < (2ULL << log2) ? ((n + 1) << 32) - p : n << 32;
+    }
   }
+};
+__constant__ const DecLenTable kDecLen{};
+__device__ uint32_t dec_len64(uint64_t v) {
+  uint32_t n = 1;
+  for (; v >= 10; v /= 10) ++n;
   return n;
 }
 
-__device__ __forceinline__ void put_dec(uint8_t *out, uint64_t v, uint32_t n) {
-  if (v < (1ULL << 32)) {
-    uint32_t x = (uint32_t)v;
-    for (uint32_t i = n; i-- > 0;) {
-      out[i] = (uint8_t)('0' + x % 10);
-      x /= 10;
-    }
-  } else {
-    for (uint32_t i = n; i-- > 0;) {
-      out[i] = (uint8_t)('0' + v % 10);
-      v /= 10;
-    }
-  }
+// Four decimal digits of x < 10000 as ascii bytes, the first in the low byte.
+__device__ __forceinline__ uint32_t dec4(uint32_t x) {
+  const uint32_t q = (x * 5243u) >> 19;  // x / 100
+  const uint32_t z = q | (x - 100 * q) << 16;
+  const uint32_t t = ((z * 103u) >> 10) & 0x000F000Fu;  // each half / 10
+  return (t | (z - 10 * t) << 8) + 0x30303030u;
 }
 
-// Ascii token of one index result: its length and its bytes.
-__device__ __forceinline__ uint32_t index_token_len(uint64_t v) {
-  return (v == SBWT_NOT_FOUND || v == SBWT_INVALID) ? 2 : dec_len(v);
-}
-__device__ __forceinline__ void index_token(uint8_t *out, uint64_t v, uint32_t n) {
-  if (v == SBWT_NOT_FOUND) {
-    out[0] = '-';
-    out[1] = '1';
-  } else if (v == SBWT_INVALID) {
-    out[0] = '-';
-    out[1] = '2';
-  } else {
-    put_dec(out, v, n);
-  }
+// Tokens of the index results (u64, two markers) and of the color ids (u32).
+__device__ __forceinline__ bool is_marker(uint64_t v) { return v >= SBWT_INVALID; }
+__device__ __forceinline__ bool is_marker(uint32_t) { return false; }
+template <class V>
+__device__ __forceinline__ uint32_t token_len(const uint64_t *table, V v) {
+  if (is_marker(v)) return 2;
+  if (sizeof(V) == 4 || (uint64_t)v < (1ULL << 32)) return dec_len32(table, (uint32_t)v);
+  return dec_len64((uint64_t)v);
 }
 
 // k-mers of read r (reads shorter than k have none), from the read ends.
@@ -78,75 +84,11 @@ __device__ __forceinline__ uint64_t kmers_of(const uint64_t *ends, uint64_t r, u
   return len >= k ? len - k + 1 : 0;
 }
 
-__device__ __forceinline__ uint64_t warp_sum(uint64_t x) {
-  for (int o = 16; o; o >>= 1) x += __shfl_xor_sync(FULL, x, o);
-  return x;
-}
-
-// Exclusive warp scan; *total = warp sum.
-__device__ __forceinline__ uint64_t warp_exclusive(uint64_t v, uint64_t *total) {
-  const uint32_t lane = threadIdx.x & 31;
-  uint64_t x = v;
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint64_t y = __shfl_up_sync(FULL, x, o);
-    if (lane >= (uint32_t)o) x += y;
-  }
-  *total = __shfl_sync(FULL, x, 31);
-  return x - v;
-}
-
-// Per read (one warp each): k-mers -> kmers[r], ascii bytes -> bytes[r].
-__global__ void index_lengths_kernel(const uint64_t *res, const uint64_t *ends, uint64_t n_reads,
-                                     uint32_t k, const uint64_t *kmer_off, uint64_t *bytes) {
-  const uint32_t lane = threadIdx.x & 31;
-  const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  for (uint64_t r = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; r < n_reads;
-       r += warps) {
-    const uint64_t m = kmers_of(ends, r, k), t0 = kmer_off[r];
-    uint64_t s = 0;
-    for (uint64_t j = lane; j < m; j += 32) s += index_token_len(res[t0 + j]);
-    s = warp_sum(s);
-    if (lane == 0) bytes[r] = s + (m ? m : 1);  // separators + '\n'
-  }
-}
-
 __global__ void kmer_counts_kernel(const uint64_t *ends, uint64_t n_reads, uint32_t k,
                                    uint64_t *kmers) {
   const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; r < n_reads; r += step)
     kmers[r] = kmers_of(ends, r, k);
-}
-
-__global__ void index_ascii_kernel(const uint64_t *res, const uint64_t *ends, uint64_t n_reads,
-                                   uint32_t k, const uint64_t *kmer_off,
-                                   const uint64_t *byte_off, uint8_t *out) {
-  const uint32_t lane = threadIdx.x & 31;
-  const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  for (uint64_t r = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; r < n_reads;
-       r += warps) {
-    const uint64_t m = kmers_of(ends, r, k), t0 = kmer_off[r];
-    uint64_t at = byte_off[r];
-    if (m == 0) {
-      if (lane == 0) out[at] = '\n';
-      continue;
-    }
-    for (uint64_t j0 = 0; j0 < m; j0 += 32) {
-      const uint64_t j = j0 + lane;
-      uint64_t v = 0;
-      uint32_t n = 0;
-      if (j < m) {
-        v = res[t0 + j];
-        n = index_token_len(v);
-      }
-      uint64_t total;
-      const uint64_t pos = at + warp_exclusive(n ? n + 1 : 0, &total);
-      if (j < m) {
-        index_token(out + pos, v, n);
-        out[pos + n] = j + 1 == m ? '\n' : ' ';
-      }
-      at += total;
-    }
-  }
 }
 
 __global__ void index_fixed_kernel(const uint64_t *res, const uint64_t *ends, uint64_t n_reads,
@@ -168,50 +110,6 @@ __global__ void index_fixed_kernel(const uint64_t *res, const uint64_t *ends, ui
         o[j] = v == SBWT_NOT_FOUND ? '1' : (v == SBWT_INVALID ? '2' : '0');
       }
       if (lane == 0) o[m] = '\n';
-    }
-  }
-}
-
-__global__ void color_lengths_kernel(const uint32_t *ids, const uint64_t *ids_off,
-                                     uint64_t n_reads, uint64_t *bytes) {
-  const uint32_t lane = threadIdx.x & 31;
-  const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  for (uint64_t r = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; r < n_reads;
-       r += warps) {
-    const uint64_t a = ids_off[r], b = ids_off[r + 1];
-    uint64_t s = 0;
-    for (uint64_t t = a + lane; t < b; t += 32) s += dec_len(ids[t]);
-    s = warp_sum(s);
-    if (lane == 0) bytes[r] = s + (b > a ? b - a : 1);
-  }
-}
-
-__global__ void color_ascii_kernel(const uint32_t *ids, const uint64_t *ids_off,
-                                   uint64_t n_reads, const uint64_t *byte_off, uint8_t *out) {
-  const uint32_t lane = threadIdx.x & 31;
-  const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  for (uint64_t r = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; r < n_reads;
-       r += warps) {
-    const uint64_t a = ids_off[r], b = ids_off[r + 1];
-    uint64_t at = byte_off[r];
-    if (b == a) {
-      if (lane == 0) out[at] = '\n';
-      continue;
-    }
-    for (uint64_t t0 = a; t0 < b; t0 += 32) {
-      const uint64_t t = t0 + lane;
-      uint32_t v = 0, n = 0;
-      if (t < b) {
-        v = ids[t];
-        n = dec_len(v);
-      }
-      uint64_t total;
-      const uint64_t pos = at + warp_exclusive(n ? n + 1 : 0, &total);
-      if (t < b) {
-        put_dec(out + pos, v, n);
-        out[pos + n] = t + 1 == b ? '\n' : ' ';
-      }
-      at += total;
     }
   }
 }
@@ -320,11 +218,432 @@ __global__ void __launch_bounds__(kScanThreads) scan_apply_kernel(uint64_t *v, u
   if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) v[n] = tops[gridDim.x];
 }
 
+// ---- ascii in tiles of tokens ------------------------------------------------
+constexpr uint32_t kTileThreads = 256, kTokens = 8, kTile = kTileThreads * kTokens;
+// Bytes of a tile that shared memory holds (16 per token); a tile with more
+// (thousands of empty reads, or tokens of 16 and more digits) is written
+// straight to its place.
+constexpr uint32_t kTileBytes = 16 * kTile;
+
+// One thread per read: first_read[t] = the first read r with off[r] - off[0]
+// >= t * kTile (t <= n / kTile), the empty reads of each tile, and the bit of
+// every read's last token in `ends` (both zeroed before).
+// status: 0 (flags, set later), off[n_reads] - off[0], off[0], 0 (a count).  Tokens
+// past max_n (< tiles * kTile) count as its last one.
+__global__ void tile_lines_kernel(const uint64_t *off, uint64_t n_reads, uint64_t max_n,
+                                  uint64_t *first_read, uint32_t *empty, uint32_t *ends,
+                                  uint64_t *status) {
+  const uint64_t step = (uint64_t)gridDim.x * blockDim.x, base = off[0];
+  const uint64_t n = min(off[n_reads] - base, max_n);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    status[0] = 0;
+    status[1] = off[n_reads] - base;
+    status[2] = base;
+    status[3] = 0;
+  }
+  const uint32_t lane = threadIdx.x & 31;
+  for (uint64_t r0 = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) & ~31ULL; r0 <= n_reads;
+       r0 += step) {
+    const uint64_t r = r0 + lane;
+    uint64_t a = 0;
+    bool none = false;
+    if (r <= n_reads) {
+      a = min(off[r] - base, n);
+      const uint64_t before = r ? min(off[r - 1] - base, n) : 0;
+      for (uint64_t t = r ? before / kTile + 1 : 0; t <= a / kTile; ++t) first_read[t] = r;
+      if (r && a > before) atomicOr(ends + (a - 1) / 32, 1u << ((a - 1) & 31));
+      none = r < n_reads && min(off[r + 1] - base, n) == a;
+    }
+    const unsigned m = __ballot_sync(FULL, none);
+    if (!m) continue;
+    const uint64_t t = a / kTile;
+    // neighbours are in the same tile nearly always: one add for them
+    const int lead = __ffs(m) - 1;
+    const uint64_t t0 = __shfl_sync(FULL, t, lead);
+    const unsigned same = __ballot_sync(FULL, none && t == t0);
+    if ((int)lane == lead) atomicAdd(empty + t0, __popc(same));
+    if (none && t != t0) atomicAdd(empty + t, 1u);
+  }
+}
+
+// This thread's kTokens tokens of the tile from slot s0 (missing ones 0).
+template <class V>
+__device__ __forceinline__ void load_tokens(const V *tok, uint64_t s0, uint64_t n,
+                                            V (&v)[kTokens]) {
+  const uint64_t i = s0 + kTokens * threadIdx.x;
+  if (i + kTokens <= n && ((uintptr_t)(tok + i) & 15) == 0) {
+#pragma unroll
+    for (uint32_t q = 0; q < kTokens; q += 16 / sizeof(V)) {
+      if constexpr (sizeof(V) == 8) {
+        const ulonglong2 a = __ldcs(reinterpret_cast<const ulonglong2 *>(tok + i + q));
+        v[q] = (V)a.x;
+        v[q + 1] = (V)a.y;
+      } else {
+        const uint4 a = __ldcs(reinterpret_cast<const uint4 *>(tok + i + q));
+        v[q] = (V)a.x;
+        v[q + 1] = (V)a.y;
+        v[q + 2] = (V)a.z;
+        v[q + 3] = (V)a.w;
+      }
+    }
+    return;
+  }
+#pragma unroll
+  for (uint32_t q = 0; q < kTokens; ++q) v[q] = i + q < n ? tok[i + q] : 0;
+}
+
+// bytes[t]: the tile's tokens and terminators plus its empty reads; *flags
+// gets bit 0 when some tile has more bytes than shared memory holds, bit 1
+// when some tile has empty reads.  kSumTiles tiles per block, all their loads in
+// flight.
+constexpr uint32_t kSumTiles = 2;
+constexpr uint64_t kFewTiles = 4 * kTileThreads;
+template <class V>
+__global__ void __launch_bounds__(kTileThreads) tile_bytes_kernel(const V *tok, uint64_t max_n,
+                                                                  uint64_t tiles,
+                                                                  const uint32_t *empty,
+                                                                  uint64_t *bytes,
+                                                                  uint64_t *flags) {
+  const uint64_t n = min(flags[1], max_n);  // tile_lines_kernel's status
+  tok += flags[2];
+  __shared__ uint64_t table[32];
+  __shared__ uint32_t sums[kSumTiles][kTileThreads / 32];
+  if (threadIdx.x < 32) table[threadIdx.x] = kDecLen.entry[threadIdx.x];
+  const uint64_t t0 = blockIdx.x * (uint64_t)kSumTiles;
+  V v[kSumTiles][kTokens];
+#pragma unroll
+  for (uint32_t i = 0; i < kSumTiles; ++i) load_tokens(tok, (t0 + i) * kTile, n, v[i]);
+  __syncthreads();
+#pragma unroll
+  for (uint32_t i = 0; i < kSumTiles; ++i) {
+    const uint64_t s0 = (t0 + i) * kTile + kTokens * threadIdx.x;
+    uint32_t s = 0;
+#pragma unroll
+    for (uint32_t q = 0; q < kTokens; ++q)
+      if (s0 + q < n) s += token_len(table, v[i][q]) + 1;
+    s = __reduce_add_sync(FULL, s);
+    if ((threadIdx.x & 31) == 0) sums[i][threadIdx.x >> 5] = s;
+  }
+  __syncthreads();
+  if (threadIdx.x < kSumTiles && t0 + threadIdx.x < tiles) {
+    const uint32_t e = empty[t0 + threadIdx.x];
+    uint64_t t = e;
+    for (uint32_t w = 0; w < kTileThreads / 32; ++w) t += sums[threadIdx.x][w];
+    bytes[t0 + threadIdx.x] = t;
+    if (e || t > kTileBytes)
+      atomicOr((unsigned long long *)flags, (e ? 2ULL : 0ULL) | (t > kTileBytes ? 1ULL : 0ULL));
+  }
+  if (tiles > kFewTiles) return;
+  // few tiles: the last block to get here turns the bytes into offsets
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0)
+    last = atomicAdd((unsigned long long *)flags + 3, 1ULL) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  uint64_t carry = 0;
+  for (uint64_t i0 = 0; i0 < tiles; i0 += kTileThreads) {
+    const uint64_t i = i0 + threadIdx.x;
+    uint64_t total;
+    const uint64_t ex = block_exclusive(i < tiles ? __ldcg(bytes + i) : 0, &total);
+    if (i < tiles) bytes[i] = carry + ex;
+    carry += total;
+  }
+  if (threadIdx.x == 0) bytes[tiles] = carry;
+}
+
+// ORs the bytes of w into the zeroed bytes at o.
+__device__ __forceinline__ void put_bytes(uint32_t *buf, uint32_t o, uint64_t w) {
+  const uint32_t g = 8 * (o & 3), lo = (uint32_t)w, hi = (uint32_t)(w >> 32);
+  atomicOr(buf + (o >> 2), lo << g);
+  const uint32_t u1 = __funnelshift_l(lo, hi, g), u2 = __funnelshift_l(hi, 0, g);
+  if (u1) atomicOr(buf + (o >> 2) + 1, u1);
+  if (u2) atomicOr(buf + (o >> 2) + 2, u2);
+}
+
+// extra[i] = the empty reads before the token of slot i of the tile.  Slot n (in
+// the last tile) stands for the end: it has no token, only the empty reads
+// after the last one.  By the whole block; the caller waits for the counts.
+__device__ __forceinline__ void count_extras(const uint64_t *off, uint64_t n_reads, uint64_t n,
+                                             const uint64_t *first_read, uint64_t tile,
+                                             uint32_t *extra) {
+  const uint64_t base = off[0], s0 = tile * kTile;
+  for (uint32_t i = threadIdx.x; i < kTile; i += kTileThreads) extra[i] = 0;
+  __syncthreads();
+  const uint64_t r_hi = s0 + kTile <= n ? first_read[tile + 1] : n_reads;
+  for (uint64_t r = first_read[tile] + threadIdx.x; r < r_hi; r += kTileThreads) {
+    const uint64_t a = min(off[r] - base, n);
+    if (min(off[r + 1] - base, n) == a && a - s0 < kTile) atomicAdd(&extra[a - s0], 1u);
+  }
+}
+
+struct TileShared {
+  uint64_t table[32];
+  __align__(16) uint32_t buf[kTileBytes / 4 + 8];
+  uint32_t sums[kTileThreads / 32];
+};
+
+// One block writes a tile of `bytes` <= kTileBytes bytes at dst.  A thread
+// turns its tokens into bytes, eight digits at a time, and ORs them into shared
+// memory at their offsets (a scan of the lengths); the block then stores the
+// bytes 16 at a time, laid out as the output's own 16-byte lines.  left: tokens
+// from the tile's first on; bits: which of this thread's tokens end a read;
+// extra: see count_extras (EXTRAS: there are any).
+template <class V, bool EXTRAS>
+__device__ __forceinline__ void write_tile(TileShared &sh, const V (&v)[kTokens], uint32_t left,
+                                           uint32_t bits, const uint32_t *extra, uint32_t bytes,
+                                           uint8_t *dst) {
+  const uint32_t tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  uint32_t *const buf = sh.buf;
+  const uint32_t shift = (uint32_t)((uintptr_t)dst & 15);  // the place in a 16-byte line
+  const uint32_t stop = shift + bytes;
+  for (uint32_t i = tid; 16 * i < stop; i += kTileThreads)
+    reinterpret_cast<uint4 *>(buf)[i] = make_uint4(0, 0, 0, 0);
+  __syncthreads();
+  uint32_t len[kTokens], mine = 0;
+#pragma unroll
+  for (uint32_t q = 0; q < kTokens; ++q) {
+    len[q] = kTokens * tid + q < left ? token_len(sh.table, v[q]) + 1 : 0;
+    mine += len[q];
+    if (EXTRAS) mine += extra[kTokens * tid + q];
+  }
+  uint32_t x = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(FULL, x, o);
+    if (lane >= (uint32_t)o) x += y;
+  }
+  if (lane == 31) sh.sums[wid] = x;
+  __syncthreads();
+  uint32_t o = shift + x - mine;
+#pragma unroll
+  for (uint32_t w = 0; w < kTileThreads / 32; ++w) o += w < wid ? sh.sums[w] : 0;
+#pragma unroll
+  for (uint32_t q = 0; q < kTokens; ++q) {
+    if (EXTRAS)
+      for (uint32_t e = extra[kTokens * tid + q]; e; --e, ++o)
+        atomicOr(buf + (o >> 2), (uint32_t)'\n' << (8 * (o & 3)));
+    if (!len[q]) continue;
+    const uint32_t term = (bits >> q) & 1u ? '\n' : ' ', end = o + len[q];
+    if (is_marker(v[q])) {
+      put_bytes(buf, o, '-' | ((uint64_t)v[q] == SBWT_NOT_FOUND ? '1' : '2') << 8 | term << 16);
+    } else {
+      uint32_t m = len[q] - 1, b = (uint32_t)v[q];
+      if (m > 8) {  // the digits before the last eight
+        if (sizeof(V) == 4 || (uint64_t)v[q] < (1ULL << 32)) {  // one or two
+          const uint32_t a = b / 100000000u, t = (a * 103u) >> 10;
+          b -= a * 100000000u;
+          const uint32_t two = (t | (a - 10 * t) << 8) + 0x3030u;
+          put_bytes(buf, o, m == 9 ? two >> 8 : two);
+        } else {
+          uint64_t a = (uint64_t)v[q] / 100000000u;
+          b = (uint32_t)((uint64_t)v[q] - a * 100000000u);
+#pragma unroll 1
+          for (uint32_t i = m - 8; i-- > 0; a /= 10)
+            put_bytes(buf, o + i, '0' + (uint32_t)(a % 10));
+        }
+        m = 8;
+      }
+      const uint32_t c = b / 10000u, skip = 8 * (8 - m);
+      const uint64_t d = (uint64_t)dec4(b - 10000u * c) << 32 | dec4(c);
+      // the last m digits and, where it fits, the terminator
+      uint64_t w = d >> skip;
+      if (skip)
+        w |= (uint64_t)term << (64 - skip);
+      else
+        atomicOr(buf + ((end - 1) >> 2), term << (8 * ((end - 1) & 3)));
+      put_bytes(buf, end - 1 - m, w);
+    }
+    o = end;
+  }
+  __syncthreads();
+  uint8_t *const line = dst - shift;
+  for (uint32_t i = tid; 16 * i < stop; i += kTileThreads) {
+    if (16 * i >= shift && 16 * i + 16 <= stop) {
+      __stcs(reinterpret_cast<uint4 *>(line) + i, reinterpret_cast<const uint4 *>(buf)[i]);
+    } else {  // the tile's first and last line
+      const uint8_t *const from = reinterpret_cast<const uint8_t *>(buf);
+      for (uint32_t p = max(16 * i, shift); p < min(16 * i + 16, stop); ++p) line[p] = from[p];
+    }
+  }
+}
+
+// One block per tile.  status: if set, the count and the tokens' place are
+// read from there (tile_lines_kernel's), and nothing is written when the
+// count is above n or the total above out_cap.
+// What bounds it: instructions (about half for the digits and their places, a
+// tenth for the stores) and the waits of a block's few steps, beside 17 bytes
+// of DRAM traffic a token.  139 M tokens: 0.94 ms; one warp per read with byte
+// stores took 1.94 ms, and its lengths pass 0.72 ms against 0.19 ms of
+// tile_bytes_kernel.  4 tokens per thread: 0.99 ms; persistent blocks that
+// load the next tile ahead: 1.16 ms (spills).  EXTRAS costs 0.09 ms, so it is
+// left out of batches without an empty read.
+template <class V, bool EXTRAS>
+__global__ void __launch_bounds__(kTileThreads, 5)
+    tile_ascii_kernel(const V *tok, uint64_t n, const uint64_t *off, uint64_t n_reads,
+                      const uint64_t *first_read, const uint32_t *ends,
+                      const uint64_t *tile_off, uint8_t *out, const uint64_t *status,
+                      uint64_t out_cap) {
+  __shared__ TileShared sh;
+  __shared__ uint32_t extra[EXTRAS ? kTile : 1];
+  if (status) {
+    if (status[1] > n || tile_off[gridDim.x] > out_cap) return;
+    n = status[1];
+    tok += status[2];
+  }
+  const uint64_t s0 = blockIdx.x * (uint64_t)kTile;
+  V v[kTokens];
+  load_tokens(tok, s0, n, v);
+  const uint64_t i0 = s0 + kTokens * threadIdx.x;
+  const uint32_t bits = i0 < n ? __ldg(ends + i0 / 32) >> (i0 & 31) : 0;
+  const uint64_t b0 = __ldg(tile_off + blockIdx.x), b1 = __ldg(tile_off + blockIdx.x + 1);
+  if (b1 == b0 || b1 - b0 > kTileBytes) return;  // past the end; tile_direct_kernel's
+  if (threadIdx.x < 32) sh.table[threadIdx.x] = kDecLen.entry[threadIdx.x];
+  if (EXTRAS) count_extras(off, n_reads, n, first_read, blockIdx.x, extra);
+  write_tile<V, EXTRAS>(sh, v, (uint32_t)min(n - s0, (uint64_t)kTile), bits, extra,
+                        (uint32_t)(b1 - b0), out + b0);
+}
+
+// A small output (out_cap <= kSmallBytes) in one launch and one block: the
+// total, then, if it fits, the tiles one after the other.  result: the total,
+// and 1 when the block did its work (not when a tile is more than shared
+// memory holds).
+constexpr uint64_t kSmallBytes = kTileBytes * 3 / 2;
+template <class V>
+__global__ void __launch_bounds__(kTileThreads)
+    small_ascii_kernel(const V *tok, const uint64_t *off, uint64_t n_reads, uint8_t *out,
+                       uint64_t out_cap, uint64_t *result) {
+  __shared__ TileShared sh;
+  __shared__ uint32_t extra[kTile], ends[kTile / 32];
+  const uint32_t tid = threadIdx.x;
+  const uint64_t base = off[0], n = off[n_reads] - base;
+  tok += base;
+  if (tid < 32) sh.table[tid] = kDecLen.entry[tid];
+  if (tid == 0) result[1] = 0;
+  if (n > kSmallBytes / 2 || n_reads > kSmallBytes) return;  // at least 2 and 1 bytes each
+  __syncthreads();
+  uint32_t mine = 0;  // a total of at most 21 kSmallBytes
+  for (uint64_t i = tid; i < n; i += kTileThreads) mine += token_len(sh.table, tok[i]) + 1;
+  for (uint64_t r = tid; r < n_reads; r += kTileThreads) mine += off[r] == off[r + 1];
+  uint64_t total;
+  block_exclusive(mine, &total);
+  if (tid == 0) {
+    result[0] = total;
+    result[1] = 1;
+  }
+  if (total > out_cap) return;
+  for (uint64_t s0 = 0, at = 0; s0 <= n; s0 += kTile) {
+    __syncthreads();
+    for (uint32_t i = tid; i < kTile; i += kTileThreads) extra[i] = 0;
+    if (tid < kTile / 32) ends[tid] = 0;
+    V v[kTokens];
+    load_tokens(tok, s0, n, v);
+    __syncthreads();
+    for (uint64_t r = tid; r < n_reads; r += kTileThreads) {
+      const uint64_t a = off[r] - base, b = off[r + 1] - base;
+      if (a == b && a - s0 < kTile) atomicAdd(&extra[a - s0], 1u);
+      if (a < b && b - 1 - s0 < kTile) atomicOr(&ends[(b - 1 - s0) / 32], 1u << ((b - 1) & 31));
+    }
+    __syncthreads();
+    mine = 0;
+#pragma unroll
+    for (uint32_t q = 0; q < kTokens; ++q) {
+      const uint32_t sl = kTokens * tid + q;
+      mine += extra[sl] + (s0 + sl < n ? token_len(sh.table, v[q]) + 1 : 0);
+    }
+    uint64_t bytes;
+    block_exclusive(mine, &bytes);
+    if (bytes > kTileBytes) {  // the same for every thread
+      if (tid == 0) result[1] = 0;
+      return;
+    }
+    write_tile<V, true>(sh, v, (uint32_t)min(n - s0, (uint64_t)kTile),
+                        ends[kTokens * tid / 32] >> (kTokens * tid % 32), extra, (uint32_t)bytes,
+                        out + at);
+    at += bytes;
+  }
+}
+
+// The tiles that shared memory does not hold (thousands of empty reads, or
+// tokens of 16 and more digits): every token straight to its place, then the
+// lines of empty reads by the whole block.
+template <class V>
+__global__ void __launch_bounds__(kTileThreads)
+    tile_direct_kernel(const V *tok, uint64_t n, uint64_t tiles, const uint64_t *off,
+                       uint64_t n_reads, const uint64_t *first_read, const uint32_t *ends,
+                       const uint64_t *tile_off, uint8_t *out) {
+  __shared__ uint64_t table[32], starts[kTile];
+  __shared__ uint32_t extra[kTile];
+  const uint32_t tid = threadIdx.x;
+  if (tid < 32) table[tid] = kDecLen.entry[tid];
+  for (uint64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    if (tile_off[tile + 1] - tile_off[tile] <= kTileBytes) continue;
+    const uint64_t s0 = tile * kTile;
+    uint8_t *const dst = out + tile_off[tile];
+    V v[kTokens];
+    load_tokens(tok, s0, n, v);
+    const uint64_t i0 = s0 + kTokens * tid;
+    const uint32_t bits = i0 < n ? ends[i0 / 32] >> (i0 & 31) : 0;
+    count_extras(off, n_reads, n, first_read, tile, extra);
+    __syncthreads();
+    uint64_t mine = 0, total;
+    uint32_t len[kTokens];
+#pragma unroll
+    for (uint32_t q = 0; q < kTokens; ++q) {
+      len[q] = i0 + q < n ? token_len(table, v[q]) : 0;
+      mine += extra[kTokens * tid + q] + (len[q] ? len[q] + 1 : 0);
+    }
+    uint64_t at = block_exclusive(mine, &total);
+#pragma unroll
+    for (uint32_t q = 0; q < kTokens; ++q) {
+      starts[kTokens * tid + q] = at;
+      at += extra[kTokens * tid + q];
+      if (!len[q]) continue;
+      if (is_marker(v[q])) {
+        dst[at] = '-';
+        dst[at + 1] = (uint64_t)v[q] == SBWT_NOT_FOUND ? '1' : '2';
+      } else {
+        uint64_t x = (uint64_t)v[q];
+        for (uint32_t i = len[q]; i-- > 0; x /= 10) dst[at + i] = (uint8_t)('0' + x % 10);
+      }
+      at += len[q];
+      dst[at++] = (bits >> q) & 1u ? '\n' : ' ';
+    }
+    __syncthreads();
+    for (uint32_t sl = 0; sl < kTile; ++sl)
+      for (uint64_t e = tid; e < extra[sl]; e += kTileThreads) dst[starts[sl] + e] = '\n';
+    __syncthreads();
+  }
+}
+
+// The same for n <= kScanSpan values, in one block.
+__global__ void __launch_bounds__(kScanThreads) scan_one_kernel(uint64_t *v, uint64_t n) {
+  const uint64_t i0 = (uint64_t)threadIdx.x * kScanPer;
+  uint64_t c[kScanPer], s = 0;
+#pragma unroll
+  for (uint32_t q = 0; q < kScanPer; ++q) {
+    c[q] = i0 + q < n ? v[i0 + q] : 0;
+    s += c[q];
+  }
+  uint64_t total;
+  uint64_t at = block_exclusive(s, &total);
+#pragma unroll
+  for (uint32_t q = 0; q < kScanPer; ++q) {
+    if (i0 + q < n) v[i0 + q] = at;
+    at += c[q];
+  }
+  if (threadIdx.x == 0) v[n] = total;
+}
+
 struct FormatWorkspace {
-  DeviceBuffer kmer_off, byte_off, tops, in_a, in_b, out;
+  DeviceBuffer kmer_off, tile_read, tile_bytes, line_bits, tops, in_a, in_b, out;
   cudaStream_t stream = nullptr;
+  u64 *host = nullptr;  // pinned: up to four counts
   ~FormatWorkspace() {
     if (stream) cudaStreamDestroy(stream);
+    if (host) cudaFreeHost(host);
   }
 };
 
@@ -335,27 +654,122 @@ FormatWorkspace &format_workspace(int device) {
   if (!p) {
     p = std::make_unique<FormatWorkspace>();
     SBWT_CUDA(cudaStreamCreateWithFlags(&p->stream, cudaStreamNonBlocking));
+    SBWT_CUDA(cudaMallocHost(&p->host, 32));
   }
   return *p;
 }
 
-// v[0..n) (n + 1 entries) -> exclusive offsets, v[n] = total (returned).
-u64 scan_inplace(uint64_t *v, u64 n, FormatWorkspace &ws, cudaStream_t st) {
-  const u64 nb = std::max<u64>((n + kScanSpan - 1) / kScanSpan, 1);
-  ws.tops.ensure((nb + 1) * 8);
-  uint64_t *tops = ws.tops.get<uint64_t>();
-  scan_tops_of_kernel<<<(unsigned)nb, kScanThreads, 0, st>>>(v, n, tops);
-  scan_tops_kernel<<<1, kScanThreads, 0, st>>>(tops, nb);
-  scan_apply_kernel<<<(unsigned)nb, kScanThreads, 0, st>>>(v, n, tops);
+// v[0..n) (n + 1 entries) -> exclusive offsets, v[n] = total.
+void enqueue_scan(uint64_t *v, u64 n, FormatWorkspace &ws, cudaStream_t st) {
+  if (n <= kScanSpan) {
+    scan_one_kernel<<<1, kScanThreads, 0, st>>>(v, n);
+  } else {
+    const u64 nb = (n + kScanSpan - 1) / kScanSpan;
+    ws.tops.ensure((nb + 1) * 8);
+    uint64_t *tops = ws.tops.get<uint64_t>();
+    scan_tops_of_kernel<<<(unsigned)nb, kScanThreads, 0, st>>>(v, n, tops);
+    scan_tops_kernel<<<1, kScanThreads, 0, st>>>(tops, nb);
+    scan_apply_kernel<<<(unsigned)nb, kScanThreads, 0, st>>>(v, n, tops);
+  }
   SBWT_CUDA(cudaGetLastError());
-  u64 total = 0;
-  SBWT_CUDA(cudaMemcpyAsync(&total, v + n, 8, cudaMemcpyDeviceToHost, st));
+}
+
+// enqueue_scan, returning the total; the first `back` (1 to 4) entries from
+// v[n] on come to ws.host.
+u64 scan_inplace(uint64_t *v, u64 n, FormatWorkspace &ws, cudaStream_t st, int back = 1,
+                 bool scanned = false) {
+  if (!scanned) enqueue_scan(v, n, ws, st);
+  SBWT_CUDA(cudaMemcpyAsync(ws.host, v + n, 8 * back, cudaMemcpyDeviceToHost, st));
   SBWT_CUDA(cudaStreamSynchronize(st));
-  return total;
+  return ws.host[0];
 }
 
 unsigned warp_grid(u64 items) {
   return (unsigned)std::min<u64>(std::max<u64>((items + 7) / 8, 1), 148 * 64);
+}
+
+// The whole of format_tokens in one launch when the output's capacity is small
+// (a few reads): false when that did not do (what it wrote is then written again).
+// 100 reads of 2 color ids: 34 us a call against 47 us with a launch per step.
+template <class V>
+bool format_small(const V *tok, const uint64_t *off, u64 n_reads, uint8_t *out, u64 out_cap,
+                  u64 *need, FormatWorkspace &ws, cudaStream_t st) {
+  if (out_cap == 0 || out_cap > kSmallBytes) return false;
+  ws.tile_bytes.ensure(16);
+  uint64_t *result = ws.tile_bytes.get<uint64_t>();
+  small_ascii_kernel<V><<<1, kTileThreads, 0, st>>>(tok, off, n_reads, out, out_cap, result);
+  SBWT_CUDA(cudaGetLastError());
+  SBWT_CUDA(cudaMemcpyAsync(ws.host, result, 16, cudaMemcpyDeviceToHost, st));
+  SBWT_CUDA(cudaStreamSynchronize(st));
+  if (!ws.host[1]) return false;
+  *need = ws.host[0];
+  if (*need > out_cap) throw Error(SBWT_E_CAPACITY, "output capacity too small");
+  return true;
+}
+
+// The tokens tok[off[0], off[n_reads]) in lines (reads) of off as ascii, at
+// most max_n of them; returns the bytes (*need set before the capacity is
+// checked).  The count itself is read on the device, so the host waits once
+// before the bytes are written, for the count, the total and the flags.
+template <class V>
+u64 format_tokens(const V *tok, u64 max_n, const uint64_t *off, u64 n_reads, uint8_t *out,
+                  u64 out_cap, u64 *need, FormatWorkspace &ws, cudaStream_t st) {
+  u64 tiles = max_n / kTile + 1;
+  const u64 words = tiles * (kTile / 32);
+  ws.tile_read.ensure(tiles * 8);
+  ws.tile_bytes.ensure((tiles + 5) * 8);     // offsets, total, status
+  ws.line_bits.ensure((tiles + words) * 4);  // empty reads of the tiles, end bits
+  uint64_t *first = ws.tile_read.get<uint64_t>(), *bytes = ws.tile_bytes.get<uint64_t>();
+  uint32_t *empty = ws.line_bits.get<uint32_t>(), *ends = empty + tiles;
+  SBWT_CUDA(cudaMemsetAsync(empty, 0, (tiles + words) * 4, st));
+  tile_lines_kernel<<<(unsigned)std::min<u64>(n_reads / 256 + 1, 148 * 16), 256, 0, st>>>(
+      off, n_reads, max_n, first, empty, ends, bytes + tiles + 1);
+  tile_bytes_kernel<V><<<(unsigned)((tiles + kSumTiles - 1) / kSumTiles), kTileThreads, 0, st>>>(
+      tok, max_n, tiles, empty, bytes, bytes + tiles + 1);
+  const uint64_t *const status = bytes + tiles + 1;
+  const bool few = tiles <= kFewTiles;  // written before the host knows the count
+  if (few)
+    tile_ascii_kernel<V, true><<<(unsigned)tiles, kTileThreads, 0, st>>>(
+        tok, max_n, off, n_reads, first, ends, bytes, out, status, out_cap);
+  const u64 total = scan_inplace(bytes, tiles, ws, st, 4, few);
+  const u64 flags = ws.host[1], n = ws.host[2], base = ws.host[3];
+  if (n > max_n) return format_tokens(tok, n, off, n_reads, out, out_cap, need, ws, st);
+  if (need) *need = total;
+  if (total > out_cap) throw Error(SBWT_E_CAPACITY, "output capacity too small");
+  tok += base;
+  tiles = n / kTile + 1;
+  if (!few) {
+    auto *const kernel = flags & 2 ? tile_ascii_kernel<V, true> : tile_ascii_kernel<V, false>;
+    kernel<<<(unsigned)tiles, kTileThreads, 0, st>>>(tok, n, off, n_reads, first, ends, bytes,
+                                                     out, nullptr, 0);
+  }
+  if (flags & 1)
+    tile_direct_kernel<V><<<(unsigned)std::min<u64>(tiles, 148 * 16), kTileThreads, 0, st>>>(
+        tok, n, tiles, off, n_reads, first, ends, bytes, out);
+  SBWT_CUDA(cudaGetLastError());
+  return total;
+}
+
+// The ascii of the tokens tok[off[0], off[n_reads]).  Their count is only known
+// on the device: a small output is one launch, a medium one takes the
+// capacity's bound on the count (two bytes a token) for its tiles, and from
+// kBoundBytes on the count is read back first (a wait of ~10 us, against tiles
+// and end bits for several times the tokens).
+constexpr u64 kBoundBytes = 64ULL << 20;
+template <class V>
+u64 format_ascii(const V *tok, const uint64_t *off, u64 n_reads, uint8_t *out, u64 out_cap,
+                 u64 *need, FormatWorkspace &ws, cudaStream_t st) {
+  u64 total = 0;
+  if (format_small(tok, off, n_reads, out, out_cap, need ? need : &total, ws, st))
+    return ws.host[0];
+  u64 max_n = out_cap / 2;
+  if (out_cap == 0 || out_cap > kBoundBytes) {
+    SBWT_CUDA(cudaMemcpyAsync(ws.host, off, 8, cudaMemcpyDeviceToHost, st));
+    SBWT_CUDA(cudaMemcpyAsync(ws.host + 1, off + n_reads, 8, cudaMemcpyDeviceToHost, st));
+    SBWT_CUDA(cudaStreamSynchronize(st));
+    max_n = ws.host[1] - ws.host[0];
+  }
+  return format_tokens(tok, max_n, off, n_reads, out, out_cap, need, ws, st);
 }
 
 // Device-resident index results -> formatted bytes (returns the byte count;
@@ -368,24 +782,16 @@ u64 format_index_device(const uint64_t *res, const uint64_t *ends, u64 n_reads, 
   uint64_t *koff = ws.kmer_off.get<uint64_t>();
   kmer_counts_kernel<<<(unsigned)std::min<u64>((n_reads + 255) / 256, 148 * 16), 256, 0, st>>>(
       ends, n_reads, k, koff);
-  const u64 n_kmers = scan_inplace(koff, n_reads, ws, st);
-  u64 bytes = 0;
   if (format == 0) {
-    ws.byte_off.ensure((n_reads + 1) * 8);
-    uint64_t *boff = ws.byte_off.get<uint64_t>();
-    index_lengths_kernel<<<warp_grid(n_reads), 256, 0, st>>>(res, ends, n_reads, k, koff, boff);
-    bytes = scan_inplace(boff, n_reads, ws, st);
-    if (need) *need = bytes;
-    if (bytes > out_cap) throw Error(SBWT_E_CAPACITY, "output capacity too small");
-    index_ascii_kernel<<<warp_grid(n_reads), 256, 0, st>>>(res, ends, n_reads, k, koff, boff,
-                                                            out);
-  } else {
-    bytes = format == 1 ? 8 * (n_kmers + n_reads) : n_kmers + n_reads;
-    if (need) *need = bytes;
-    if (bytes > out_cap) throw Error(SBWT_E_CAPACITY, "output capacity too small");
-    index_fixed_kernel<<<warp_grid(n_reads), 256, 0, st>>>(res, ends, n_reads, k, koff, format,
-                                                            out);
+    enqueue_scan(koff, n_reads, ws, st);
+    return format_ascii(res, koff, n_reads, out, out_cap, need, ws, st);
   }
+  const u64 n_kmers = scan_inplace(koff, n_reads, ws, st);
+  const u64 bytes = format == 1 ? 8 * (n_kmers + n_reads) : n_kmers + n_reads;
+  if (need) *need = bytes;
+  if (bytes > out_cap) throw Error(SBWT_E_CAPACITY, "output capacity too small");
+  index_fixed_kernel<<<warp_grid(n_reads), 256, 0, st>>>(res, ends, n_reads, k, koff, format,
+                                                          out);
   SBWT_CUDA(cudaGetLastError());
   return bytes;
 }
@@ -396,13 +802,7 @@ u64 format_colors_device(const uint32_t *ids, const uint64_t *ids_off, u64 n_rea
   if (n_reads == 0) return 0;
   u64 bytes = 0;
   if (format == 0) {
-    ws.byte_off.ensure((n_reads + 1) * 8);
-    uint64_t *boff = ws.byte_off.get<uint64_t>();
-    color_lengths_kernel<<<warp_grid(n_reads), 256, 0, st>>>(ids, ids_off, n_reads, boff);
-    bytes = scan_inplace(boff, n_reads, ws, st);
-    if (need) *need = bytes;
-    if (bytes > out_cap) throw Error(SBWT_E_CAPACITY, "output capacity too small");
-    color_ascii_kernel<<<warp_grid(n_reads), 256, 0, st>>>(ids, ids_off, n_reads, boff, out);
+    bytes = format_ascii(ids, ids_off, n_reads, out, out_cap, need, ws, st);
   } else if (format == 1) {
     u64 n_ids = 0;
     SBWT_CUDA(cudaMemcpyAsync(&n_ids, ids_off + n_reads, 8, cudaMemcpyDeviceToHost, st));

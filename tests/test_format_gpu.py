@@ -109,3 +109,67 @@ def test_device_buffers_and_capacity():
                                         S.DEVICE_POINTERS, 0, st))
     assert d_out.cpu().numpy().tobytes() == exp
     assert S.format_index_results(np.zeros(0, np.uint64), np.zeros(0, np.uint64), 31, 0) == b""
+
+
+def _edge_values(rng, n, top):
+    v = rng.integers(0, top, n, dtype=np.uint64)
+    edges = [10 ** i + d for i in range(1, 20) for d in (-1, 0, 1)] + \
+        [2 ** i + d for i in range(1, 40) for d in (-1, 0)]
+    edges = np.array([e for e in edges if e < top], np.uint64)
+    at = rng.random(n) < 0.5
+    v[at] = rng.choice(edges, int(at.sum()))
+    return v
+
+
+@pytest.mark.parametrize("n_tokens", [0, 1, 2047, 2048, 2049, 4096, 9001])
+@pytest.mark.parametrize("empty", [0, 3, 20_000])
+@pytest.mark.parametrize("kind", ["index", "index_wide", "colors"])
+def test_ascii_tiles_match_host_writer(n_tokens, empty, kind):
+    """Token counts at the edges of tiles, reads that end on them, no or many
+    empty reads before, between and after the others, digits of every length,
+    and outputs and inputs at every alignment."""
+    import torch
+    rng = np.random.default_rng(n_tokens + empty)
+    cuts = np.unique(np.concatenate([rng.integers(0, n_tokens + 1, 40), [0, n_tokens],
+                                     np.arange(0, n_tokens, 2048)]))
+    sizes = np.diff(cuts)
+    where = np.concatenate([[0, len(sizes)], rng.integers(0, len(sizes) + 1, 2)])
+    lines = list(sizes)
+    for w in sorted(where)[::-1]:
+        lines[w:w] = [0] * (empty // 4 + (empty > 0))
+    lines = np.array(lines, np.int64)
+    k = 5
+    if kind == "colors":
+        vals = _edge_values(rng, n_tokens, 1 << 32).astype(np.uint32)
+        offs = np.concatenate([[0], np.cumsum(lines)]).astype(np.uint64)
+        exp = host_color_bytes(vals, offs, 100, 0, "tiles_c")
+    else:
+        vals = _edge_values(rng, n_tokens, 1 << (32 if kind == "index" else 63))
+        vals[rng.random(n_tokens) < 0.1] = O.NOT_FOUND
+        vals[rng.random(n_tokens) < 0.1] = O.INVALID
+        ends = np.cumsum(np.where(lines > 0, lines + k - 1, rng.integers(0, k, len(lines))))
+        ends = ends.astype(np.uint64)
+        exp = host_index_bytes(vals, ends, k, 0, "tiles_i")
+    L, nb = S.lib(), C.c_uint64()
+    for shift in range(0, 16, 5):
+        lead = shift % 2  # tokens on and off a 16-byte boundary
+        pad = np.concatenate([np.zeros(lead, vals.dtype), vals])
+        d_v = torch.from_numpy(pad.view(np.int64 if vals.itemsize == 8 else np.int32)).cuda()
+        out = torch.full((shift + len(exp) + 16,), 7, dtype=torch.uint8, device="cuda")
+        torch.cuda.synchronize()
+        if kind == "colors":  # offsets that do not start at 0
+            d_o = torch.from_numpy((offs + np.uint64(lead)).view(np.int64)).cuda()
+            torch.cuda.synchronize()
+            rc = L.sbwt_format_color_results(d_v.data_ptr(), d_o.data_ptr(), len(lines), 100, 0,
+                                             out.data_ptr() + shift, len(exp), C.byref(nb),
+                                             S.DEVICE_POINTERS, 0, None)
+        else:
+            d_e = torch.from_numpy(ends.view(np.int64)).cuda()
+            torch.cuda.synchronize()
+            rc = L.sbwt_format_index_results(d_v.data_ptr() + 8 * lead, d_e.data_ptr(),
+                                             len(lines), k, 0, out.data_ptr() + shift, len(exp),
+                                             C.byref(nb), S.DEVICE_POINTERS, 0, None)
+        assert rc == S.OK and nb.value == len(exp)
+        h = out.cpu().numpy()
+        assert h[shift:shift + len(exp)].tobytes() == exp
+        assert (h[:shift] == 7).all() and (h[shift + len(exp):] == 7).all()
