@@ -83,3 +83,49 @@ def test_device_pointers_and_capacity():
                                S.DEVICE_POINTERS, 0, torch.cuda.current_stream().cuda_stream))
     assert d_chars[:nc.value].cpu().numpy().tobytes() == hc.tobytes()
     assert d_ends.cpu().numpy().view(np.uint64).tolist() == he.tolist()
+
+
+def _layout(kind: str, n: int) -> bytes:
+    rng = np.random.default_rng(n)
+    base = np.frombuffer(b"ACGTN", np.uint8)
+
+    def seq(m):
+        return bytes(rng.choice(base, m))
+
+    if kind == "fastq":  # four lines a record: chunks start on records
+        return b"".join(b"@r\n%s\n+\n%s\n" % (s, b"@" * len(s))
+                        for s in (seq(int(rng.integers(1, 300))) for _ in range(n)))
+    if kind == "one_char_lines":  # hundreds of lines in 512 output bytes
+        return b">x\n" + b"".join(seq(1) + b"\n" for _ in range(n)) + b">y\r\n" + seq(n) + b"\r\n"
+    if kind == "one_line":
+        return b">x\n" + seq(n)
+    return b"".join(b">%d\n%s\n\n" % (i, b"\r\n".join(seq(w) for w in (1, 15, 16, 17, i % 70 + 1)))
+                    for i in range(n))
+
+
+@pytest.mark.parametrize("kind", ["fastq", "one_char_lines", "one_line", "wrapped"])
+@pytest.mark.parametrize("n", [1, 7, 8, 9, 700, 40_000])
+def test_layouts_at_every_alignment(kind, n, tmp_path):
+    """Texts and outputs at any place in a 16-byte line, lines from one char to
+    the whole text, chunks entered searching and inside a sequence; nothing is
+    written around the outputs."""
+    import torch
+    text = _layout(kind, n)
+    hc, he = host_fastx(text, tmp_path / "in.fx")
+    L, nc, nr = S.lib(), C.c_uint64(), C.c_uint64()
+    for a, b in ((0, 0), (1, 15), (7, 8), (15, 1)):
+        buf = np.full(a + len(text) + 16, ord("\n"), np.uint8)
+        buf[a:a + len(text)] = np.frombuffer(text, np.uint8)
+        d_text = torch.from_numpy(buf).cuda()
+        d_chars = torch.full((b + len(hc) + 16,), 7, dtype=torch.uint8, device="cuda")
+        d_ends = torch.full((len(he) + 1,), -7, dtype=torch.int64, device="cuda")
+        torch.cuda.synchronize()
+        S.check(L.sbwt_fastx_parse(d_text.data_ptr() + a, len(text), d_chars.data_ptr() + b,
+                                   len(hc), d_ends.data_ptr(), len(he), C.byref(nc),
+                                   C.byref(nr), S.DEVICE_POINTERS, 0, None))
+        assert (nc.value, nr.value) == (len(hc), len(he))
+        out = d_chars.cpu().numpy()
+        assert out[b:b + len(hc)].tobytes() == hc
+        assert (out[:b] == 7).all() and (out[b + len(hc):] == 7).all()
+        ends = d_ends.cpu().numpy()
+        assert ends[:-1].tolist() == he.tolist() and ends[-1] == -7
