@@ -169,18 +169,33 @@ __global__ void pack16_kernel(const char *__restrict__ chars, uint64_t n,
   }
 }
 
+// Codes (first char on top) and invalid bits of 4 chars, as pack_4chars gives
+// them except that an invalid char's code is whatever its bits say: no kernel
+// that reads entries looks at it.  The letter that a code stands for comes from
+// a byte permute of "ACGT" and is compared with the char in either case.
+__device__ __forceinline__ void pack_entry4(uint32_t x, uint32_t &codes8, uint32_t &inv4) {
+  const uint32_t c = ((x >> 1) ^ (x >> 2)) & 0x03030303u;
+  codes8 = (c * 0x40100401u) >> 24;
+  const uint32_t sel = __byte_perm(c | c >> 4, 0, 0x4420);  // one nibble per char
+  const uint32_t t = (x & 0xDFDFDFDFu) ^ __byte_perm(0x54474341u, 0, sel);
+  const uint32_t bad = (((t & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | t) & 0x80808080u;
+  inv4 = ((bad >> 7) * 0x10204080u) >> 28;
+}
+
 // Packing into interleaved entries (32 chars and their invalid bits in 16
-// bytes; two empty entries past the end).  A lane packs 16 consecutive chars
-// and stores half an entry, so loads and stores are whole lines: 2-bit codes
-// and bits of 16 chars come from one 16-byte load.  ALIGNED: chars are 16-byte
-// aligned, else they are read byte by byte.
+// bytes; two empty entries past the end), halves [h0, h0 + step, ...).  A lane
+// packs 16 consecutive chars and stores half an entry, so loads and stores are
+// whole lines.  ALIGNED: chars are 16-byte aligned, else they are read byte by
+// byte.  All lanes of a warp take part (h0 is the warp's first half + lane).
+// Bound by DRAM: 510 M chars (and the block sums of 3 M reads) in 171 us, 4.5
+// TB/s; 339 us with the byte compares of pack_4chars.
 template <bool ALIGNED>
-__global__ void pack_entries_kernel(const char *__restrict__ chars, uint64_t n,
-                                    uint2 *__restrict__ halves, uint64_t n_words) {
-  const uint64_t step = (uint64_t)gridDim.x * blockDim.x, n_half = 2 * (n_words + 2);
+__device__ __forceinline__ void pack_entries(const char *__restrict__ chars, uint64_t n,
+                                             uint2 *__restrict__ halves, uint64_t n_words,
+                                             uint64_t h0, uint64_t step) {
+  const uint64_t n_half = 2 * (n_words + 2);
   constexpr int U = 4;  // loads in flight per thread
-  for (uint64_t h0 = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; h0 < ((n_half + 31) & ~31ULL);
-       h0 += U * step) {
+  for (; h0 < ((n_half + 31) & ~31ULL); h0 += U * step) {
     uint4 x[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
@@ -201,10 +216,10 @@ __global__ void pack_entries_kernel(const char *__restrict__ chars, uint64_t n,
     for (int u = 0; u < U; ++u) {
       const uint64_t h = h0 + u * step;
       uint32_t c[4], b[4];
-      pack_4chars(x[u].x, c[0], b[0]);
-      pack_4chars(x[u].y, c[1], b[1]);
-      pack_4chars(x[u].z, c[2], b[2]);
-      pack_4chars(x[u].w, c[3], b[3]);
+      pack_entry4(x[u].x, c[0], b[0]);
+      pack_entry4(x[u].y, c[1], b[1]);
+      pack_entry4(x[u].z, c[2], b[2]);
+      pack_entry4(x[u].w, c[3], b[3]);
       const uint32_t codes = c[0] << 24 | c[1] << 16 | c[2] << 8 | c[3];
       const uint32_t bits = b[0] | b[1] << 4 | b[2] << 8 | b[3] << 12;
       // even lane: the entry's 64 code bits; odd lane: its 32 invalid bits
@@ -217,16 +232,12 @@ __global__ void pack_entries_kernel(const char *__restrict__ chars, uint64_t n,
 }
 
 // --- exclusive scan of per-read k-mer counts -> kmer_off[0..n_reads] ---------
+// 1024 reads per block: with 4096, 5,003 reads of 90 tiles each were two
+// blocks' work (160 us).
 constexpr int kScanThreads = 256;
-constexpr int kScanItems = 16;
+constexpr int kScanItems = 4;
 constexpr uint64_t kScanTile = (uint64_t)kScanThreads * kScanItems;
-
-__device__ __forceinline__ uint64_t read_kmers(const uint64_t *ends, uint64_t r,
-                                               uint64_t base, uint32_t k) {
-  const uint64_t st = r ? ends[r - 1] : base;
-  const uint64_t len = ends[r] - st;
-  return len >= k ? len - k + 1 : 0;
-}
+static_assert(kScanTile == kReadsPerScanBlock, "scratch size");
 
 template <class T>
 __device__ __forceinline__ T block_exclusive_scan(T v, T *total) {
@@ -256,69 +267,175 @@ __device__ __forceinline__ T block_exclusive_scan(T v, T *total) {
   return warp_prefix + x - v;
 }
 
-__global__ void scan_reduce_kernel(const uint64_t *ends, uint64_t n_reads,
-                                   uint64_t base, uint32_t k, uint64_t n_chars,
-                                   uint64_t *block_sums, uint32_t *err) {
-  const uint64_t t0 = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
-  uint64_t s = 0;
-  for (int i = 0; i < kScanItems; ++i)
-    if (t0 + i < n_reads) {
-      const uint64_t r = t0 + i;
-      const uint64_t st = r ? ends[r - 1] : base;
-      if (ends[r] < st || ends[r] - base > n_chars) atomicOr(err, 4u);
-      s += read_kmers(ends, r, base, k);
-    }
-  uint64_t total;
-  block_exclusive_scan<uint64_t>(s, &total);
-  if (threadIdx.x == 0) block_sums[blockIdx.x] = total;
-}
+// What the search kernels need of a read batch: k-mer offsets, the tile table
+// and the packed chars.
+struct PrepareJob {
+  const uint64_t *ends;
+  uint64_t n_reads, base;
+  uint32_t k;
+  uint64_t n_chars;
+  uint64_t *block_sums;      // k-mers of each scan block (n_blocks > 1)
+  uint64_t n_blocks;         // scan blocks of kScanTile reads
+  uint64_t *kmer_off;        // n_reads + 1
+  uint64_t *total;
+  uint32_t *err;             // bit 4: bad read ends
+  unsigned long long *queue; // zeroed
+  // tile table: tile_read[t] = the read holding k-mer slot t * tile, with the
+  // char of that k-mer in the high half when with_pos
+  uint64_t tile;
+  uint32_t with_pos;
+  uint64_t *tile_read;
+  // packing into entries (halves == nullptr: not here)
+  const char *chars;
+  uint2 *halves;
+  uint64_t n_words;
+};
 
-// A batch whose read ends failed the check (err bit 4) gets a total of 0 and
-// all-zero k-mer offsets: the launches queued after the scan then do nothing
-// (no host round trip is needed before them).
-__global__ void scan_sums_kernel(uint64_t *block_sums, uint64_t n_blocks,
-                                 uint64_t *grand_total, const uint32_t *err) {
-  __shared__ uint64_t carry;
-  if (threadIdx.x == 0) carry = 0;
-  __syncthreads();
-  for (uint64_t b0 = 0; b0 < n_blocks; b0 += kScanThreads) {
-    const uint64_t b = b0 + threadIdx.x;
-    uint64_t v = b < n_blocks ? block_sums[b] : 0;
-    uint64_t total;
-    uint64_t ex = block_exclusive_scan<uint64_t>(v, &total);
-    if (b < n_blocks) block_sums[b] = carry + ex;
-    __syncthreads();
-    if (threadIdx.x == 0) carry += total;
-    __syncthreads();
+// k-mers of the reads of one warp's kScanItems rows of 32 (row q: reads r0 +
+// 32 q + lane): cnt[q] of this lane's read, st[q] its first char.  Checks the
+// ends.  Rows are whole lines of loads.
+template <class C>
+__device__ __forceinline__ bool rows_of_kmers(const PrepareJob &j, uint64_t r0,
+                                              C (&cnt)[kScanItems], C (&st)[kScanItems]) {
+  const uint32_t lane = threadIdx.x & 31;
+  uint64_t e[kScanItems];
+#pragma unroll
+  for (int q = 0; q < kScanItems; ++q) {
+    const uint64_t r = r0 + 32 * q + lane;
+    e[q] = r < j.n_reads ? __ldg(j.ends + r) : 0;
   }
-  if (threadIdx.x == 0) *grand_total = (*err & 4u) ? 0 : carry;
+  uint64_t before = r0 && r0 <= j.n_reads ? __ldg(j.ends + r0 - 1) : j.base;
+  bool bad = false;
+#pragma unroll
+  for (int q = 0; q < kScanItems; ++q) {
+    const uint64_t up = __shfl_up_sync(0xFFFFFFFFu, e[q], 1);
+    const uint64_t s = lane ? up : before;
+    const bool in = r0 + 32 * q + lane < j.n_reads;
+    bad |= in && (e[q] < s || e[q] - j.base > j.n_chars);
+    const uint64_t len = e[q] - s;
+    cnt[q] = in && len >= j.k ? (C)(len - j.k + 1) : 0;
+    st[q] = (C)(s - j.base);
+    before = __shfl_sync(0xFFFFFFFFu, e[q], 31);
+  }
+  return bad;
 }
 
-__global__ void scan_write_kernel(const uint64_t *ends, uint64_t n_reads,
-                                  uint64_t base, uint32_t k,
-                                  const uint64_t *block_sums, uint64_t *kmer_off,
-                                  const uint32_t *err) {
-  const uint64_t t0 = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
-  if (*err & 4u) {  // the same word for every thread: a uniform return
-    for (int i = 0; i < kScanItems; ++i) {
-      if (t0 + i < n_reads) kmer_off[t0 + i] = 0;
-      if (t0 + i == n_reads - 1) kmer_off[n_reads] = 0;
+// One warp's part of the offsets and the tile table: its reads' k-mers start
+// at slot `at`.
+template <class C>
+__device__ __forceinline__ void write_rows(const PrepareJob &j, uint64_t r0, uint64_t at,
+                                           const C (&cnt)[kScanItems], const C (&st)[kScanItems]) {
+  const uint32_t lane = threadIdx.x & 31;
+  const C tile = (C)j.tile;
+#pragma unroll
+  for (int q = 0; q < kScanItems; ++q) {
+    const uint64_t r = r0 + 32 * q + lane;
+    if (r0 + 32 * q >= j.n_reads) break;  // the same for the whole warp
+    C x = cnt[q];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const C y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+      if (lane >= (uint32_t)o) x += y;
+    }
+    const C row = __shfl_sync(0xFFFFFFFFu, x, 31);
+    const uint64_t a = at + (x - cnt[q]);
+    if (r < j.n_reads) j.kmer_off[r] = a;
+    if (r == j.n_reads - 1) j.kmer_off[j.n_reads] = a + cnt[q];
+    // tiles that start in this read: a few by its thread, more by the warp
+    C t = 0, t_end = 0;
+    uint64_t entry = r;
+    if (cnt[q]) {
+      t = ((C)a + tile - 1) / tile;
+      t_end = ((C)a + cnt[q] + tile - 1) / tile;
+      if (j.with_pos) entry |= ((uint64_t)st[q] - a) << 32;  // the char at slot 0, mod 2^32
+    }
+    const uint64_t up = j.with_pos ? j.tile << 32 : 0;
+    if (t_end - t <= 16)
+      for (; t < t_end; ++t) j.tile_read[t] = entry + t * up;
+    for (unsigned m = __ballot_sync(0xFFFFFFFFu, t < t_end); m; m &= m - 1) {
+      const int o = __ffs(m) - 1;
+      const C o_end = __shfl_sync(0xFFFFFFFFu, t_end, o);
+      const uint64_t o_entry = __shfl_sync(0xFFFFFFFFu, entry, o);
+      for (C i = __shfl_sync(0xFFFFFFFFu, t, o) + lane; i < o_end; i += 32)
+        j.tile_read[i] = o_entry + i * up;
+    }
+    at += row;
+  }
+}
+
+// First launch: a block per kScanTile reads sums its k-mers and checks its
+// read ends (a batch of one such block is finished here), the blocks after
+// them pack the chars.  C: u32 for batches of fewer than 2^32 chars.
+// A batch whose read ends fail the check (err bit 4) gets a total of 0 and
+// all-zero k-mer offsets: the launches queued after it then do nothing (no
+// host round trip is needed before them).
+template <class C, bool ALIGNED>
+__global__ void __launch_bounds__(kScanThreads) prepare_kernel(PrepareJob j) {
+  if (blockIdx.x >= j.n_blocks) {
+    const uint64_t step = (uint64_t)(gridDim.x - j.n_blocks) * blockDim.x;
+    pack_entries<ALIGNED>(j.chars, j.n_chars, j.halves, j.n_words,
+                          (blockIdx.x - j.n_blocks) * (uint64_t)blockDim.x + threadIdx.x, step);
+    return;
+  }
+  const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const uint64_t r0 = blockIdx.x * kScanTile + wid * (32ULL * kScanItems);
+  C cnt[kScanItems], st[kScanItems];
+  const bool bad = rows_of_kmers(j, r0, cnt, st);
+  if (blockIdx.x == 0 && threadIdx.x == 0) *j.queue = 0;
+  uint64_t s = 0;
+#pragma unroll
+  for (int q = 0; q < kScanItems; ++q) s += cnt[q];
+#pragma unroll
+  for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
+  uint64_t total;
+  const uint64_t at = block_exclusive_scan<uint64_t>(lane == 0 ? s : 0, &total);
+  if (j.n_blocks > 1) {
+    if (bad) atomicOr(j.err, 4u);
+    if (threadIdx.x == 0) j.block_sums[blockIdx.x] = total;
+    return;
+  }
+  if (__syncthreads_or(bad)) {
+    for (uint64_t r = threadIdx.x; r <= j.n_reads; r += kScanThreads) j.kmer_off[r] = 0;
+    if (threadIdx.x == 0) {
+      *j.total = 0;
+      atomicOr(j.err, 4u);
     }
     return;
   }
-  uint64_t v[kScanItems];
+  if (threadIdx.x == 0) *j.total = total;
+  write_rows(j, r0, __shfl_sync(0xFFFFFFFFu, at, 0), cnt, st);
+}
+
+// Second launch, for more than one scan block: every block adds up the sums of
+// the blocks before it and writes its offsets and tiles.
+template <class C>
+__global__ void __launch_bounds__(kScanThreads) offsets_kernel(PrepareJob j) {
+  const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const uint64_t r0 = blockIdx.x * kScanTile + wid * (32ULL * kScanItems);
+  if (*j.err & 4u) {  // the same word for every thread: a uniform return
+    for (uint64_t r = blockIdx.x * kScanTile + threadIdx.x;
+         r < (blockIdx.x + 1) * kScanTile && r <= j.n_reads; r += kScanThreads)
+      j.kmer_off[r] = 0;
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
+      j.kmer_off[j.n_reads] = 0;
+      *j.total = 0;
+    }
+    return;
+  }
+  uint64_t sum = 0, before;
+  for (uint64_t b = threadIdx.x; b < blockIdx.x; b += kScanThreads) sum += __ldg(j.block_sums + b);
+  block_exclusive_scan<uint64_t>(sum, &before);
+  C cnt[kScanItems], st[kScanItems];
+  rows_of_kmers(j, r0, cnt, st);
   uint64_t s = 0;
-  for (int i = 0; i < kScanItems; ++i) {
-    v[i] = (t0 + i < n_reads) ? read_kmers(ends, t0 + i, base, k) : 0;
-    s += v[i];
-  }
+#pragma unroll
+  for (int q = 0; q < kScanItems; ++q) s += cnt[q];
+#pragma unroll
+  for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
   uint64_t total;
-  uint64_t ex = block_exclusive_scan<uint64_t>(s, &total) + block_sums[blockIdx.x];
-  for (int i = 0; i < kScanItems; ++i) {
-    if (t0 + i < n_reads) kmer_off[t0 + i] = ex;
-    if (t0 + i == n_reads - 1) kmer_off[n_reads] = ex + v[i];
-    ex += v[i];
-  }
+  const uint64_t at = block_exclusive_scan<uint64_t>(lane == 0 ? s : 0, &total);
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *j.total = before + total;
+  write_rows(j, r0, before + __shfl_sync(0xFFFFFFFFu, at, 0), cnt, st);
 }
 
 // --- search ------------------------------------------------------------------
@@ -511,39 +628,6 @@ __global__ void ends_upper_bound_kernel(const uint64_t *ends, uint64_t r0, uint6
   }
   out[0] = lo;
   out[1] = lo > r0 ? ends[lo - 1] : limit;
-}
-
-// First read of every work tile: tile_read[t] = the read holding k-mer slot
-// t * tile, with the char of that k-mer in the high half when with_pos.  One
-// thread per read (a read of more than a few tiles is shared by its warp);
-// reads without k-mers own no tile.
-__global__ void tile_reads_kernel(const uint64_t *kmer_off, const uint64_t *ends, uint64_t base,
-                                  uint64_t n_reads, uint64_t tile, uint32_t with_pos,
-                                  uint64_t *tile_read) {
-  const uint32_t lane = threadIdx.x & 31;
-  const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t r0 = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) & ~31ULL; r0 < n_reads;
-       r0 += step) {
-    const uint64_t r = r0 + lane;
-    uint64_t t = 0, t_end = 0, entry = 0;
-    if (r < n_reads) {
-      const uint64_t a = kmer_off[r], b = kmer_off[r + 1];
-      t = (a + tile - 1) / tile;
-      t_end = (b + tile - 1) / tile;
-      entry = r;
-      if (with_pos && t < t_end)  // the char at slot 0, modulo 2^32
-        entry |= ((r ? ends[r - 1] : base) - base - a) << 32;
-    }
-    const uint64_t up = with_pos ? tile << 32 : 0;
-    for (uint32_t i = 0; i < 32 && t < t_end; ++i, ++t) tile_read[t] = entry + t * up;
-    for (unsigned m = __ballot_sync(0xFFFFFFFFu, t < t_end); m; m &= m - 1) {
-      const int q = __ffs(m) - 1;
-      const uint64_t q_end = __shfl_sync(0xFFFFFFFFu, t_end, q);
-      const uint64_t q_entry = __shfl_sync(0xFFFFFFFFu, entry, q);
-      for (uint64_t x = __shfl_sync(0xFFFFFFFFu, t, q) + lane; x < q_end; x += 32)
-        tile_read[x] = q_entry + x * up;
-    }
-  }
 }
 
 // Fused index step over reads.
@@ -2812,14 +2896,16 @@ static Workspace &workspace(int device) {
       SBWT_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
     for (auto &e : p->done) SBWT_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     SBWT_CUDA(cudaMallocHost(&p->err_host, 16));
-    p->err_dev.resize(sizeof(uint32_t));
-    SBWT_CUDA(cudaMemset(p->err_dev.get(), 0, sizeof(uint32_t)));
+    p->err_dev.resize(16);  // the error word, then (at +8 bytes) the k-mer count of slot 0
+    SBWT_CUDA(cudaMemset(p->err_dev.get(), 0, 16));
   }
   return *p;
 }
 
+// Waits for the stream; the error word (turned into an exception) and slot 0's
+// k-mer count come back in one copy.
 static void check_err_word(Workspace &ws, cudaStream_t st) {
-  SBWT_CUDA(cudaMemcpyAsync(ws.err_host, ws.err_dev.get(), 4, cudaMemcpyDeviceToHost, st));
+  SBWT_CUDA(cudaMemcpyAsync(ws.err_host, ws.err_dev.get(), 16, cudaMemcpyDeviceToHost, st));
   SBWT_CUDA(cudaStreamSynchronize(st));
   const uint32_t e = *ws.err_host;
   if (e) {
@@ -2888,53 +2974,80 @@ static u64 tile_size(int device, u64 n_kmers, const LaunchConfig &cfg, bool path
   return (std::min<u64>(std::max<u64>(tile, 16), 128) + 15) & ~15ULL;
 }
 
-// Scan of per-read k-mer counts and the packing of the chars (device-resident
-// inputs).  The k-mer total lands in *sc.total.
-// entries: packed as interleaved entries, for search_paths_kernel.
+// What a batch's preparation and search have to agree on.
+struct BatchPlan {
+  bool paths;  // search_paths_kernel runs: chars packed as entries
+  u64 tile;    // k-mer slots per tile
+};
+static BatchPlan plan_batch(const IndexImpl &ix, u64 n_chars, u64 n_reads, u64 n_kmers, u32 flags,
+                            const LaunchConfig &cfg) {
+  const bool paths = paths_kernel_applies(ix, reads_bound(n_chars, n_reads), flags, cfg);
+  return BatchPlan{paths, tile_size(ix.device, std::max<u64>(n_kmers, 1), cfg, paths)};
+}
+
+// Offsets, tile table and packed chars of a device-resident batch, with the
+// work queue zeroed.  The k-mer total lands in *sc.total.
+// Launches: one (up to kScanTile reads) or two, and the packing's own when it
+// is not into entries.  On 100 reads a launch each for the block sums, their
+// scan, the offsets, the packing, the queue and the tiles took 19 us of device
+// time, one launch 5 us; on 3 M reads the offsets and tiles took 100 us, now
+// 37 us.
 static void launch_prepare(int device, u32 k, const char *d_chars, u64 n_chars,
                            const u64 *d_ends, u64 n_reads, u64 base,
-                           const ReadsScratch &sc, bool entries, cudaStream_t st) {
+                           const ReadsScratch &sc, const BatchPlan &plan, cudaStream_t st) {
   const u64 n_words = (n_chars + 31) / 32;
-  const u64 n_scan_blocks = (n_reads + kScanTile - 1) / kScanTile;
-  scan_reduce_kernel<<<(unsigned)n_scan_blocks, kScanThreads, 0, st>>>(
-      d_ends, n_reads, base, k, n_chars, sc.block_sums, sc.err);
-  scan_sums_kernel<<<1, kScanThreads, 0, st>>>(sc.block_sums, n_scan_blocks, sc.total,
-                                               sc.err);
-  scan_write_kernel<<<(unsigned)n_scan_blocks, kScanThreads, 0, st>>>(
-      d_ends, n_reads, base, k, sc.block_sums, sc.kmer_off, sc.err);
-  if (entries) {
-    const int grid = grid_for(device, (2 * (n_words + 2) + 3) / 4, 256, 8);
-    if (((uintptr_t)d_chars & 15) == 0)
-      pack_entries_kernel<true><<<grid, 256, 0, st>>>(
-          d_chars, n_chars, reinterpret_cast<uint2 *>(sc.packed), n_words);
-    else
-      pack_entries_kernel<false><<<grid, 256, 0, st>>>(
-          d_chars, n_chars, reinterpret_cast<uint2 *>(sc.packed), n_words);
-    SBWT_CUDA(cudaGetLastError());
-    note_launches(4);
-    return;
+  PrepareJob j{};
+  j.ends = d_ends;
+  j.n_reads = n_reads;
+  j.base = base;
+  j.k = k;
+  j.n_chars = n_chars;
+  j.block_sums = sc.block_sums;
+  j.n_blocks = (n_reads + kScanTile - 1) / kScanTile;
+  j.kmer_off = sc.kmer_off;
+  j.total = sc.total;
+  j.err = sc.err;
+  j.queue = sc.queue;
+  j.tile = plan.tile;
+  j.with_pos = plan.paths;
+  j.tile_read = sc.tile_read;
+  j.chars = d_chars;
+  j.n_words = n_words;
+  u64 pack_blocks = 0;
+  if (plan.paths) {
+    j.halves = reinterpret_cast<uint2 *>(sc.packed);
+    pack_blocks = (u64)grid_for(device, (2 * (n_words + 2) + 3) / 4, 256, 8);
   }
+  const bool wide = n_chars >= (1ULL << 32) - 64, aligned = ((uintptr_t)d_chars & 15) == 0;
+  auto *const kernel = wide ? (aligned ? prepare_kernel<u64, true> : prepare_kernel<u64, false>)
+                            : (aligned ? prepare_kernel<u32, true> : prepare_kernel<u32, false>);
+  kernel<<<(unsigned)(j.n_blocks + pack_blocks), kScanThreads, 0, st>>>(j);
+  if (j.n_blocks > 1)
+    (wide ? offsets_kernel<u64> : offsets_kernel<u32>)<<<(unsigned)j.n_blocks, kScanThreads, 0,
+                                                         st>>>(j);
+  SBWT_CUDA(cudaGetLastError());
+  note_launches(j.n_blocks > 1 ? 2 : 1);
+  if (plan.paths) return;
   SBWT_CUDA(cudaMemsetAsync(sc.packed + n_words, 0, 16, st));
   SBWT_CUDA(cudaMemsetAsync(sc.invalid + n_words, 0, 8, st));
-  if (n_words && ((uintptr_t)d_chars & 15) == 0)
+  if (n_words && aligned)
     pack16_kernel<<<grid_for(device, (n_words + 1) / 2, 256, 8), 256, 0, st>>>(
         d_chars, n_chars, sc.packed, sc.invalid, n_words);
   else if (n_words)
     pack_kernel<<<grid_for(device, n_words * 32, 256, 32), 256, 0, st>>>(
         d_chars, n_chars, sc.packed, sc.invalid, n_words);
   SBWT_CUDA(cudaGetLastError());
-  note_launches(n_words ? 4 : 3);
+  note_launches(n_words ? 1 : 0);
 }
 
-// Tile table + the read search kernel over a prepared batch of n_kmers.
-// With d_total the kernels read the k-mer count from device memory (the
+// The read search kernel over a prepared batch of n_kmers.  With d_total the kernels read the k-mer count from device memory (the
 // scan's total) and n_kmers is only an upper bound, for the tiling.
 static void launch_search(const IndexImpl &ix, u64 n_chars, const u64 *d_ends, u64 n_reads,
                           u64 base,
                           u64 n_kmers, u64 *d_out, u64 out_capacity, u32 flags,
                           const LaunchConfig &cfg, const ReadsScratch &sc,
-                          cudaStream_t st, uint32_t *d_out32 = nullptr,
-                          const u64 *d_total = nullptr) {
+                          const BatchPlan &plan, cudaStream_t st, uint32_t *d_out32 = nullptr,
+                          const u64 *d_total = nullptr, bool instrument = true) {
   if (n_reads == 0 || n_kmers == 0) return;
   ReadsView rv{};
   rv.out32 = d_out32;
@@ -2947,19 +3060,13 @@ static void launch_search(const IndexImpl &ix, u64 n_chars, const u64 *d_ends, u
   rv.base = base;
   rv.n_reads = n_reads;
   rv.n_kmers = n_kmers;
-  const bool paths = paths_kernel_applies(ix, rv.n_kmers_bound, flags, cfg);
-  rv.tile = tile_size(ix.device, n_kmers, cfg, paths);
+  rv.tile = plan.tile;
   rv.n_tiles = (n_kmers + rv.tile - 1) / rv.tile;
   rv.out = d_out;
   rv.out_capacity = out_capacity;
   rv.probe_len = probe_length(ix.num_bits, ix.k, cfg);
   rv.n_kmers_dev = d_total;
   rv.queue = sc.queue;
-  SBWT_CUDA(cudaMemsetAsync(sc.queue, 0, 8, st));
-  tile_reads_kernel<<<grid_for(ix.device, n_reads, 256, 16), 256, 0, st>>>(
-      sc.kmer_off, d_ends, rv.base, n_reads, rv.tile, paths, sc.tile_read);
-  SBWT_CUDA(cudaGetLastError());
-  note_launches(1);
   const int threads = (int)cfg.block_threads;
   const int grid = grid_for(ix.device, rv.n_tiles, threads, cfg.blocks_per_sm);
   const SbwtView sv = ix.view_for(cfg.presearch_letters);
@@ -2980,7 +3087,7 @@ static void launch_search(const IndexImpl &ix, u64 n_chars, const u64 *d_ends, u
   launch_search_kernel(stream, sv, rv, sc.tile_read, mtk, sc.err, grid, threads, st,
                        persist ? search_attrs(ix.hot.get(), ix.window_bytes, persist)
                                : LaunchAttrs{},
-                       cfg.table_kernel);
+                       cfg.table_kernel, instrument);
 }
 
 // The index step of one device-resident batch without any host
@@ -2993,16 +3100,14 @@ void enqueue_index_step(const IndexImpl &ix, const char *d_chars, u64 n_chars,
                         u64 out_capacity, u64 max_kmers, u32 flags, const LaunchConfig &cfg,
                         cudaStream_t st) {
   SBWT_CUDA(cudaMemsetAsync(sc.err, 0, 4, st));
-  SBWT_CUDA(cudaMemsetAsync(sc.queue, 0, 8, st));
   if (n_reads == 0) {
     SBWT_CUDA(cudaMemsetAsync(sc.total, 0, 8, st));
     return;
   }
-  const u64 bound = reads_bound(n_chars, n_reads);
-  const bool paths = paths_kernel_applies(ix, bound, flags, cfg);
-  launch_prepare(ix.device, ix.k, d_chars, n_chars, d_ends, n_reads, 0, sc, paths, st);
+  const BatchPlan plan = plan_batch(ix, n_chars, n_reads, max_kmers, flags, cfg);
+  launch_prepare(ix.device, ix.k, d_chars, n_chars, d_ends, n_reads, 0, sc, plan, st);
   ReadsView rv{};
-  rv.n_kmers_bound = bound;
+  rv.n_kmers_bound = reads_bound(n_chars, n_reads);
   rv.packed = sc.packed;
   rv.entries = reinterpret_cast<const PathEntry *>(sc.packed);
   rv.invalid = sc.invalid;
@@ -3012,14 +3117,12 @@ void enqueue_index_step(const IndexImpl &ix, const char *d_chars, u64 n_chars,
   rv.n_reads = n_reads;
   rv.n_kmers = 0;
   rv.n_kmers_dev = sc.total;
-  rv.tile = tile_size(ix.device, std::max<u64>(max_kmers, 1), cfg, paths);
+  rv.tile = plan.tile;
   rv.n_tiles = 0;  // computed on the device from the total
   rv.out = d_out;
   rv.out_capacity = out_capacity;
   rv.probe_len = probe_length(ix.num_bits, ix.k, cfg);
   rv.queue = sc.queue;
-  tile_reads_kernel<<<grid_for(ix.device, n_reads, 256, 16), 256, 0, st>>>(
-      sc.kmer_off, d_ends, rv.base, n_reads, rv.tile, paths, sc.tile_read);
   const int grid = (int)((u64)sm_count(ix.device) * cfg.blocks_per_sm);
   const SbwtView sv = ix.view_for(cfg.presearch_letters);
   const bool stream = !(flags & SBWT_PER_KMER_WALK) && ix.view.suffix_group_starts;
@@ -3052,7 +3155,8 @@ static ReadsScratch scratch_for(Workspace &ws, int b, u64 n_chars, u64 n_reads,
   ws.queue[b].ensure(8);
   return ReadsScratch{ws.kmer_off[b].get<u64>(), ws.packed[b].get<u64>(),
                       ws.invalid[b].get<uint32_t>(), ws.block_sums[b].get<u64>(),
-                      ws.total[b].get<u64>(), ws.tile_read[b].get<u64>(),
+                      b == 0 ? ws.err_dev.get<u64>() + 1 : ws.total[b].get<u64>(),
+                      ws.tile_read[b].get<u64>(),
                       ws.err_dev.get<uint32_t>(),
                       ws.queue[b].get<unsigned long long>()};
 }
@@ -3095,16 +3199,14 @@ void IndexImpl::search_reads_device_pieces(const char *chars, u64 n_chars,
       throw Error(SBWT_E_INVALID, "read_ends are not non-decreasing within n_chars");
     const u64 nc = c1 - c0, nr = r1 - r0;
     const ReadsScratch sc = scratch_for(ws, 0, nc, nr, nc, tile_min(cfg));
-    launch_prepare(device, k, chars + c0, nc, read_ends + r0, nr, c0, sc,
-                   paths_kernel_applies(*this, reads_bound(nc, nr), flags, cfg), st);
-    u64 n_k = 0;
-    SBWT_CUDA(cudaMemcpyAsync(&n_k, sc.total, 8, cudaMemcpyDeviceToHost, st));
-    SBWT_CUDA(cudaStreamSynchronize(st));
+    const BatchPlan plan = plan_batch(*this, nc, nr, nc, flags, cfg);
+    launch_prepare(device, k, chars + c0, nc, read_ends + r0, nr, c0, sc, plan, st);
     check_err_word(ws, st);
+    const u64 n_k = reinterpret_cast<const u64 *>(ws.err_host)[1];
     if (k_acc + n_k > capacity) over = true;
     if (!over)
       launch_search(*this, nc, read_ends + r0, nr, c0, n_k, results + k_acc,
-                    capacity - k_acc, flags, cfg, sc, st);
+                    capacity - k_acc, flags, cfg, sc, plan, st);
     k_acc += n_k;
     r0 = r1;
     c0 = c1;
@@ -3151,15 +3253,12 @@ void IndexImpl::search_reads(const char *chars, u64 n_chars, const u64 *read_end
       // ends has a total of 0), tiles are sized for n_chars (>= the count),
       // and no kernel writes at or past `capacity`.  The count and the error
       // word come back under one synchronisation (check_err_word's).
-      launch_prepare(device, k, chars, n_chars, read_ends, n_reads, 0, sc,
-                     paths_kernel_applies(*this, reads_bound(n_chars, n_reads), flags, cfg),
-                     user_stream);
+      const BatchPlan plan = plan_batch(*this, n_chars, n_reads, n_chars, flags, cfg);
+      launch_prepare(device, k, chars, n_chars, read_ends, n_reads, 0, sc, plan, user_stream);
       launch_search(*this, n_chars, read_ends, n_reads, 0, n_chars, results, capacity, flags,
-                    cfg, sc, user_stream, nullptr, sc.total);
-      u64 *const total_host = reinterpret_cast<u64 *>(ws.err_host + 2);
-      SBWT_CUDA(cudaMemcpyAsync(total_host, sc.total, 8, cudaMemcpyDeviceToHost, user_stream));
+                    cfg, sc, plan, user_stream, nullptr, sc.total);
       check_err_word(ws, user_stream);
-      n_k = *total_host;
+      n_k = reinterpret_cast<const u64 *>(ws.err_host)[1];
       if (n_results) *n_results = n_k;
       if (n_k > capacity)
         throw Error(SBWT_E_CAPACITY, "results_capacity smaller than the k-mer count");
@@ -3231,12 +3330,13 @@ void IndexImpl::search_reads(const char *chars, u64 n_chars, const u64 *read_end
     SBWT_CUDA(cudaMemcpyAsync(ws.chars[b].get(), chars + c0, nc, cudaMemcpyHostToDevice, st));
     SBWT_CUDA(cudaMemcpyAsync(ws.ends[b].get(), read_ends + r0, nr * 8,
                               cudaMemcpyHostToDevice, st));
-    launch_prepare(device, k, ws.chars[b].get<char>(), nc, ws.ends[b].get<u64>(), nr, c0, sc,
-                   paths_kernel_applies(*this, reads_bound(nc, nr), flags, cfg), st);
+    const BatchPlan plan = plan_batch(*this, nc, nr, nk, flags, cfg);
+    launch_prepare(device, k, ws.chars[b].get<char>(), nc, ws.ends[b].get<u64>(), nr, c0, sc, plan,
+                   st);
     if (narrow) {
       uint32_t *stage = ws.staging(b, std::max<u64>(nk, 1));
       launch_search(*this, nc, ws.ends[b].get<u64>(), nr, c0, nk, nullptr, nk, flags, cfg, sc,
-                    st, ws.results32[b].get<uint32_t>());
+                    plan, st, ws.results32[b].get<uint32_t>());
       if (nk)
         SBWT_CUDA(cudaMemcpyAsync(stage, ws.results32[b].get(), nk * 4,
                                   cudaMemcpyDeviceToHost, st));
@@ -3249,7 +3349,7 @@ void IndexImpl::search_reads(const char *chars, u64 n_chars, const u64 *read_end
     } else {
       drain();
       launch_search(*this, nc, ws.ends[b].get<u64>(), nr, c0, nk, ws.results[b].get<u64>(), nk,
-                    flags, cfg, sc, st);
+                    flags, cfg, sc, plan, st);
       if (nk)
         SBWT_CUDA(cudaMemcpyAsync(results + kacc, ws.results[b].get(), nk * 8,
                                   cudaMemcpyDeviceToHost, st));
@@ -3395,54 +3495,29 @@ void IndexImpl::search_reads_noalloc(const char *d_chars, u64 n_chars, const u64
                   reinterpret_cast<u64 *>(base + kNoAllocOffTileRead),
                   reinterpret_cast<uint32_t *>(base + kNoAllocOffErr),
                   reinterpret_cast<unsigned long long *>(base + kNoAllocOffQueue)};
-  // the error word and the work-queue counter keep the last call's values:
-  // clear them first
-  SBWT_CUDA(cudaMemsetAsync(sc.err, 0, 4, st));
-  SBWT_CUDA(cudaMemsetAsync(sc.queue, 0, 8, st));
-  const bool paths = paths_kernel_applies(*this, reads_bound(n_chars, n_reads), flags, cfg_in);
-  u64 n_k = 0;
-  uint32_t err = 0;
-  if (n_reads) {
-    launch_prepare(device, k, d_chars, n_chars, d_ends, n_reads, 0, sc, paths, st);
-    SBWT_CUDA(cudaMemcpyAsync(&n_k, sc.total, 8, cudaMemcpyDeviceToHost, st));
-    SBWT_CUDA(cudaMemcpyAsync(&err, sc.err, 4, cudaMemcpyDeviceToHost, st));
-    SBWT_CUDA(cudaStreamSynchronize(st));
-    if (err) throw Error(SBWT_E_INVALID, "read_ends are not non-decreasing within n_chars");
-  }
-  if (n_results) *n_results = n_k;
-  if (n_k > capacity)
-    throw Error(SBWT_E_CAPACITY, "results_capacity smaller than the k-mer count");
-  if (n_k == 0) return;
   LaunchConfig cfg = cfg_in;  // the tile table is sized for tiles of >= 16
   if (cfg.tile && cfg.tile < kNoAllocTileMin) cfg.tile = kNoAllocTileMin;
-  ReadsView rv{};
-  rv.n_kmers_bound = reads_bound(n_chars, n_reads);
-  rv.packed = sc.packed;
-  rv.entries = reinterpret_cast<const PathEntry *>(sc.packed);
-  rv.invalid = sc.invalid;
-  rv.ends = d_ends;
-  rv.kmer_off = sc.kmer_off;
-  rv.base = 0;
-  rv.n_reads = n_reads;
-  rv.n_kmers = n_k;
-  rv.tile = tile_size(device, n_k, cfg, paths);
-  rv.n_tiles = (n_k + rv.tile - 1) / rv.tile;
-  rv.out = d_results;
-  rv.out_capacity = capacity;
-  rv.probe_len = probe_length(num_bits, k, cfg);
-  rv.queue = sc.queue;
-  tile_reads_kernel<<<grid_for(device, n_reads, 256, 16), 256, 0, st>>>(
-      sc.kmer_off, d_ends, 0, n_reads, rv.tile, paths, sc.tile_read);
-  const int grid = grid_for(device, rv.n_tiles, (int)cfg.block_threads, cfg.blocks_per_sm);
-  const SbwtView sv = view_for(cfg.presearch_letters);
-  const u32 mtk = (flags & SBWT_MOVE_TO_KEY_KMER) ? 1u : 0u;
-  const bool stream = !(flags & SBWT_PER_KMER_WALK) && view.suffix_group_starts;
-  // the same kernel choice as sbwt_search_reads, without the profiler
-  launch_search_kernel(stream, sv, rv, sc.tile_read, mtk, sc.err, grid,
-                       (int)cfg.block_threads, st, LaunchAttrs{}, cfg.table_kernel,
-                       /*instrument=*/false);
-  SBWT_CUDA(cudaMemcpyAsync(&err, sc.err, 4, cudaMemcpyDeviceToHost, st));
-  SBWT_CUDA(cudaStreamSynchronize(st));
+  cfg.l2_window = 0;
+  // the total and the error word, one after the other, keep the last call's
+  // values: clear them first
+  static_assert(kNoAllocOffErr == kNoAllocOffTotal + 8, "read back together");
+  u64 status[2] = {0, 0};  // the k-mer count, the error word
+  if (n_reads) {
+    SBWT_CUDA(cudaMemsetAsync(sc.total, 0, 16, st));
+    // all launches queued back to back, as in search_reads; the same kernel
+    // choice, without the profiler
+    const BatchPlan plan = plan_batch(*this, n_chars, n_reads, n_chars, flags, cfg);
+    launch_prepare(device, k, d_chars, n_chars, d_ends, n_reads, 0, sc, plan, st);
+    launch_search(*this, n_chars, d_ends, n_reads, 0, n_chars, d_results, capacity, flags, cfg, sc,
+                  plan, st, nullptr, sc.total, /*instrument=*/false);
+    SBWT_CUDA(cudaMemcpyAsync(status, sc.total, 16, cudaMemcpyDeviceToHost, st));
+    SBWT_CUDA(cudaStreamSynchronize(st));
+  }
+  const uint32_t err = (uint32_t)status[1];
+  if (err & 4u) throw Error(SBWT_E_INVALID, "read_ends are not non-decreasing within n_chars");
+  if (n_results) *n_results = status[0];
+  if (status[0] > capacity)
+    throw Error(SBWT_E_CAPACITY, "results_capacity smaller than the k-mer count");
   if (err)
     throw Error(SBWT_E_TIMEOUT,
                 "key k-mer walk did not reach a key k-mer (node without an outgoing "

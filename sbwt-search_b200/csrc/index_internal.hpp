@@ -93,13 +93,15 @@ struct IndexImpl {
 
 u64 count_kmers_host(const u64 *ends, u64 n_reads, u32 k, u64 base);
 
+constexpr u64 kReadsPerScanBlock = 1024;
+
 // Device scratch of one read batch: scan outputs, packed chars, invalid
 // bits, the tile table, the error word and the work-queue counter.
 struct ReadsScratch {
   u64 *kmer_off;      // n_reads + 1
   u64 *packed;        // n_words + 2
   uint32_t *invalid;  // n_words + 2
-  u64 *block_sums;    // ceil(n_reads / 4096) + 1
+  u64 *block_sums;    // ceil(n_reads / kReadsPerScanBlock) + 1
   u64 *total;         // 1
   u64 *tile_read;     // n_tiles + 2
   uint32_t *err;      // 1

@@ -68,7 +68,7 @@ struct PipelineImpl {
     kmer_off.resize((max_reads + 1) * 8);
     packed.resize((n_words + 2) * 16);  // words, or interleaved entries
     invalid.resize((n_words + 2) * 4);
-    block_sums.resize(((max_reads + 4095) / 4096 + 1) * 8);
+    block_sums.resize((max_reads / kReadsPerScanBlock + 2) * 8);
     total.resize(8);
     tile_read.resize((max_chars / index_tile_size(*ix, max_chars, cfg) + 2) * 8);
     err.resize(8);
@@ -320,7 +320,7 @@ struct ServerImpl {
   std::unique_ptr<PipelineImpl> fresh;  // built, not yet adopted (under mu)
 
   static double slot_size(const ColorsImpl *ci, u64 chars, u64 reads) {
-    const double per_char = 1 + 8 + 0.375 + 1.0 / 16 + 1;  // chars, results, packing, tiles
+    const double per_char = 1 + 8 + 0.625 + 1.0 / 16 + 1;  // chars, results, packing, tiles
     const double per_read = 8 * 2 + (ci ? (ci->num_colors / 8.0 + 4 + 8 + 64 * 4) : 0);
     return chars * per_char + reads * per_read;
   }
