@@ -48,7 +48,8 @@ struct IndexImpl {
   bool build_kmer_table();
   void drop_kmer_table();
   // path cover and L-mer filter of a table under construction
-  bool build_path_cover(const u64 *key, const u8 *alive, u64 n_kmers, DeviceBuffer &pos);
+  bool build_path_cover(const u64 *key, const u8 *alive, u64 n_kmers, u32 *pos, u8 *scratch,
+                        u64 scratch_bytes);
   void drop_path_cover();
   u64 held_bytes() const {  // device memory of the handle
     return presearch.size() + hot.size() + key_buf.size() + l0_all.size() + kmer_table.size() +

@@ -11,9 +11,12 @@
 // Labels are recovered from the SBWT itself: the last char of node v is the
 // c with C[c] <= v < C[c + 1] (node 0 is the root, all '$'), and its
 // predecessor (the node whose marked c-edge reaches v) is the
-// (v - C[c])-th set bit of vector c.  k rounds of "char, then predecessor"
-// over all nodes spell every label; a node whose chain reaches the root
-// within k chars is a dummy ($-padded) and is not a k-mer.
+// (v - C[c])-th set bit of vector c: the set bits of A, C, G and T, one vector
+// after the other, are the predecessors of the nodes 1, 2, ...  A node's last m
+// chars and the node m steps back give its last 2 m chars and the node 2 m
+// steps back with one look at that node's own, so a label takes about
+// 1.6 log2(k) passes over the nodes instead of k; a node whose chain reaches
+// the root within k chars is a dummy ($-padded) and is not a k-mer.
 //
 // Table: 2^m slots of 16 bytes (key, value), value = the node, with the k-mer's
 // position in the path cover (path_cover.cu) in the high half when the index
@@ -51,47 +54,76 @@ __device__ __forceinline__ uint64_t vec_word(const Block *blocks, uint64_t w) {
   return j == 0 ? b.w0 : (j == 1 ? b.w1 : b.w2);
 }
 
-__global__ void word_ones_kernel(const Block *blocks, uint64_t n_words, uint64_t *cnt) {
+// Set bits of each word of the four vectors, one vector after the other.
+__global__ void word_ones_kernel(SbwtView s, uint64_t n_words, uint64_t *cnt) {
   const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t w = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; w < n_words; w += step)
-    cnt[w] = __popcll(vec_word(blocks, w));
+  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < 4 * n_words; i += step)
+    cnt[i] = __popcll(vec_word(s.blocks[i / n_words], i % n_words));
 }
 
-// positions of the set bits of one vector, in order
-__global__ void ones_positions_kernel(const Block *blocks, uint64_t n_words,
-                                      const uint64_t *off, uint64_t *pos) {
+// prev[1 + i] = position of the i-th of these set bits (n nodes; prev[0] = 0).
+template <class I>
+__global__ void prev_kernel(SbwtView s, uint64_t n_words, const uint64_t *off, uint64_t n,
+                            I *prev) {
   const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t w = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; w < n_words; w += step) {
-    uint64_t m = vec_word(blocks, w), o = off[w];
-    while (m) {
-      pos[o++] = w * 64 + __ffsll((long long)m) - 1;
-      m &= m - 1;
+  const uint64_t i0 = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+  if (i0 == 0) prev[0] = 0;
+  for (uint64_t i = i0; i < 4 * n_words; i += step) {
+    const uint64_t w = i % n_words;
+    uint64_t m = vec_word(s.blocks[i / n_words], w), o = 1 + off[i];
+    for (; m && o < n; m &= m - 1) {
+      const uint64_t at = w * 64 + __ffsll((long long)m) - 1;
+      prev[o++] = at < n ? (I)at : 0;
     }
   }
 }
 
-struct LabelView {
-  const uint64_t *ones[4];
-  uint64_t c_map[5];
+// The last chars of a node (the last one in the low bits) and the node that
+// many steps back.
+template <class I>
+struct __align__(16) Back {
+  uint64_t chars;
+  I node;
 };
 
-// One round of label recovery: the char of cur[v] lands at bits 2t of key[v],
-// and cur[v] moves to its predecessor; a chain that reaches the root marks a
-// dummy (alive = 0).
-__global__ void label_round_kernel(LabelView lv, uint64_t n, uint32_t t, uint64_t *cur,
-                                   uint64_t *key, uint8_t *alive) {
+__device__ __forceinline__ uint64_t last_char(const SbwtView &s, uint64_t v) {
+  return (v >= s.c_map[1]) + (v >= s.c_map[2]) + (v >= s.c_map[3]);  // 0 for the root
+}
+
+template <class I>
+__global__ void back_one_kernel(SbwtView s, uint64_t n, const I *prev, Back<I> *out) {
+  const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
+  for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < n; v += step)
+    out[v] = Back<I>{last_char(s, v), prev[v]};
+}
+// m steps back -> 2 m steps back.
+template <class I>
+__global__ void back_double_kernel(uint64_t n, uint32_t m, const Back<I> *in, Back<I> *out) {
   const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < n; v += step) {
-    if (!alive[v]) continue;
-    const uint64_t x = t == 0 ? v : cur[v];
-    if (x == 0) {
-      alive[v] = 0;
-      continue;
-    }
-    uint32_t c = 0;
-    while (c < 3 && x >= lv.c_map[c + 1]) ++c;
-    key[v] = (t == 0 ? 0 : key[v]) | ((uint64_t)c << (2 * t));
-    cur[v] = lv.ones[c][x - lv.c_map[c]];
+    const Back<I> a = in[v], b = in[a.node];
+    out[v] = Back<I>{a.chars | b.chars << (2 * m), b.node};
+  }
+}
+// m steps back -> m + 1 steps back.
+template <class I>
+__global__ void back_next_kernel(SbwtView s, uint64_t n, uint32_t m, const I *prev,
+                                 Back<I> *back) {
+  const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
+  for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < n; v += step) {
+    const Back<I> a = back[v];
+    back[v] = Back<I>{a.chars | last_char(s, a.node) << (2 * m), prev[a.node]};
+  }
+}
+// k - 1 steps back -> the label and whether the node is a k-mer.
+template <class I>
+__global__ void label_kernel(SbwtView s, uint64_t n, uint32_t k, const Back<I> *back,
+                             uint64_t *key, uint8_t *alive) {
+  const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
+  for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < n; v += step) {
+    const Back<I> a = back[v];
+    key[v] = a.chars | last_char(s, a.node) << (2 * (k - 1));
+    alive[v] = a.node != 0;
   }
 }
 
@@ -147,49 +179,79 @@ unsigned grid_of(uint64_t n) {
 
 }  // namespace
 
+// Labels of all nodes; `prev` and the two arrays of n Back records are scratch,
+// key and alive lie in the one of the two that is returned last.
+template <class I>
+static void recover_labels(const SbwtView &s, u64 n, u32 k, I *prev, Back<I> *a, Back<I> *b,
+                           u64 **key, u8 **alive) {
+  const u64 nw = (n + 63) / 64;
+  u64 *const cnt = reinterpret_cast<u64 *>(b);  // 4 nw + 1 words, before b is used
+  DeviceBuffer tmp;
+  size_t tb = 0;
+  word_ones_kernel<<<grid_of(4 * nw), 256>>>(s, nw, cnt);
+  SBWT_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb, cnt, cnt, (int64_t)(4 * nw)));
+  tmp.resize(std::max<size_t>(tb, 1));
+  SBWT_CUDA(cub::DeviceScan::ExclusiveSum(tmp.get(), tb, cnt, cnt, (int64_t)(4 * nw)));
+  SBWT_CUDA(cudaMemsetAsync(prev, 0, n * sizeof(I)));  // should the vectors lack bits
+  prev_kernel<I><<<grid_of(4 * nw), 256>>>(s, nw, cnt, n, prev);
+  back_one_kernel<I><<<grid_of(n), 256>>>(s, n, prev, a);
+  // m from 1 to k - 1 by the bits of k - 1: double, and one more for a set bit
+  u32 m = 1;
+  int bit = 31 - __builtin_clz(k - 1);
+  for (--bit; bit >= 0; --bit) {
+    back_double_kernel<I><<<grid_of(n), 256>>>(n, m, a, b);
+    std::swap(a, b);
+    m *= 2;
+    if (((k - 1) >> bit) & 1u) {
+      back_next_kernel<I><<<grid_of(n), 256>>>(s, n, m, prev, a);
+      ++m;
+    }
+  }
+  *key = reinterpret_cast<u64 *>(b);
+  *alive = reinterpret_cast<u8 *>(*key + n);
+  label_kernel<I><<<grid_of(n), 256>>>(s, n, k, a, *key, *alive);
+  SBWT_CUDA(cudaGetLastError());
+  SBWT_CUDA(cudaDeviceSynchronize());  // tmp goes
+}
+
 // Builds the table from the index's rank blocks.  Returns false (and builds
-// nothing) when k > 31 or the table would not fit in kKmerTableMaxBytes or a
-// quarter of the free device memory.
+// nothing) when k > 31, when the vectors' set bits are not one per node (no
+// SBWT), or when the table would not fit in kKmerTableMaxBytes or a quarter of
+// the free device memory.
 bool IndexImpl::build_kmer_table() {
   DeviceGuard g(device);
   drop_kmer_table();
-  if (k > 31 || k < 2) return false;
-  const u64 n = num_bits, nw = (num_bits + 63) / 64;
-  // predecessor tables: positions of the ones of each vector
-  DeviceBuffer cnt((nw + 1) * 8), ones[4];
-  size_t tb = 0;
-  DeviceBuffer tmp;
-  LabelView lv{};
-  for (int c = 0; c < 5; ++c) lv.c_map[c] = c_map[c];
-  for (int c = 0; c < 4; ++c) {
-    const u64 total = c_map[c + 1] - c_map[c];
-    ones[c].resize(std::max<u64>(total, 1) * 8);
-    word_ones_kernel<<<grid_of(nw), 256>>>(view.blocks[c], nw, cnt.get<u64>());
-    SBWT_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb, cnt.get<u64>(), cnt.get<u64>(),
-                                            (int64_t)nw));
-    tmp.ensure(std::max<size_t>(tb, 1));
-    SBWT_CUDA(cub::DeviceScan::ExclusiveSum(tmp.get(), tb, cnt.get<u64>(), cnt.get<u64>(),
-                                            (int64_t)nw));
-    ones_positions_kernel<<<grid_of(nw), 256>>>(view.blocks[c], nw, cnt.get<u64>(),
-                                                ones[c].get<u64>());
-    SBWT_CUDA(cudaGetLastError());
-    lv.ones[c] = ones[c].get<u64>();
+  if (k > 31 || k < 2 || c_map[4] != num_bits) return false;
+  const u64 n = num_bits;
+  // one allocation: two arrays of 16-byte records, and the predecessors
+  const bool narrow = n < (1ULL << 32) - 1;
+  const u64 rec_bytes = (n * 16 + 4096 + 255) / 256 * 256;
+  DeviceBuffer arena;
+  try {
+    arena.resize(2 * rec_bytes + n * (narrow ? 4 : 8));
+  } catch (const Error &e) {
+    if (e.code != SBWT_E_OOM) throw;
+    cudaGetLastError();
+    return false;  // every search also works without the table
   }
-  cnt.release();
-  // labels
-  DeviceBuffer cur(n * 8), key(n * 8), alive(n);
-  SBWT_CUDA(cudaMemset(alive.get(), 1, n));
-  for (u32 t = 0; t < k; ++t)
-    label_round_kernel<<<grid_of(n), 256>>>(lv, n, t, cur.get<u64>(), key.get<u64>(),
-                                            alive.get<uint8_t>());
-  SBWT_CUDA(cudaGetLastError());
-  for (auto &o : ones) o.release();
-  cur.release();
+  u8 *const rec[2] = {arena.get<u8>(), arena.get<u8>() + rec_bytes};
+  u8 *const prev = arena.get<u8>() + 2 * rec_bytes;
+  u64 *key = nullptr;
+  u8 *alive = nullptr;
+  if (narrow)
+    recover_labels(view, n, k, reinterpret_cast<u32 *>(prev),
+                   reinterpret_cast<Back<u32> *>(rec[0]), reinterpret_cast<Back<u32> *>(rec[1]),
+                   &key, &alive);
+  else
+    recover_labels(view, n, k, reinterpret_cast<u64 *>(prev),
+                   reinterpret_cast<Back<u64> *>(rec[0]), reinterpret_cast<Back<u64> *>(rec[1]),
+                   &key, &alive);
+  // the record array that does not hold the labels is free from here on
+  u8 *const free_rec = reinterpret_cast<u8 *>(key) == rec[0] ? rec[1] : rec[0];
   // k-mer count -> table size (load <= 1/2)
-  DeviceBuffer d_n(8);
-  SBWT_CUDA(cudaMemset(d_n.get(), 0, 8));
-  count_alive_kernel<<<grid_of(n), 256>>>(alive.get<uint8_t>(), n,
-                                          d_n.get<unsigned long long>());
+  DeviceBuffer d_n(16);  // the count, an error word
+  SBWT_CUDA(cudaMemset(d_n.get(), 0, 16));
+  count_alive_kernel<<<grid_of(n), 256>>>(alive, n, d_n.get<unsigned long long>());
   SBWT_CUDA(cudaGetLastError());
   u64 n_kmers = 0;
   SBWT_CUDA(cudaMemcpy(&n_kmers, d_n.get(), 8, cudaMemcpyDeviceToHost));
@@ -203,25 +265,22 @@ bool IndexImpl::build_kmer_table() {
     return false;
   // the path cover first: the table's values hold its positions.  An index
   // that cannot have it (or no memory for it) keeps the table alone.
-  DeviceBuffer pos;
+  u32 *pos = reinterpret_cast<u32 *>(prev);  // the predecessors are done with
   try {
-    if (!build_path_cover(key.get<u64>(), alive.get<u8>(), n_kmers, pos)) pos.release();
+    if (!narrow || !build_path_cover(key, alive, n_kmers, pos, free_rec, rec_bytes)) pos = nullptr;
   } catch (const Error &e) {
     if (e.code != SBWT_E_OOM) throw;
     cudaGetLastError();
-    pos.release();
+    pos = nullptr;
     drop_path_cover();
   }
   kmer_table.resize(slots * 16);
   SBWT_CUDA(cudaMemset(kmer_table.get(), 0xFF, slots * 16));
-  DeviceBuffer d_err(4);
-  SBWT_CUDA(cudaMemset(d_err.get(), 0, 4));
-  table_insert_kernel<<<grid_of(n), 256>>>(key.get<u64>(), alive.get<uint8_t>(), n,
-                                           pos.get<u32>(), kmer_table.get<u64>(), slots - 1,
-                                           d_err.get<uint32_t>());
+  table_insert_kernel<<<grid_of(n), 256>>>(key, alive, n, pos, kmer_table.get<u64>(), slots - 1,
+                                           d_n.get<uint32_t>() + 2);
   SBWT_CUDA(cudaGetLastError());
   uint32_t e = 0;
-  SBWT_CUDA(cudaMemcpy(&e, d_err.get(), 4, cudaMemcpyDeviceToHost));
+  SBWT_CUDA(cudaMemcpy(&e, d_n.get<uint32_t>() + 2, 4, cudaMemcpyDeviceToHost));
   if (e) {
     kmer_table.release();
     drop_path_cover();
@@ -229,8 +288,7 @@ bool IndexImpl::build_kmer_table() {
   }
   kmer_filter.resize(filter_words * 8);
   SBWT_CUDA(cudaMemset(kmer_filter.get(), 0, filter_words * 8));
-  filter_insert_kernel<<<grid_of(n), 256>>>(key.get<u64>(), alive.get<uint8_t>(), n,
-                                            kmer_filter.get<unsigned long long>(),
+  filter_insert_kernel<<<grid_of(n), 256>>>(key, alive, n, kmer_filter.get<unsigned long long>(),
                                             filter_words);
   SBWT_CUDA(cudaGetLastError());
   view.kmer_table = kmer_table.get<u64>();

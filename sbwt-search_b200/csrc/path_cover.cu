@@ -322,10 +322,11 @@ uint32_t lmer_length(u64 n_kmers, u32 k) {
 
 // Builds the path cover and the L-mer filter from the labels of the k-mer
 // table's construction; pos[v] (u32 per node) receives each k-mer's position.
-// Returns false (and builds nothing) for SBWTs without suffix-group words, of
-// 64-bit nodes, or when device memory is short.
-bool IndexImpl::build_path_cover(const u64 *key, const u8 *alive, u64 n_kmers,
-                                 DeviceBuffer &pos_buf) {
+// scratch: at least 16 bytes per node.  Returns false (and builds nothing) for
+// SBWTs without suffix-group words, of 64-bit nodes, or when device memory is
+// short.
+bool IndexImpl::build_path_cover(const u64 *key, const u8 *alive, u64 n_kmers, u32 *pos,
+                                 u8 *scratch, u64 scratch_bytes) {
   const u64 n = num_bits;
   if (!view.suffix_group_starts || n >= (u64)kBlockBits << kSuperchunkShift || n_kmers == 0)
     return false;
@@ -334,95 +335,92 @@ bool IndexImpl::build_path_cover(const u64 *key, const u8 *alive, u64 n_kmers,
   const u64 lm_words = L ? std::max<u64>((n_kmers * kLmerFilterBits + 63) / 64, 1) : 0;
   size_t free_b = 0, total_b = 0;
   SBWT_CUDA(cudaMemGetInfo(&free_b, &total_b));
-  if (n * 25 + n_kmers * 4 + n_entries * 16 + lm_words * 8 > free_b / 2) return false;
+  if (n_kmers * 4 + n_entries * 16 + lm_words * 8 > free_b / 2) return false;
   const unsigned gn = grid_of(n);
 
-  DeviceBuffer nxt(n * 4), prv(n * 4), pair(n * 4), outd(n), ind(n);
-  SBWT_CUDA(cudaMemset(nxt.get(), 0xFF, n * 4));
-  SBWT_CUDA(cudaMemset(prv.get(), 0xFF, n * 4));
-  SBWT_CUDA(cudaMemset(outd.get(), 0, n));
-  SBWT_CUDA(cudaMemset(ind.get(), 0, n));
-  degrees_kernel<<<gn, 256>>>(view, alive, nxt.get<u32>(), prv.get<u32>(), outd.get<u8>(),
-                              ind.get<u8>());
-  SBWT_CUDA(cudaMemcpy(pair.get(), nxt.get(), n * 4, cudaMemcpyDeviceToDevice));
-  pair_kernel<<<gn, 256>>>(view, alive, nxt.get<u32>(), prv.get<u32>(), outd.get<u8>(),
-                           ind.get<u8>(), pair.get<u32>());
+  // three u32 arrays and three byte arrays of n, 256-byte aligned
+  const u64 a4 = (n * 4 + 255) / 256 * 256, a1 = (n + 255) / 256 * 256;
+  if (3 * a4 + 3 * a1 > scratch_bytes) return false;
+  u32 *const nxt = reinterpret_cast<u32 *>(scratch);
+  u32 *const prv = reinterpret_cast<u32 *>(scratch + a4);
+  u32 *const pair = reinterpret_cast<u32 *>(scratch + 2 * a4);
+  u8 *const outd = scratch + 3 * a4, *const ind = outd + a1, *const hp = ind + a1;
+  SBWT_CUDA(cudaMemsetAsync(nxt, 0xFF, 2 * a4));
+  SBWT_CUDA(cudaMemsetAsync(outd, 0, 3 * a1));
+  degrees_kernel<<<gn, 256>>>(view, alive, nxt, prv, outd, ind);
+  SBWT_CUDA(cudaMemcpyAsync(pair, nxt, n * 4, cudaMemcpyDeviceToDevice));
+  pair_kernel<<<gn, 256>>>(view, alive, nxt, prv, outd, ind, pair);
   SBWT_CUDA(cudaGetLastError());
   if (L) {
     lmer_filter.resize(lm_words * 8);
-    SBWT_CUDA(cudaMemset(lmer_filter.get(), 0, lm_words * 8));
-    lmer_insert_kernel<<<gn, 256>>>(key, alive, prv.get<u32>(), n, k, L,
+    SBWT_CUDA(cudaMemsetAsync(lmer_filter.get(), 0, lm_words * 8));
+    lmer_insert_kernel<<<gn, 256>>>(key, alive, prv, n, k, L,
                                     lmer_filter.get<unsigned long long>(), (u32)lm_words);
   }
   // splitters: path heads and one k-mer in 64
-  DeviceBuffer has_prev(n);
-  u8 *hp = has_prev.get<u8>(), *sp = ind.get<u8>();  // the in-degrees are done with
-  SBWT_CUDA(cudaMemset(hp, 0, n));
-  has_prev_kernel<<<gn, 256>>>(alive, pair.get<u32>(), n, hp);
+  u8 *const sp = ind;  // the in-degrees are done with
+  has_prev_kernel<<<gn, 256>>>(alive, pair, n, hp);
   splitters_kernel<<<gn, 256>>>(alive, hp, n, sp);
   SBWT_CUDA(cudaGetLastError());
-  u32 *list = nxt.get<u32>(), *map = prv.get<u32>();  // done with as well
-  DeviceBuffer small(16);
-  size_t tb = 0;
+  u32 *const list = nxt, *const map = prv;  // done with as well
   cub::CountingInputIterator<u32> ids(0);
-  SBWT_CUDA(cub::DeviceSelect::Flagged(nullptr, tb, ids, sp, list, small.get<u32>(), (int64_t)n));
-  DeviceBuffer tmp(std::max<size_t>(tb, 1));
-  SBWT_CUDA(cub::DeviceSelect::Flagged(tmp.get(), tb, ids, sp, list, small.get<u32>(),
-                                       (int64_t)n));
+  size_t tb = 0, tb2 = 0;
+  SBWT_CUDA(cub::DeviceSelect::Flagged(nullptr, tb, ids, sp, list, list, (int64_t)n));
+  SBWT_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb2, list, list, (int64_t)n));
+  DeviceBuffer tmp(std::max<size_t>(std::max(tb, tb2), 1) + 256);
+  u32 *const small = reinterpret_cast<u32 *>(tmp.get<u8>());  // a word before the rest
+  void *const cub_tmp = tmp.get<u8>() + 256;
+  SBWT_CUDA(cub::DeviceSelect::Flagged(cub_tmp, tb, ids, sp, list, small, (int64_t)n));
   u32 ns = 0;
-  SBWT_CUDA(cudaMemcpy(&ns, small.get(), 4, cudaMemcpyDeviceToHost));
-  pos_buf.resize(n * 4);
-  SBWT_CUDA(cudaMemset(pos_buf.get(), 0xFF, n * 4));
+  SBWT_CUDA(cudaMemcpy(&ns, small, 4, cudaMemcpyDeviceToHost));
+  SBWT_CUDA(cudaMemsetAsync(pos, 0xFF, n * 4));
   path_nodes.resize(n_kmers * 4);
+  path_entries.resize(n_entries * sizeof(PathEntry));
   u32 placed = 0;
+  DeviceBuffer ranks;  // of the splitters
   if (ns) {
     const unsigned gs = grid_of(ns);
-    DeviceBuffer len(ns * 4ULL), nxs(ns * 4ULL), prs(ns * 4ULL), total((ns + 1) * 4ULL),
-        jump[2] = {DeviceBuffer(ns * sizeof(Jump)), DeviceBuffer(ns * sizeof(Jump))};
-    SBWT_CUDA(cudaMemset(prs.get(), 0xFF, ns * 4ULL));
-    SBWT_CUDA(cudaMemset(total.get(), 0, (ns + 1) * 4ULL));
+    const u64 s4 = ((ns + 1) * 4ULL + 255) / 256 * 256, sj = (ns * sizeof(Jump) + 255) / 256 * 256;
+    ranks.resize(4 * s4 + 2 * sj);
+    u8 *const r = ranks.get<u8>();
+    u32 *const len = reinterpret_cast<u32 *>(r), *const nxs = reinterpret_cast<u32 *>(r + s4);
+    u32 *const prs = reinterpret_cast<u32 *>(r + 2 * s4);
+    u32 *const total = reinterpret_cast<u32 *>(r + 3 * s4);
+    Jump *const jump[2] = {reinterpret_cast<Jump *>(r + 4 * s4),
+                           reinterpret_cast<Jump *>(r + 4 * s4 + sj)};
+    SBWT_CUDA(cudaMemsetAsync(prs, 0xFF, ns * 4ULL));
+    SBWT_CUDA(cudaMemsetAsync(total, 0, (ns + 1) * 4ULL));
     splitter_map_kernel<<<gs, 256>>>(list, ns, map);
-    stretch_kernel<<<gs, 256>>>(list, ns, pair.get<u32>(), sp, map, len.get<u32>(),
-                                nxs.get<u32>(), prs.get<u32>());
+    stretch_kernel<<<gs, 256>>>(list, ns, pair, sp, map, len, nxs, prs);
     SBWT_CUDA(cudaGetLastError());
     u32 rounds = 1;
     while ((1ULL << rounds) < ns) ++rounds;
     Jump *j = nullptr;
     auto rank = [&] {
-      jump_init_kernel<<<gs, 256>>>(ns, prs.get<u32>(), len.get<u32>(), jump[0].get<Jump>());
+      jump_init_kernel<<<gs, 256>>>(ns, prs, len, jump[0]);
       int at = 0;
-      for (u32 r = 0; r <= rounds; ++r, at ^= 1)
-        jump_kernel<<<gs, 256>>>(ns, jump[at].get<Jump>(), jump[at ^ 1].get<Jump>());
-      j = jump[at].get<Jump>();
+      for (u32 q = 0; q <= rounds; ++q, at ^= 1)
+        jump_kernel<<<gs, 256>>>(ns, jump[at], jump[at ^ 1]);
+      j = jump[at];
     };
     rank();
     u32 cut = 0;
-    SBWT_CUDA(cudaMemset(small.get(), 0, 4));
-    cut_cycles_kernel<<<gs, 256>>>(ns, j, prs.get<u32>(), small.get<u32>());
-    SBWT_CUDA(cudaMemcpy(&cut, small.get(), 4, cudaMemcpyDeviceToHost));
+    SBWT_CUDA(cudaMemsetAsync(small, 0, 4));
+    cut_cycles_kernel<<<gs, 256>>>(ns, j, prs, small);
+    SBWT_CUDA(cudaMemcpy(&cut, small, 4, cudaMemcpyDeviceToHost));
     if (cut) rank();
-    path_totals_kernel<<<gs, 256>>>(ns, nxs.get<u32>(), prs.get<u32>(), len.get<u32>(), j,
-                                    total.get<u32>());
-    SBWT_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb, total.get<u32>(), total.get<u32>(),
-                                            (int64_t)ns + 1));
-    tmp.ensure(std::max<size_t>(tb, 1));
-    SBWT_CUDA(cub::DeviceScan::ExclusiveSum(tmp.get(), tb, total.get<u32>(), total.get<u32>(),
-                                            (int64_t)ns + 1));
-    SBWT_CUDA(cudaMemcpy(&placed, total.get<u32>() + ns, 4, cudaMemcpyDeviceToHost));
+    path_totals_kernel<<<gs, 256>>>(ns, nxs, prs, len, j, total);
+    SBWT_CUDA(cub::DeviceScan::ExclusiveSum(cub_tmp, tb2, total, total, (int64_t)ns + 1));
+    SBWT_CUDA(cudaMemcpy(&placed, total + ns, 4, cudaMemcpyDeviceToHost));
     if (placed > n_kmers) throw Error(SBWT_E_FORMAT, "the SBWT's edges are not one-to-one");
-    place_kernel<<<gs, 256>>>(list, ns, pair.get<u32>(), len.get<u32>(), j, total.get<u32>(),
-                              pos_buf.get<u32>(), path_nodes.get<u32>());
+    place_kernel<<<gs, 256>>>(list, ns, pair, len, j, total, pos, path_nodes.get<u32>());
     SBWT_CUDA(cudaGetLastError());
   }
-  SBWT_CUDA(cudaMemcpy(small.get(), &placed, 4, cudaMemcpyHostToDevice));
-  place_rest_kernel<<<gn, 256>>>(alive, n, pos_buf.get<u32>(), path_nodes.get<u32>(),
-                                 small.get<u32>());
-  path_entries.resize(n_entries * sizeof(PathEntry));
-  path_chars_kernel<<<grid_of(n_entries), 256>>>(view, path_nodes.get<u32>(), (u32)n_kmers,
-                                                 pair.get<u32>(), outd.get<u8>(),
-                                                 path_entries.get<PathEntry>(), n_entries);
+  SBWT_CUDA(cudaMemcpyAsync(small, &placed, 4, cudaMemcpyHostToDevice));
+  place_rest_kernel<<<gn, 256>>>(alive, n, pos, path_nodes.get<u32>(), small);
+  path_chars_kernel<<<grid_of(n_entries), 256>>>(view, path_nodes.get<u32>(), (u32)n_kmers, pair,
+                                                 outd, path_entries.get<PathEntry>(), n_entries);
   SBWT_CUDA(cudaGetLastError());
-  SBWT_CUDA(cudaDeviceSynchronize());
   view.path_node = path_nodes.get<u32>();
   view.path_entry = path_entries.get<PathEntry>();
   view.lmer_filter = L ? lmer_filter.get<u64>() : nullptr;

@@ -91,3 +91,23 @@ def test_positions_over_the_cover_match_oracle(kind, k):
     with pytest.raises(S.SbwtError) as e:
         idx.search(bits, np.array([0, last + 1], np.uint64))
     assert e.value.code == S.E_INVALID
+
+
+@pytest.mark.parametrize("k", [2, 3, 4, 5, 7, 8, 9, 15, 16, 17, 29])
+def test_labels_of_every_k(k):
+    """The table's labels are put together by doublings and single steps chosen
+    by the bits of k - 1: every k-mer of the index, and 2 000 others, found by
+    the table as by the oracle."""
+    g = genomes_of("strains", k)
+    path = TMP / f"cover_labels_{k}.sbwt"
+    T.build_sbwt(g, k, str(path))
+    idx = S.SbwtIndex.open(path)
+    rng = np.random.default_rng(k)
+    noise = np.frombuffer(b"ACGT", np.uint8)[rng.integers(0, 4, 2000)]
+    chars = np.concatenate([g.chars, noise])
+    chars = chars[:len(chars) // 32 * 32]
+    bits, _ = O.seq_to_bits(chars.tobytes())
+    bits = bits[:len(chars) // 32]
+    pos = np.arange(len(chars) - k + 1, dtype=np.uint64)
+    exp = oracle_index(str(path), min(k, 6)).search_positions(bits, pos)
+    assert np.array_equal(idx.search(bits, pos), exp)
