@@ -597,7 +597,7 @@ def parse():
     ap.add_argument("--colors-plain-reads", type=int, default=500_000)
     ap.add_argument("--kernel", type=int, default=-1,
                     help="read search kernel with a k-mer table (sbwt_set_table_kernel): "
-                         "0 general, 1 table, 2..5 walks variants, -1 library default")
+                         "0 general, 1 table, 2..5 walks variants, 7 paths, -1 library default")
     ap.add_argument("--colors-only", action="store_true",
                     help="run only the colors and serving sections (profiling runs)")
     ap.add_argument("--cfg1-only", action="store_true",
@@ -815,7 +815,8 @@ KERNELS = {0: "search_reads_kernel", 1: "search_table_kernel", 2: "search_walks_
            16: "search_walks_kernel", 17: "search_walks_kernel", 18: "search_walks_kernel",
            19: "search_kmers_kernel"}
 DEFAULT_KERNEL_MODE = 7
-KMERS_KERNEL_MAX_BYTES = 256 << 20  # mode 7 picks the k-mers kernel up to this
+KMERS_KERNEL_MAX_BYTES = 256 << 20  # without a cover, mode 7 picks the k-mers kernel up to this
+PATHS_KERNEL_MAX_NODES = 192 << 24  # an index with its k-mer table has its path cover below this
 
 
 def search_kernel_name(idx, mode: int) -> str:
@@ -826,21 +827,38 @@ def search_kernel_name(idx, mode: int) -> str:
     if not table:
         return KERNELS[0]
     if mode == 7:
+        if idx.num_bits < PATHS_KERNEL_MAX_NODES:
+            return "search_paths_kernel"
         mode = 11 if 0 < idx.filter_bytes() and table + idx.filter_bytes() <= \
             KMERS_KERNEL_MAX_BYTES else 17
     return KERNELS[mode]
 
 
-FILTER_KERNELS = ("search_walks_kernel", "search_kmers_kernel", "search_kmers_seq_kernel")
+FILTER_KERNELS = ("search_paths_kernel", "search_walks_kernel", "search_kmers_kernel",
+                  "search_kmers_seq_kernel")
 
 
-def index_working_sets(idx):
+def search_sectors(kernel: str, ctr):
+    """(hot sectors, table or presearch lookups, filter words) of the counters
+    of one read search, in the classes of index_working_sets.  The paths
+    kernel counts two cover entries (16 bytes each) per look at the cover."""
+    if kernel == "search_paths_kernel":
+        return int(ctr[2]), int(ctr[0]), int(ctr[3]) + int(ctr[1]) // 2
+    return (int(ctr[1]) + int(ctr[2]), int(ctr[0]),
+            int(ctr[3]) if kernel in FILTER_KERNELS else 0)
+
+
+def index_working_sets(idx, kernel):
     """Bytes the read search touches at random: the rank blocks of the four
     vectors plus the suffix-group-start words (every step); the table it
     starts a k-mer from (one lookup per k-mer not reached by a stream step):
     the k-mer table when the index has one, else the presearch level; and
-    the k-mer filter in front of the table (10 bits per k-mer)."""
+    the k-mer filter in front of the table (10 bits per k-mer).  The
+    paths kernel: the cover's nodes (4 B per k-mer); the k-mer table; the
+    L-mer filter and the cover's chars (1 and 0.5 B per k-mer)."""
     n = idx.num_bits
+    if kernel == "search_paths_kernel":
+        return 4 * n, idx.set_kmer_table(True), n + n // 2
     hot = 4 * (n // 192 + 1) * 32 + (n + 63) // 64 * 8
     table = idx.set_kmer_table(True)  # its size (kept when present)
     if table:
@@ -849,17 +867,16 @@ def index_working_sets(idx):
     return hot, (4 ** idx.presearch_letters) * entry, 0
 
 
-def sector_roofline(S, dev, idx, n_hot, n_pre, kernel_s, n_filter=0, cold=False):
+def sector_roofline(S, dev, idx, kernel, n_hot, n_pre, kernel_s, n_filter=0, cold=False):
     """Random-sector roofline of the read search: the time the kernel's
     sectors take at the measured random-gather rate of their own working set
-    (rank blocks + group words; the k-mer table or presearch level; the
-    k-mer filter), over the kernel time.  The rates are those of a warm L2
+    (index_working_sets), over the kernel time.  The rates are those of a warm L2
     (the microbenchmark repeats its gathers over one buffer).  cold=True
     (L2 flushed before the timed launch) adds `cold_l2`: each class's
     expected distinct sectors, S * (1 - exp(-n / S)) for n uniform random
     loads over S sectors, are first touches served by DRAM at the measured
     rate of a 2 GiB buffer; the rest at the class's warm rate."""
-    hot_b, pre_b, filt_b = index_working_sets(idx)
+    hot_b, pre_b, filt_b = index_working_sets(idx, kernel)
     r_hot = random_sector_peak(S, dev, hot_b)
     r_pre = random_sector_peak(S, dev, pre_b)
     r_filt = random_sector_peak(S, dev, filt_b) if (filt_b and n_filter) else 0.0
@@ -927,8 +944,8 @@ def bench_cfg1(args, S, torch, dev, tmpdir):
     L.sbwt_profile_read(None, None, None, ctr)
     L.sbwt_profile_enable(0, 0)
     kernel = search_kernel_name(idx, args.kernel)
-    n_filter = int(ctr[3]) if kernel in FILTER_KERNELS else 0
-    sectors = int(ctr[0]) + int(ctr[1]) + int(ctr[2]) + n_filter
+    n_hot, n_pre, n_filter = search_sectors(kernel, ctr)
+    sectors = n_hot + n_pre + n_filter
     for _ in range(max(3, args.warmup)):
         step()
     flush = torch.empty(256 << 20, dtype=torch.uint8, device=f"cuda:{dev}")
@@ -954,8 +971,8 @@ def bench_cfg1(args, S, torch, dev, tmpdir):
            "kmers_per_s": nk / (total_ms / n_steps / 1e3), "ms_per_step": total_ms / n_steps,
            "l2": "flushed (256 MB write) before every timed step",
            "kernel": kernel,
-           "random_sector": dict(sector_roofline(S, dev, idx, int(ctr[1]) + int(ctr[2]),
-                                                 int(ctr[0]), kern_s, n_filter, cold=True),
+           "random_sector": dict(sector_roofline(S, dev, idx, kernel, n_hot, n_pre, kern_s,
+                                                 n_filter, cold=True),
                                  sectors_per_kmer=sectors / nk)}
     r = cpu_reference_rate(path, chars, ends, 31, len(ends))
     if r is not None:
@@ -1410,22 +1427,24 @@ def main():
     # roofline of the dominant kernel (the read search kernel)
     peak, peak_kind = load_peaks()
     kern_ms = search_ms.value / max(1, search_launches.value)
-    # the kernel that ran: with the k-mer table (k <= 31) the walks kernel by
+    # the kernel that ran: with the k-mer table (k <= 31) the paths kernel by
     # default, else the general kernel
     kernel = search_kernel_name(idx, args.kernel)
-    n_filter = n_probe if kernel in FILTER_KERNELS else 0
+    paths = kernel == "search_paths_kernel"
+    n_hot, _, n_filter = search_sectors(kernel, ctr)
     if n_filter:
         n_probe = 0
     # algorithmic bytes per launch (what this kernel's algorithm must move):
-    # one 32-byte sector per k-mer-table or presearch lookup, per k-mer filter
-    # word, per rank block and per suffix-group word the search reads; 8 B
+    # one 32-byte sector per k-mer-table or presearch lookup, per filter word,
+    # per rank block and per suffix-group word the search reads (paths kernel:
+    # per look at the cover's chars, and per 8 nodes of its runs); 8 B
     # result per k-mer; 2 bits of packed input + 1 invalid bit per char.
-    alg_bytes = ((n_pre + n_block + n_sg + n_filter) * 32 + n_kmers * 8 + n_chars / 4 +
+    alg_bytes = ((n_pre + n_hot + n_filter) * 32 + n_kmers * 8 + n_chars / 4 +
                  n_chars / 8)
     achieved = alg_bytes / (kern_ms / 1e3) / 1e9
     traffic_pk = profiled_traffic_per_kmer(kernel)
     try:
-        rs = sector_roofline(S, dev, idx, n_block + n_sg, n_pre, kern_ms / 1e3, n_filter)
+        rs = sector_roofline(S, dev, idx, kernel, n_hot, n_pre, kern_ms / 1e3, n_filter)
     except Exception as e:  # reported as unmeasured, never hides the headline
         rs = {"error": repr(e)}
 
@@ -1486,9 +1505,11 @@ def main():
                    "kernels": f"{kernel}"
                               + (" (the default, automatic mode 7 picks it for this index)"
                                  if args.kernel < 0 else f" (mode {args.kernel})")
-                              + ", grid of 8 x 256-thread blocks per SM, tiles of "
-                                "k-mers / (resident threads x 8) rounded up to 16 slots, "
-                                "16 to 128"},
+                              + (", grid of 4 x 256-thread blocks per SM, tiles of k-mers / "
+                                 "(SMs x 4096) rounded up to 16 slots, 16 to 64" if paths else
+                                 ", grid of 8 x 256-thread blocks per SM, tiles of "
+                                 "k-mers / (resident threads x 8) rounded up to 16 slots, "
+                                 "16 to 128")},
         "gpu_launches": int(launches.value),
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak,
@@ -1497,7 +1518,13 @@ def main():
                                        f"({profile_file(kernel).relative_to(REPO)})",
                      "peak_kind": peak_kind, "kernel": kernel,
                      "kernel_ms": kern_ms,
-                     "work": {"table_or_presearch_lookups": n_pre,
+                     "work": ({"kmer_table_lookups": n_pre, "cover_entries": n_block,
+                               "node_sectors": n_sg, "filter_words": int(ctr[3]),
+                               "bytes_per_kmer": alg_bytes / n_kmers,
+                               "warp_iterations": n_iter, "runs": n_lane,
+                               "kmers_written_without_search": n_known,
+                               "kmers_found": n_searched} if paths else
+                              {"table_or_presearch_lookups": n_pre,
                               "rank_block_sectors": n_block,
                               "suffix_group_words": n_sg, "probe_iterations": n_probe,
                               "filter_words": n_filter,
@@ -1510,7 +1537,8 @@ def main():
                                   ["stream", "filter" if n_filter else "presearch", "walk",
                                    "group_scan", "kmer_table", "probe"],
                                   [int(x) for x in ctr[8:14]])),
-                              "distinct_paths_per_iteration": int(ctr[14]) / max(n_iter, 1)},
+                              "distinct_paths_per_iteration":
+                                  int(ctr[14]) / max(n_iter, 1)}),
                      "random_sector": rs},
         "cpu_baseline": cpu,
         "e2e": e2e,

@@ -408,8 +408,10 @@ int sbwt_set_probe_length(uint32_t probe_len);
  *       (2, 3), (4, 2);
  *   6 = the k-mers kernel (every k-mer on its own: filter, then table; no
  *       stream steps, all loads of a lane independent);
- *   7 = automatic, the default: 11 when the table and filter take at most
- *       256 MiB, else 17;
+ *   7 = automatic, the default: the paths kernel (one table lookup per run
+ *       of consecutive k-mers, the rest of the run read along a cover of the
+ *       graph's edges by paths) on an index with its path cover; without one
+ *       11 when the table and filter take at most 256 MiB, else 17;
  *   8, 9 = the walks kernel without the filter and the staged stores, 1 or 2
  *       walks per lane; 10 = the same with 1 walk and the filter in front of
  *       the table, one k-mer at a time; 11, 12 = the k-mers kernel with 2 or
@@ -449,9 +451,9 @@ int sbwt_measure_random_sectors(int device, uint64_t bytes, int chains,
  * unit) {auto, 64, 256}, blocks per SM in the grid {2, 4, 6, 8} and threads
  * per block {128, 256}, checks that every configuration gives the same results,
  * and makes the fastest the process-wide launch configuration.  The first
- * axis is the read search kernel (sbwt_set_table_kernel 1..6: the table
- * kernel, the walks kernel with 1, 2 or 4 walks per lane, the k-mers
- * kernel) when the index has its k-mer table, else the presearch depth (8 up
+ * axis is the read search kernel (sbwt_set_table_kernel 1, 2, 6, 7, 11, 17
+ * and 18: the table kernel, walks kernels, k-mers kernels, and the automatic
+ * choice) when the index has its k-mer table, else the presearch depth (8 up
  * to the index's); the block size (128 or 256 threads) is swept too.
  * sbwt_get_launch_config reads the choice back. */
 int sbwt_autotune(const sbwt_index_t *index, const char *d_chars,
@@ -460,7 +462,10 @@ int sbwt_autotune(const sbwt_index_t *index, const char *d_chars,
                   uint32_t *best_presearch, uint32_t *best_blocks_per_sm,
                   uint64_t *best_tile, double *best_ms);
 /* Reads and resets the totals (any pointer may be NULL).  counters (count
- * mode): presearch lookups, rank-block sectors, suffix-group words, probe
+ * mode; the paths kernel's are k-mer table lookups, path cover entries, node
+ * sectors, filter words, warp iterations, runs, k-mers written without a
+ * search and k-mers found, and of the lane steps the filter's and the
+ * table's): presearch lookups, rank-block sectors, suffix-group words, probe
  * iterations, warp iterations, lane load steps, k-mers written without a
  * search, k-mers searched, lane steps of each search path (stream step,
  * presearch of a new k-mer, walk, group scan, k-mer table lookup, probe),

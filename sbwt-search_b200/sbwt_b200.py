@@ -168,8 +168,8 @@ def set_block_threads(threads: int = 256) -> None:
 def set_table_kernel(mode: int = TABLE_KERNEL_DEFAULT) -> None:
     """Read search kernel of an index with a k-mer table: 0 general, 1 table
     (True), 2..5 walks kernel with (walks per lane, blocks per SM) = (1, 5),
-    (2, 4), (2, 3), (4, 2), 6 k-mers kernel, 7 automatic (11 for small
-    tables, else 17), 8/9 walks kernel without filter and staging (1/2
+    (2, 4), (2, 3), (4, 2), 6 k-mers kernel, 7 automatic (the paths kernel
+    with a path cover; without one 11 for small tables, else 17), 8/9 walks kernel without filter and staging (1/2
     walks), 10 the same with 1 walk and a one-k-mer filter, 11/12 k-mers
     kernel with 2/8 k-mers per lane, 13/14 = 8/10 with staged stores,
     15 k-mers kernel over consecutive slots, 16/17 = 13 staging 8/16 slots,
@@ -517,10 +517,11 @@ AUTOTUNE_CACHE = HERE / "_build" / "autotune.json"
 
 def autotune(index: SbwtIndex, d_chars, d_read_ends, sample_chars: int = 256 << 20,
              use_cache: bool = True) -> dict:
-    """Chooses the read search kernel (walks per lane) or presearch depth,
+    """Chooses the read search kernel or presearch depth,
     tile size and blocks per SM for this GPU and index with the library's
     autotuner (sbwt_autotune) and applies them; the choice is cached per
-    (GPU name, SBWT nodes, k, k-mer table present) in _build/autotune.json."""
+    (GPU name, SBWT nodes, k, k-mer table present, kernels swept) in
+    _build/autotune.json."""
     import json
     try:
         import torch
@@ -529,7 +530,8 @@ def autotune(index: SbwtIndex, d_chars, d_read_ends, sample_chars: int = 256 << 
         gpu = "cuda"
     info = IndexInfo()
     check(lib().sbwt_index_get_info(index._h, C.byref(info)))
-    key = f"{gpu}|{index.num_bits}|{index.k}|table={int(info.kmer_table_bytes > 0)}"
+    # "paths": choices kept from before the paths kernel existed are not taken
+    key = f"{gpu}|{index.num_bits}|{index.k}|table={int(info.kmer_table_bytes > 0)}|paths"
     cache = {}
     if use_cache and AUTOTUNE_CACHE.exists():
         try:
