@@ -10,9 +10,11 @@
 //   -1 / -2 mapping        IndexResultsPrinter/ContinuousIndexResultsPrinter.hpp:196-205
 #include <cuda_runtime.h>
 #include <emmintrin.h>
+#include <sys/mman.h>
 
 #include <algorithm>
 #include <atomic>
+#include <condition_variable>
 #include <cstring>
 #include <map>
 #include <memory>
@@ -2821,18 +2823,28 @@ struct Workspace {
       block_sums[2], total[2], tile_read[2], queue[2], positions, bits, results32[2];
   uint32_t *err_host = nullptr;  // pinned: the error word, then (at +8 bytes) a k-mer count
   DeviceBuffer err_dev;
-  cudaEvent_t done[2] = {nullptr, nullptr};
   uint32_t *stage[2] = {nullptr, nullptr};  // pinned: 32-bit results of a chunk
-  u64 stage_cap[2] = {0, 0};
-  uint32_t *staging(int b, u64 n) {
-    if (stage_cap[b] < n) {
-      if (stage[b]) cudaFreeHost(stage[b]);
-      stage[b] = nullptr;
-      stage_cap[b] = 0;
-      SBWT_CUDA(cudaHostAlloc((void **)&stage[b], n * 4, cudaHostAllocDefault));
-      stage_cap[b] = n;
+  char *stage_in[2] = {nullptr, nullptr};   // pinned: the chars of a chunk
+  u64 stage_cap[2] = {0, 0}, stage_in_cap[2] = {0, 0};  // bytes
+  cudaEvent_t arrived[2][16] = {};  // a slice's codes are in `stage`
+  template <class T>
+  static T *pinned(T *&p, u64 &cap, u64 bytes) {
+    if (cap < bytes) {
+      if (p) cudaFreeHost(p);
+      p = nullptr;
+      cap = 0;
+      SBWT_CUDA(cudaHostAlloc((void **)&p, bytes, cudaHostAllocDefault));
+      cap = bytes;
     }
-    return stage[b];
+    return p;
+  }
+  uint32_t *staging(int b, u64 n) { return pinned(stage[b], stage_cap[b], n * 4); }
+  char *staging_in(int b, u64 n) { return pinned(stage_in[b], stage_in_cap[b], n); }
+  const cudaEvent_t *arrivals(int b) {
+    for (auto &e : arrived[b])
+      if (!e)
+        SBWT_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    return arrived[b];
   }
   ~Workspace() {
     if (device < 0) return;
@@ -2841,11 +2853,14 @@ struct Workspace {
     cudaSetDevice(device);
     for (auto &s : streams)
       if (s) cudaStreamDestroy(s);
-    for (auto &e : done)
-      if (e) cudaEventDestroy(e);
     if (err_host) cudaFreeHost(err_host);
     for (auto *p : stage)
       if (p) cudaFreeHost(p);
+    for (auto *p : stage_in)
+      if (p) cudaFreeHost(p);
+    for (auto &es : arrived)
+      for (auto &e : es)
+        if (e) cudaEventDestroy(e);
     cudaSetDevice(prev);
   }
 };
@@ -2869,22 +2884,138 @@ static void widen_range(const uint32_t *src, u64 *dst, u64 n) {
   for (; i < n; ++i) dst[i] = widen_code(src[i]);
   _mm_sfence();
 }
-static void widen_results(const uint32_t *src, u64 *dst, u64 n) {
-  const u64 per = 4ULL << 20;  // k-mers per thread at least
-  const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
-  const unsigned T = (unsigned)std::min<u64>(std::min<u64>(hw, 32), std::max<u64>(n / per, 1));
-  if (T <= 1) {
-    widen_range(src, dst, n);
-    return;
+
+// The host's share of a chunk with pageable buffers, on threads of its own, a
+// slice of the chunk each.  A thread copies its slice of the chars into the
+// pinned buffer the GPU reads (the driver's own staging of a pageable copy
+// runs at 11 GB/s), has the pages of its slice of the results mapped while the
+// GPU works, and widens the slice's codes as soon as they have arrived, while
+// the next slices still cross.
+// What bounds it: the two copies over PCIe (4 ms) and the first touch of the
+// results' pages.  28 M k-mers of 34 MB of reads on 16 cores, into a new
+// buffer: whole call 16.3 ms when the driver staged the chars and 6 threads
+// widened the codes at the end, 7.4 ms here (12 threads 7.7 to 8.4, 8 threads
+// 9.9; without mapping the pages ahead 10.2); 8.4 M k-mers 9.3 -> 3.1 ms.
+// Slices of at least kSliceKmers: with half of that 8.4 M k-mers take 4.1 ms
+// and 1.7 M 1.3 ms against 0.9 on the calling thread alone.
+class HostSlices {
+ public:
+  static constexpr u64 kSliceKmers = 1ULL << 20;
+  static unsigned slices_for(u64 n) {
+    const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
+    return (unsigned)std::min<u64>(std::min(hw, (unsigned)kMaxSlices),
+                                   std::max<u64>(n / kSliceKmers, 1));
   }
-  std::vector<std::thread> th;
-  th.reserve(T);
-  for (unsigned t = 0; t < T; ++t) {
-    const u64 a = n * t / T, b = n * (t + 1) / T;
-    th.emplace_back(widen_range, src + a, dst + a, b - a);
+  static constexpr int kMaxSlices = 16;
+
+  // in: the chars to copy to in_stage (nullptr: none), events: one per slice.
+  HostSlices(int device, const char *in, char *in_stage, u64 n_in, const uint32_t *codes, u64 *dst,
+             u64 n, const cudaEvent_t *events)
+      : device_(device), in_(in), in_stage_(in_stage), n_in_(in ? n_in : 0), codes_(codes),
+        dst_(dst), n_(n), T_(slices_for(n)), events_(events) {
+    if (T_ < 2) return;
+    try {
+      th_.reserve(T_);
+      for (unsigned t = 0; t < T_; ++t) th_.emplace_back(&HostSlices::work, this, t);
+    } catch (const std::exception &) {  // no more threads: finish() does the rest
+    }
   }
-  for (auto &x : th) x.join();
-}
+  ~HostSlices() {
+    {
+      std::lock_guard<std::mutex> g(m_);
+      if (state_ == kWaiting) state_ = kCancelled;
+    }
+    cv_.notify_all();
+    for (auto &x : th_) x.join();
+  }
+  HostSlices(const HostSlices &) = delete;
+  HostSlices &operator=(const HostSlices &) = delete;
+
+  unsigned slices() const { return T_; }
+  u64 in_at(unsigned t) const { return n_in_ * t / T_; }
+  // results at 2 MiB borders of the buffer, so that no two threads map a page
+  u64 at(unsigned t) const {
+    if (t == 0 || t == T_) return t ? n_ : 0;
+    const u64 a = (reinterpret_cast<uintptr_t>(dst_ + n_ * t / T_) & ~((2ULL << 20) - 1));
+    const u64 d = reinterpret_cast<uintptr_t>(dst_);
+    return a <= d ? 0 : (a - d + 7) / 8;
+  }
+  // Returns once slice t of the chars is in the pinned buffer.
+  void wait_in(unsigned t) {
+    if (t >= th_.size()) {
+      copy_in(t);
+      return;
+    }
+    std::unique_lock<std::mutex> g(m_);
+    cv_in_.wait(g, [&] { return (in_done_ >> t) & 1u; });
+  }
+  void go() {  // every slice's copy is enqueued, its event recorded
+    {
+      std::lock_guard<std::mutex> g(m_);
+      state_ = kGo;
+    }
+    cv_.notify_all();
+  }
+  void finish() {  // after go()
+    for (unsigned t = (unsigned)th_.size(); t < T_; ++t) widen(t);
+    for (auto &x : th_) x.join();
+    th_.clear();
+    SBWT_CUDA(err_);
+  }
+
+ private:
+  enum { kWaiting, kGo, kCancelled };
+  void copy_in(unsigned t) {
+    const u64 a = in_at(t), b = in_at(t + 1);
+    if (in_ && b > a) std::memcpy(in_stage_ + a, in_ + a, b - a);
+  }
+  void widen(unsigned t) {
+    const cudaError_t e = cudaEventSynchronize(events_[t]);
+    if (e != cudaSuccess) {
+      std::lock_guard<std::mutex> g(m_);
+      err_ = e;
+      return;
+    }
+    const u64 a = at(t), b = at(t + 1);
+    if (b > a) widen_range(codes_ + a, dst_ + a, b - a);
+  }
+  void work(unsigned t) {
+    copy_in(t);
+    {
+      std::lock_guard<std::mutex> g(m_);
+      in_done_ |= 1u << t;
+    }
+    cv_in_.notify_all();
+    // maps the pages without changing what they hold; a kernel or a mapping
+    // that cannot do it leaves them to the stores
+    const uintptr_t page = 4096;
+    const uintptr_t p0 = (reinterpret_cast<uintptr_t>(dst_ + at(t)) + page - 1) & ~(page - 1);
+    const uintptr_t p1 = reinterpret_cast<uintptr_t>(dst_ + at(t + 1)) & ~(page - 1);
+    if (p1 > p0) madvise(reinterpret_cast<void *>(p0), p1 - p0, 23 /* MADV_POPULATE_WRITE */);
+    {
+      std::unique_lock<std::mutex> g(m_);
+      cv_.wait(g, [&] { return state_ != kWaiting; });
+      if (state_ == kCancelled) return;
+    }
+    cudaSetDevice(device_);
+    widen(t);
+  }
+  int device_;
+  const char *in_;
+  char *in_stage_;
+  u64 n_in_;
+  const uint32_t *codes_;
+  u64 *dst_;
+  u64 n_;
+  unsigned T_;
+  const cudaEvent_t *events_;
+  std::vector<std::thread> th_;
+  std::mutex m_;
+  std::condition_variable cv_, cv_in_;
+  uint32_t in_done_ = 0;
+  int state_ = kWaiting;
+  cudaError_t err_ = cudaSuccess;
+};
 
 static Workspace &workspace(int device) {
   thread_local std::map<int, std::unique_ptr<Workspace>> ws;
@@ -2894,7 +3025,6 @@ static Workspace &workspace(int device) {
     p->device = device;
     for (auto &s : p->streams)
       SBWT_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-    for (auto &e : p->done) SBWT_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     SBWT_CUDA(cudaMallocHost(&p->err_host, 16));
     p->err_dev.resize(16);  // the error word, then (at +8 bytes) the k-mer count of slot 0
     SBWT_CUDA(cudaMemset(p->err_dev.get(), 0, 16));
@@ -3276,22 +3406,19 @@ void IndexImpl::search_reads(const char *chars, u64 n_chars, const u64 *read_end
   // would take them through the driver's staging copies; with the walks or
   // k-mers kernel the results of a chunk then cross PCIe as 32-bit codes into
   // a pinned staging buffer instead and are widened to u64 on host threads
-  // while the next chunk runs (half the device-to-host bytes).
+  // (half the device-to-host bytes; HostSlices).
   const u64 chunk_chars = cfg.chunk_chars ? cfg.chunk_chars : (64ULL << 20);
-  const bool pinned_in = is_host_pinned(chars) && is_host_pinned(read_ends);
+  const bool pinned_chars = is_host_pinned(chars);
+  const bool pinned_in = pinned_chars && is_host_pinned(read_ends);
   const bool pinned = pinned_in && is_host_pinned(results);
   const SbwtView sv_host = view_for(cfg.presearch_letters);
   const bool stream_host = !(flags & SBWT_PER_KMER_WALK) && view.suffix_group_starts;
   const u32 mtk_host = (flags & SBWT_MOVE_TO_KEY_KMER) ? 1u : 0u;
-  struct Pending {
-    int b = -1;
-    u64 at = 0, n = 0;
-  } pend;
-  auto drain = [&]() {  // widens the chunk whose 32-bit results are in flight
-    if (pend.b < 0) return;
-    SBWT_CUDA(cudaEventSynchronize(ws.done[pend.b]));
-    widen_results(ws.stage[pend.b], results + pend.at, pend.n);
-    pend.b = -1;
+  std::unique_ptr<HostSlices> pend;  // the chunk whose 32-bit results are in flight
+  auto drain = [&]() {
+    if (!pend) return;
+    const std::unique_ptr<HostSlices> p = std::move(pend);
+    p->finish();
   };
   u64 r = 0, kacc = 0, prev_end = 0;
   bool over = false, unordered = false;
@@ -3327,24 +3454,45 @@ void IndexImpl::search_reads(const char *chars, u64 n_chars, const u64 *read_end
     else
       ws.results[b].ensure(std::max<u64>(nk, 1) * 8);
     const ReadsScratch sc = scratch_for(ws, b, nc, nr, nk, index_tile_size(*this, nk, cfg));
-    SBWT_CUDA(cudaMemcpyAsync(ws.chars[b].get(), chars + c0, nc, cudaMemcpyHostToDevice, st));
+    std::unique_ptr<HostSlices> slices;
+    uint32_t *stage = nullptr;
+    bool staged = false;  // the chars go through the pinned buffer
+    if (narrow) {
+      stage = ws.staging(b, std::max<u64>(nk, 1));
+      staged = !pinned_chars && HostSlices::slices_for(nk) > 1;
+      slices = std::make_unique<HostSlices>(
+          device, staged ? chars + c0 : nullptr, staged ? ws.staging_in(b, nc) : nullptr, nc, stage,
+          results + kacc, nk, ws.arrivals(b));
+    }
+    if (staged) {
+      for (unsigned t = 0; t < slices->slices(); ++t) {
+        slices->wait_in(t);
+        const u64 a = slices->in_at(t), n = slices->in_at(t + 1) - a;
+        if (n)
+          SBWT_CUDA(cudaMemcpyAsync(ws.chars[b].get<char>() + a, ws.stage_in[b] + a, n,
+                                    cudaMemcpyHostToDevice, st));
+      }
+    } else {
+      SBWT_CUDA(cudaMemcpyAsync(ws.chars[b].get(), chars + c0, nc, cudaMemcpyHostToDevice, st));
+    }
     SBWT_CUDA(cudaMemcpyAsync(ws.ends[b].get(), read_ends + r0, nr * 8,
                               cudaMemcpyHostToDevice, st));
     const BatchPlan plan = plan_batch(*this, nc, nr, nk, flags, cfg);
     launch_prepare(device, k, ws.chars[b].get<char>(), nc, ws.ends[b].get<u64>(), nr, c0, sc, plan,
                    st);
     if (narrow) {
-      uint32_t *stage = ws.staging(b, std::max<u64>(nk, 1));
       launch_search(*this, nc, ws.ends[b].get<u64>(), nr, c0, nk, nullptr, nk, flags, cfg, sc,
                     plan, st, ws.results32[b].get<uint32_t>());
-      if (nk)
-        SBWT_CUDA(cudaMemcpyAsync(stage, ws.results32[b].get(), nk * 4,
-                                  cudaMemcpyDeviceToHost, st));
-      SBWT_CUDA(cudaEventRecord(ws.done[b], st));
+      for (unsigned t = 0; t < slices->slices(); ++t) {
+        const u64 a = slices->at(t), n = slices->at(t + 1) - a;
+        if (n)
+          SBWT_CUDA(cudaMemcpyAsync(stage + a, ws.results32[b].get<uint32_t>() + a, n * 4,
+                                    cudaMemcpyDeviceToHost, st));
+        SBWT_CUDA(cudaEventRecord(ws.arrived[b][t], st));
+      }
+      slices->go();
       drain();  // the previous chunk, while this one runs
-      pend.b = b;
-      pend.at = kacc;
-      pend.n = nk;
+      pend = std::move(slices);
       if (!pinned_in) drain();
     } else {
       drain();
