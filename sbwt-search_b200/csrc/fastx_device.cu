@@ -74,19 +74,60 @@ __device__ __forceinline__ uint64_t char_class(uint32_t c) {
 // Line i: its first byte, its length (without the '\r' before its '\n') and
 // its first char as far as it matters ('>' for a header, '+', '\n' for an
 // empty line, else 'A').
-__device__ __forceinline__ void line_at(const Lines &L, uint64_t i, uint64_t &start,
-                                        uint32_t &len, uint8_t &c0) {
-  const uint64_t before = i ? __ldg(L.nl + i - 1) : 0;
+// before, e: the entries of the newlines before and after it.
+__device__ __forceinline__ void line_of(const Lines &L, uint64_t i, uint64_t before, uint64_t e,
+                                        uint64_t &start, uint32_t &len, uint8_t &c0) {
   const uint64_t cls = i ? before & 3 : char_class(L.text[0]);
   start = i ? (before >> 3) + 1 : 0;
   uint64_t n = L.n_bytes - start;
   if (i < L.n_nl) {
-    const uint64_t e = __ldg(L.nl + i);
     n = (e >> 3) - start;
     if (n > 0 && (e & kCr)) --n;
   }
   len = (uint32_t)min(n, (uint64_t)0xFFFFFFFFu);
   c0 = n == 0 ? '\n' : (cls == kHeaderClass ? '>' : (cls == kPlusClass ? '+' : 'A'));
+}
+__device__ __forceinline__ void line_at(const Lines &L, uint64_t i, uint64_t &start,
+                                        uint32_t &len, uint8_t &c0) {
+  line_of(L, i, i ? __ldg(L.nl + i - 1) : 0, i < L.n_nl ? __ldg(L.nl + i) : 0, start, len, c0);
+}
+
+// f(start, length, first char) of the lines [l0, l0 + n), l0 a multiple of 8:
+// the entries of eight newlines are loaded together, those of the next eight
+// while these lines are looked at.
+template <class F>
+__device__ __forceinline__ void each_line(const Lines &L, uint64_t l0, uint32_t n, F f) {
+  uint64_t e[8], next[8];
+  auto load = [&](uint64_t i, uint64_t (&x)[8]) {
+    if (i + 8 <= L.n_nl) {
+#pragma unroll
+      for (int q = 0; q < 8; q += 2) {
+        const ulonglong2 v = __ldg(reinterpret_cast<const ulonglong2 *>(L.nl + i + q));
+        x[q] = v.x;
+        x[q + 1] = v.y;
+      }
+    } else {
+#pragma unroll
+      for (int q = 0; q < 8; ++q) x[q] = i + q < L.n_nl ? __ldg(L.nl + i + q) : 0;
+    }
+  };
+  uint64_t before = l0 ? __ldg(L.nl + l0 - 1) : 0;
+  load(l0, next);
+  for (uint32_t j = 0; j < n; j += 8) {
+#pragma unroll
+    for (int q = 0; q < 8; ++q) e[q] = next[q];
+    if (j + 8 < n) load(l0 + j + 8, next);
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      if (j + q >= n) break;
+      uint64_t start;
+      uint32_t len;
+      uint8_t c0;
+      line_of(L, l0 + j + q, before, e[q], start, len, c0);
+      before = e[q];
+      f(start, len, c0);
+    }
+  }
 }
 
 // One line through the record state machine; returns its role.
@@ -160,8 +201,10 @@ __device__ __forceinline__ uint32_t equal_bits16(const uint4 &x, uint32_t c) {
 // text may start inside one: `lead` bytes into it), kNlLoads per lane.
 constexpr int kNlLoads = kWarpBytes / 512;
 
+// marks: a bit per byte, a word of kNlLoads 16-bit masks per lane.
+static_assert(kNlLoads == 8, "a lane's masks fill a uint4");
 __global__ void nl_count_kernel(const uint8_t *text, uint64_t n, uint32_t lead,
-                                uint64_t *warp_counts, uint64_t n_warps) {
+                                uint64_t *warp_counts, uint64_t n_warps, uint4 *marks) {
   const uint32_t lane = threadIdx.x & 31;
   const uint64_t w = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
   if (w >= n_warps) return;
@@ -169,31 +212,36 @@ __global__ void nl_count_kernel(const uint8_t *text, uint64_t n, uint32_t lead,
   uint4 x[kNlLoads];
 #pragma unroll
   for (int i = 0; i < kNlLoads; ++i) x[i] = text16(text, n, p0 + 512 * i);
-  uint32_t cnt = 0;
+  uint32_t m[kNlLoads / 2], cnt = 0;
 #pragma unroll
-  for (int i = 0; i < kNlLoads; ++i) cnt += __popc(equal_bits16(x[i], '\n'));
+  for (int i = 0; i < kNlLoads / 2; ++i) {
+    m[i] = equal_bits16(x[2 * i], '\n') | equal_bits16(x[2 * i + 1], '\n') << 16;
+    cnt += __popc(m[i]);
+  }
+  marks[w * 32 + lane] = make_uint4(m[0], m[1], m[2], m[3]);
   cnt = __reduce_add_sync(FULL, cnt);
   if (lane == 0) warp_counts[w] = cnt;
 }
 
 // The lanes collect the places of the warp's newlines in shared memory, then
 // take one newline each (its neighbours from L1, whole lines of stores).
-// Bound by DRAM and instructions alike: 355 MB of FASTQ with 4 M lines in 111
-// us (200 us with a scan per load and the stores beside it, 370 us byte by
-// byte); nl_count_kernel 63 us (190 us byte by byte).
+// What is left is the scan's instructions and the neighbours' sectors: 355 MB of
+// FASTQ with 4 M lines in 66 us from nl_count_kernel's marks (44 MB, mostly in
+// L2), 111 us when it read the text again, 200 us with a scan per load and the
+// stores beside it, 370 us byte by byte; nl_count_kernel 62 us, the text at
+// 5.7 TB/s, with or without the marks (190 us byte by byte).
 constexpr uint32_t kNlList = 1024;  // places held before they are written
 __global__ void __launch_bounds__(256)
     nl_write_kernel(const uint8_t *text, uint64_t n, uint32_t lead, const uint64_t *warp_off,
-                    uint64_t n_warps, uint64_t *nl) {
+                    uint64_t n_warps, const uint4 *marks, uint64_t *nl) {
   __shared__ uint16_t sh_list[8][kNlList];
   const uint32_t lane = threadIdx.x & 31;
   const uint64_t w = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
   if (w >= n_warps) return;
   uint16_t *const list = sh_list[threadIdx.x >> 5];
-  const int64_t w0 = (int64_t)(w * kWarpBytes) - lead, p0 = w0 + 16 * lane;
-  uint4 x[kNlLoads];
-#pragma unroll
-  for (int i = 0; i < kNlLoads; ++i) x[i] = text16(text, n, p0 + 512 * i);
+  const int64_t w0 = (int64_t)(w * kWarpBytes) - lead;
+  const uint4 mk = __ldcs(marks + w * 32 + lane);
+  const uint32_t m2[kNlLoads / 2] = {mk.x, mk.y, mk.z, mk.w};
   uint32_t mask[kNlLoads];
   // counts of four loads per word, 16 bits each, scanned over the lanes
   uint64_t cnt[kNlLoads / 4], incl[kNlLoads / 4];
@@ -202,7 +250,7 @@ __global__ void __launch_bounds__(256)
     cnt[g] = 0;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      mask[4 * g + i] = equal_bits16(x[4 * g + i], '\n');
+      mask[4 * g + i] = (m2[2 * g + i / 2] >> (16 * (i & 1))) & 0xFFFFu;
       cnt[g] |= (uint64_t)__popc(mask[4 * g + i]) << (16 * i);
     }
     incl[g] = cnt[g];
@@ -525,9 +573,10 @@ __global__ void emit_kernel(Lines L, const uint8_t *roles, const ChunkInfo *ci,
 }
 
 // ---- chunks of kFewLines lines -----------------------------------------------
-// 4 M lines: few_lines_kernel 40 us, the scan 21 us, list_lines_kernel 47 us
-// (latency of a thread's own lines); the roles by one warp per kChunkLines and
-// the one-warp fix-up took 450 us.
+// 4 M lines: few_lines_kernel 20 us, the scan 21 us, list_lines_kernel 23 us
+// (latency of a thread's own lines: 40 and 47 us when each newline's entry was
+// loaded as its line came up, instead of eight together and ahead); the roles
+// by one warp per kChunkLines and the one-warp fix-up took 450 us.
 // What a run of lines does when entered searching (0) or inside a sequence (1):
 // the state after it (kHard: none of the two) and the chars and non-empty
 // sequence lines in it; its headers are the same either way.
@@ -565,11 +614,7 @@ __global__ void __launch_bounds__(256) few_lines_kernel(Lines L, uint64_t n_chun
   uint64_t pre_chars = 0, pre_lines = 0, a = 0;
   uint32_t mode = S_SEARCH;
   bool before_special = true, plus_first = false;
-  for (uint32_t j = 0; j < n_in; ++j) {
-    uint64_t start;
-    uint32_t len;
-    uint8_t c0;
-    line_at(L, l0 + j, start, len, c0);
+  each_line(L, l0, n_in, [&](uint64_t, uint32_t len, uint8_t c0) {
     if (before_special) {
       if (is_special(len, c0)) {
         before_special = false;
@@ -585,7 +630,7 @@ __global__ void __launch_bounds__(256) few_lines_kernel(Lines L, uint64_t n_chun
       t.lines[0] += len > 0;
     }
     t.headers += role == R_HEADER;
-  }
+  });
   t.to[0] = mode == S_SEARCH ? 0 : (mode == S_SEQ ? 1 : kHard);
   t.to[1] = before_special ? 1 : (plus_first ? kHard : t.to[0]);
   t.chars[1] = pre_chars + t.chars[0];
@@ -679,11 +724,7 @@ __global__ void __launch_bounds__(256)
   const uint32_t n_in = (uint32_t)min((uint64_t)kFewLines, L.n_lines - l0);
   uint64_t at = e.chars, line = e.lines, h = e.headers, a = 0;
   uint32_t mode = e.state ? S_SEQ : S_SEARCH;
-  for (uint32_t j = 0; j < n_in; ++j) {
-    uint64_t start;
-    uint32_t len;
-    uint8_t c0;
-    line_at(L, l0 + j, start, len, c0);
+  each_line(L, l0, n_in, [&](uint64_t start, uint32_t len, uint8_t c0) {
     const uint8_t role = step(mode, a, len, c0);
     if (role == R_HEADER) {
       if (h) ends[h - 1] = at;
@@ -694,7 +735,7 @@ __global__ void __launch_bounds__(256)
       ++line;
       at += len;
     }
-  }
+  });
   if (c == n_chunks - 1) {
     line_off[status[2]] = status[0];
     if (status[1]) ends[status[1] - 1] = status[0];
@@ -804,7 +845,7 @@ __global__ void set_u64_kernel(uint64_t *p, const uint64_t *value) { *p = *value
 
 struct FastxWorkspace {
   DeviceBuffer text, warp_counts, nl, roles, chunks, chars_tot, hdr_tot, stats, chars, ends;
-  DeviceBuffer trans, tops, entries, line_off, line_src;
+  DeviceBuffer trans, tops, entries, line_off, line_src, marks;
   cudaStream_t stream = nullptr;
   u64 *host = nullptr;  // pinned: four counts
   ~FastxWorkspace() {
@@ -892,7 +933,10 @@ ParsePlan fastx_count(const uint8_t *d_text, u64 n_bytes, cudaStream_t st, Fastx
   const u64 n_warps = (lead + n_bytes + kWarpBytes - 1) / kWarpBytes;
   ws.warp_counts.ensure((n_warps + 1) * 8);
   u64 *wc = ws.warp_counts.get<u64>();
-  nl_count_kernel<<<grid_for_warps(n_warps), 256, 0, st>>>(d_text, n_bytes, lead, wc, n_warps);
+  ws.marks.ensure(n_warps * 32 * sizeof(uint4));
+  uint4 *marks = ws.marks.get<uint4>();
+  nl_count_kernel<<<grid_for_warps(n_warps), 256, 0, st>>>(d_text, n_bytes, lead, wc, n_warps,
+                                                           marks);
   enqueue_scan(wc, n_warps, ws, st);
   SBWT_CUDA(cudaMemcpyAsync(ws.host, wc + n_warps, 8, cudaMemcpyDeviceToHost, st));
   SBWT_CUDA(cudaMemcpyAsync(ws.host + 1, d_text + n_bytes - 1, 1, cudaMemcpyDeviceToHost, st));
@@ -901,7 +945,7 @@ ParsePlan fastx_count(const uint8_t *d_text, u64 n_bytes, cudaStream_t st, Fastx
   const uint8_t last = *reinterpret_cast<const uint8_t *>(ws.host + 1);
   ws.nl.ensure(std::max<u64>(n_nl, 1) * 8);
   nl_write_kernel<<<grid_for_warps(n_warps), 256, 0, st>>>(d_text, n_bytes, lead, wc, n_warps,
-                                                            ws.nl.get<u64>());
+                                                            marks, ws.nl.get<u64>());
   SBWT_CUDA(cudaGetLastError());
   P.L = Lines{d_text, n_bytes, ws.nl.get<u64>(), n_nl, n_nl + (last != '\n' ? 1 : 0)};
   if (count_few(P, st, ws)) return P;

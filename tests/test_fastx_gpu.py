@@ -129,3 +129,13 @@ def test_layouts_at_every_alignment(kind, n, tmp_path):
         assert (out[:b] == 7).all() and (out[b + len(hc):] == 7).all()
         ends = d_ends.cpu().numpy()
         assert ends[:-1].tolist() == he.tolist() and ends[-1] == -7
+
+
+@pytest.mark.parametrize("lines", [*range(1, 20), 31, 32, 33, 39, 40, 41, 63, 64, 65, 8191, 8193])
+@pytest.mark.parametrize("newline", [False, True])
+def test_line_counts_around_the_groups(lines, newline, tmp_path):
+    """Newline entries are read eight at a time, the last group's one by one:
+    every number of lines in a group, with and without a newline at the end."""
+    rng = np.random.default_rng(lines)
+    rows = [b">%d" % i if i % 5 == 0 else b"ACGTN"[:int(rng.integers(0, 6))] for i in range(lines)]
+    check_same(b"\n".join(rows) + (b"\n" if newline else b""), tmp_path)
