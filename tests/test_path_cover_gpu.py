@@ -111,3 +111,21 @@ def test_labels_of_every_k(k):
     pos = np.arange(len(chars) - k + 1, dtype=np.uint64)
     exp = oracle_index(str(path), min(k, 6)).search_positions(bits, pos)
     assert np.array_equal(idx.search(bits, pos), exp)
+
+
+def test_pipeline_batches_around_a_scan_block():
+    """One pipeline, its graph updated from batch to batch: none, one, 1024 (a
+    scan block), 1025 and more reads, in and out of order."""
+    g = genomes_of("strains", 31)
+    path = TMP / "cover_pipeline.sbwt"
+    T.build_sbwt(g, 31, str(path))
+    idx = S.SbwtIndex.open(path)
+    chars, ends = mixed_reads(g, 23, 3000, median=90, sigma=0.6, sub=0.01, n_rate=0.01, frac=0.9,
+                              len_min=0, len_max=400)
+    pipe = S.Pipeline(idx, None, len(chars), len(ends))
+    exp = oracle_results(oracle_index(str(path), 6), chars, ends)
+    for n in (3000, 1, 1024, 1025, 0, 2048, 2049, 1, 1023, 3000):
+        last = int(ends[n - 1]) if n else 0
+        k = idx.count_kmers(ends[:n])
+        assert np.array_equal(pipe.run(chars[:last], ends[:n]), exp[:k])
+    pipe.close()
