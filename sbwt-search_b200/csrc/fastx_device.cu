@@ -24,9 +24,9 @@
 //      position);
 //   4. warps copy the chars by ranges of the output, 16 bytes per lane, each
 //      lane finding its line in the list: long and short lines cost the same.
-// A chunk that ends inside quality, or is entered inside a sequence and meets a
-// '+' line first, has no such summary (multi-line FASTQ, or FASTQ whose records
-// do not start on a chunk): then the roles come from chunks of kChunkLines,
+// A chunk that is entered inside quality, or inside a sequence and meets a '+'
+// line first, has no such summary (multi-line FASTQ, or FASTQ whose records do
+// not start on a chunk): then the roles come from chunks of kChunkLines,
 // one warp per chunk, speculatively from "searching" too, and one warp walks
 // the chunks in order with the true entering state: a chunk entered
 // "searching" is right as it is; one entered inside a sequence whose first
@@ -578,9 +578,12 @@ __global__ void emit_kernel(Lines L, const uint8_t *roles, const ChunkInfo *ci,
 // loaded as its line came up, instead of eight together and ahead); the roles
 // by one warp per kChunkLines and the one-warp fix-up took 450 us.
 // What a run of lines does when entered searching (0) or inside a sequence (1):
-// the state after it (kHard: none of the two) and the chars and non-empty
-// sequence lines in it; its headers are the same either way.
-constexpr uint32_t kHard = 2;
+// the state after it (kQuality: inside quality) and the chars and non-empty
+// sequence lines in it; its headers are the same either way.  kUnknown: some
+// chunk of the run is entered inside quality, or inside a sequence and meets a
+// '+' line first (how much quality is due depends on the chunks before it): the
+// state, chars, lines and headers are not known.
+constexpr uint32_t kQuality = 2, kUnknown = 3;
 struct Trans {
   uint64_t chars[2], lines[2], headers;
   uint32_t to[2];
@@ -590,13 +593,15 @@ __device__ __forceinline__ Trans then(const Trans &a, const Trans &b) {
 #pragma unroll
   for (int s = 0; s < 2; ++s) {
     const uint32_t m = a.to[s];
-    r.to[s] = m == kHard ? kHard : (m ? b.to[1] : b.to[0]);
+    r.to[s] = m >= kQuality ? kUnknown : (m ? b.to[1] : b.to[0]);
     r.chars[s] = a.chars[s] + (m ? b.chars[1] : b.chars[0]);
     r.lines[s] = a.lines[s] + (m ? b.lines[1] : b.lines[0]);
   }
   r.headers = a.headers + b.headers;
   return r;
 }
+// The run of no lines.  To the right of a run it stands only where a chunk
+// follows (which is then entered in that run's state) or past the last chunk.
 __device__ __forceinline__ Trans no_lines() { return Trans{{0, 0}, {0, 0}, 0, {0, 1}}; }
 
 // Where a chunk starts: its entering state and what is before it.
@@ -631,8 +636,8 @@ __global__ void __launch_bounds__(256) few_lines_kernel(Lines L, uint64_t n_chun
     }
     t.headers += role == R_HEADER;
   });
-  t.to[0] = mode == S_SEARCH ? 0 : (mode == S_SEQ ? 1 : kHard);
-  t.to[1] = before_special ? 1 : (plus_first ? kHard : t.to[0]);
+  t.to[0] = mode == S_SEARCH ? 0 : (mode == S_SEQ ? 1 : kQuality);
+  t.to[1] = before_special ? 1 : (plus_first ? kUnknown : t.to[0]);
   t.chars[1] = pre_chars + t.chars[0];
   t.lines[1] = pre_lines + t.lines[0];
   out[c] = t;
@@ -691,7 +696,7 @@ __global__ void __launch_bounds__(kScanBlock) trans_tops_kernel(Trans *tops, uin
   }
 }
 // Every chunk's entry; status: chars, reads, sequence lines of the text, and 1
-// when some chunk is entered in no known state.
+// when they are not known.
 __global__ void __launch_bounds__(kScanBlock) trans_apply_kernel(const Trans *t, uint64_t n,
                                                                  const Trans *tops, Entry *entry,
                                                                  uint64_t *status) {
@@ -702,9 +707,9 @@ __global__ void __launch_bounds__(kScanBlock) trans_apply_kernel(const Trans *t,
   if (tops) x = then(tops[blockIdx.x], x);
   for (uint32_t q = 0; q < kPerThread && c0 + q < n; ++q) {
     entry[c0 + q] = Entry{x.chars[0], x.lines[0], x.headers, x.to[0]};
-    if (x.to[0] == kHard) status[3] = 1;
     x = then(x, t[c0 + q]);
-    if (c0 + q == n - 1) {
+    if (c0 + q == n - 1) {  // (a text may end inside quality)
+      status[3] = x.to[0] == kUnknown;
       status[0] = x.chars[0];
       status[1] = x.headers;
       status[2] = x.lines[0];

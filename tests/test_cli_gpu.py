@@ -102,3 +102,22 @@ def test_colors_cli_matches_oracle(tmp_path):
     csv = (tmp_path / "col_csv.csv").read_text().split("\n")[:-1]
     assert csv[0] == ",".join(str(i) for i in range(1, 41))
     assert [[i for i, x in enumerate(row.split(",")) if x == "1"] for row in csv[1:]] == exp
+
+
+def test_index_cli_on_shifted_fastq(tmp_path):
+    """A short FASTQ whose records do not start on multiples of four lines: the
+    file parsed on the device gives what the host-parsed one gives."""
+    rng = np.random.default_rng(3)
+    rows = [b"", b""]
+    for i in range(10):
+        s = bytes(rng.choice(np.frombuffer(b"ACGT", np.uint8), 60))
+        rows += [b"@r%d" % i, s, b"+", b"@" + b"I" * 59]
+    q = tmp_path / "in.fnq"
+    q.write_bytes(b"\n".join(rows) + b"\n")
+    out = []
+    for name, piece in (("device", None), ("host", "1")):
+        env = dict(os.environ, SBWT_CLI_DEVICE_PIECE_BYTES=piece) if piece else None
+        run("index", "-i", golden_sbwt_path(), "-q", q, "-o", tmp_path / name, env=env)
+        out.append((tmp_path / (name + ".txt")).read_bytes())
+    assert out[0] == out[1]
+    assert len(O.read_ascii_index_results(tmp_path / "device.txt")) == 10

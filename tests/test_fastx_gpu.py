@@ -139,3 +139,46 @@ def test_line_counts_around_the_groups(lines, newline, tmp_path):
     rng = np.random.default_rng(lines)
     rows = [b">%d" % i if i % 5 == 0 else b"ACGTN"[:int(rng.integers(0, 6))] for i in range(lines)]
     check_same(b"\n".join(rows) + (b"\n" if newline else b""), tmp_path)
+
+
+def _records(n: int, shift: int, per: int, first: bytes) -> bytes:
+    """n FASTQ records of `per` sequence and `per` quality lines after `shift`
+    blank lines; every quality line starts with `first`."""
+    rows = [b""] * shift
+    for i in range(n):
+        rows += [b"@r%d" % i, *[b"ACGT"] * per, b"+", *[first + b"II" + first] * per]
+    return b"\n".join(rows) + b"\n"
+
+
+@pytest.mark.parametrize("first", [b"@", b">", b"+", b"I"])
+@pytest.mark.parametrize("per", [1, 2])
+def test_last_group_entered_inside_a_sequence(per, first, tmp_path):
+    """Lines are summed up in groups of 32.  A group that is entered inside a
+    sequence and meets a '+' line first has no sum, the last group of a text
+    included, which no other group follows: 33 to 96 lines at every shift of
+    the records against the groups, from host and device pointers."""
+    import torch
+    L, nc, nr = S.lib(), C.c_uint64(), C.c_uint64()
+    for shift in range(4):
+        for n in range(32 // (2 + 2 * per), 96 // (2 + 2 * per) + 1):
+            text = _records(n, shift, per, first)
+            assert check_same(text, tmp_path) == n
+            hc, he = host_fastx(text, tmp_path / "in.fx")
+            d_text = torch.frombuffer(bytearray(text), dtype=torch.uint8).cuda()
+            d_chars = torch.full((len(hc) + 1,), 7, dtype=torch.uint8, device="cuda")
+            d_ends = torch.full((n + 1,), -7, dtype=torch.int64, device="cuda")
+            torch.cuda.synchronize()
+            S.check(L.sbwt_fastx_parse(d_text.data_ptr(), len(text), d_chars.data_ptr(), len(hc),
+                                       d_ends.data_ptr(), n, C.byref(nc), C.byref(nr),
+                                       S.DEVICE_POINTERS, 0, None))
+            assert (nc.value, nr.value) == (len(hc), n)
+            assert d_chars.cpu().numpy().tobytes() == hc + b"\x07"
+            assert d_ends.cpu().numpy().tolist() == [*he.tolist(), -7]
+
+
+@pytest.mark.parametrize("before", [14, 15, 16, 23_999, 39_999])
+def test_fastq_record_after_fasta(before, tmp_path):
+    """FASTA records, then one FASTQ record that may lie across the last group's
+    start; the largest has more groups than one block sums up."""
+    text = b"".join(b">%d\nAC\n" % i for i in range(before)) + b"@q\nACGT\n+\n@III\n"
+    assert check_same(text, tmp_path) == before + 1
