@@ -2,6 +2,7 @@
 // thread-local last-error message.  No exception crosses this boundary.
 #include <cstring>
 #include <memory>
+#include <mutex>
 #include <string>
 
 #include "common.hpp"
@@ -12,12 +13,17 @@
 namespace sbwt {
 static thread_local std::string g_last_error;
 void set_last_error(const std::string &msg) { g_last_error = msg; }
-LaunchConfig &default_launch_config() {
-  static LaunchConfig cfg;
-  return cfg;
+
+static std::mutex g_config_mutex;
+static LaunchConfig g_config;
+LaunchConfig default_launch_config() {
+  std::lock_guard<std::mutex> lock(g_config_mutex);
+  return g_config;
 }
-}  // namespace sbwt
-namespace sbwt {
+void change_launch_config(const std::function<void(LaunchConfig &)> &change) {
+  std::lock_guard<std::mutex> lock(g_config_mutex);
+  change(g_config);
+}
 }  // namespace sbwt
 
 using namespace sbwt;
@@ -273,17 +279,12 @@ int sbwt_search_reads_noalloc(const sbwt_index_t *index, const char *d_chars,
 // reference-facing surface): sets the process-wide launch configuration.
 int sbwt_set_launch_config(uint32_t presearch_letters, uint32_t blocks_per_sm,
                            uint64_t tile, uint64_t chunk_chars) {
-  LaunchConfig &c = default_launch_config();
-  const uint32_t probe = c.probe_len, l2w = c.l2_window, tk = c.table_kernel,
-                 bt = c.block_threads;
-  c.presearch_letters = presearch_letters;
-  c.blocks_per_sm = blocks_per_sm ? blocks_per_sm : 8;
-  c.tile = tile;
-  c.chunk_chars = chunk_chars;
-  c.probe_len = probe;
-  c.l2_window = l2w;
-  c.table_kernel = tk;
-  c.block_threads = bt;
+  change_launch_config([&](LaunchConfig &c) {
+    c.presearch_letters = presearch_letters;
+    c.blocks_per_sm = blocks_per_sm ? blocks_per_sm : 8;
+    c.tile = tile;
+    c.chunk_chars = chunk_chars;
+  });
   return SBWT_OK;
 }
 
@@ -294,7 +295,7 @@ int sbwt_set_block_threads(uint32_t threads) {
     set_last_error("block threads must be 128 or 256");
     return SBWT_E_INVALID;
   }
-  default_launch_config().block_threads = threads ? threads : 256;
+  change_launch_config([&](LaunchConfig &c) { c.block_threads = threads ? threads : 256; });
   return SBWT_OK;
 }
 
@@ -303,7 +304,7 @@ int sbwt_set_block_threads(uint32_t threads) {
 int sbwt_get_launch_config(uint32_t *presearch_letters, uint32_t *blocks_per_sm,
                            uint64_t *tile, uint64_t *chunk_chars, int *table_kernel,
                            uint32_t *block_threads) {
-  const LaunchConfig &c = default_launch_config();
+  const LaunchConfig c = default_launch_config();
   if (block_threads) *block_threads = c.block_threads;
   if (presearch_letters) *presearch_letters = c.presearch_letters;
   if (blocks_per_sm) *blocks_per_sm = c.blocks_per_sm;
@@ -316,14 +317,14 @@ int sbwt_get_launch_config(uint32_t *presearch_letters, uint32_t *blocks_per_sm,
 // Tuning hook: persisting-L2 access-policy window over the index's rank
 // blocks on the search launches (0 = off, the default; 1 = on).
 int sbwt_set_l2_window(int enabled) {
-  default_launch_config().l2_window = enabled ? 1u : 0u;
+  change_launch_config([&](LaunchConfig &c) { c.l2_window = enabled ? 1u : 0u; });
   return SBWT_OK;
 }
 
 // Tuning hook: length of the absent-prefix probe of the read search
 // (0 = automatic, 0xFFFFFFFF = off).  Results do not depend on it.
 int sbwt_set_probe_length(uint32_t probe_len) {
-  default_launch_config().probe_len = probe_len;
+  change_launch_config([&](LaunchConfig &c) { c.probe_len = probe_len; });
   return SBWT_OK;
 }
 
@@ -339,7 +340,9 @@ int sbwt_set_table_kernel(int mode) {
     set_last_error("table kernel mode must be 0..19 (or negative for the default)");
     return SBWT_E_INVALID;
   }
-  default_launch_config().table_kernel = mode < 0 ? kDefaultTableKernel : (uint32_t)mode;
+  change_launch_config([&](LaunchConfig &c) {
+    c.table_kernel = mode < 0 ? kDefaultTableKernel : (uint32_t)mode;
+  });
   return SBWT_OK;
 }
 

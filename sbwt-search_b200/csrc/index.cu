@@ -2471,6 +2471,7 @@ static uint32_t resolve_kernel_mode(const SbwtView &sv, uint32_t kernel_mode) {
   return sv.kmer_table && sv.kmer_filter && bytes <= kKmersKernelMaxBytes ? 11u : 17u;
 }
 
+// kernel_mode: resolved (BatchPlan::kernel).
 // instrument = false keeps the launch free of the profiler's events and
 // counter buffer (the allocation-free entry point).
 static void launch_search_kernel(bool stream, const SbwtView &sv, const ReadsView &rv,
@@ -2501,7 +2502,6 @@ static void launch_search_kernel(bool stream, const SbwtView &sv, const ReadsVie
   const bool narrow = sv.num_bits < kNarrowLimit && rv.n_kmers_bound < (1ULL << 32);
   const bool table = kernel_mode != 0 && stream && narrow && sv.kmer_table && sv.k <= 31 &&
                      mtk == 0 && sv.suffix_group_starts;
-  kernel_mode = resolve_kernel_mode(sv, kernel_mode);
   const bool walks = walks_kernel_applies(sv, rv, stream, mtk, kernel_mode);
   if (rv.out32 && !walks)
     throw Error(SBWT_E_INVALID, "32-bit results need the walks kernel");
@@ -3075,15 +3075,14 @@ static uint32_t probe_length(u64 num_bits, u32 k, const LaunchConfig &cfg) {
 // More than every chunk position, slot and read number of a batch.
 static u64 reads_bound(u64 n_chars, u64 n_reads) { return std::max<u64>(n_chars, n_reads) + 64; }
 
-// Whether a read search of this index runs search_paths_kernel.
-static bool paths_kernel_applies(const IndexImpl &ix, u64 n_kmers_bound, u32 flags,
-                                 const LaunchConfig &cfg) {
+// Whether a read search of this index with this (resolved) kernel runs the
+// walks kernel or one with its conditions.
+static bool walks_kernel_applies(const IndexImpl &ix, u64 n_kmers_bound, u32 flags, u32 kernel) {
   ReadsView rv{};
   rv.n_kmers_bound = n_kmers_bound;
   const bool stream = !(flags & SBWT_PER_KMER_WALK) && ix.view.suffix_group_starts;
   const u32 mtk = (flags & SBWT_MOVE_TO_KEY_KMER) ? 1u : 0u;
-  return resolve_kernel_mode(ix.view, cfg.table_kernel) == kPathsKernel &&
-         walks_kernel_applies(ix.view, rv, stream, mtk, kPathsKernel);
+  return walks_kernel_applies(ix.view, rv, stream, mtk, kernel);
 }
 
 // paths: for search_paths_kernel, where a tile costs its lane a table lookup
@@ -3107,13 +3106,18 @@ static u64 tile_size(int device, u64 n_kmers, const LaunchConfig &cfg, bool path
 
 // What a batch's preparation and search have to agree on.
 struct BatchPlan {
-  bool paths;  // search_paths_kernel runs: chars packed as entries
+  u32 kernel;  // the search kernel (resolve_kernel_mode)
+  bool walks;  // it has the walks kernel's conditions: can write 32-bit results
+  bool paths;  // it is search_paths_kernel: chars packed as entries
   u64 tile;    // k-mer slots per tile
 };
 static BatchPlan plan_batch(const IndexImpl &ix, u64 n_chars, u64 n_reads, u64 n_kmers, u32 flags,
                             const LaunchConfig &cfg) {
-  const bool paths = paths_kernel_applies(ix, reads_bound(n_chars, n_reads), flags, cfg);
-  return BatchPlan{paths, tile_size(ix.device, std::max<u64>(n_kmers, 1), cfg, paths)};
+  const u32 kernel = resolve_kernel_mode(ix.view, cfg.table_kernel);
+  const bool walks = walks_kernel_applies(ix, reads_bound(n_chars, n_reads), flags, kernel);
+  const bool paths = walks && kernel == kPathsKernel;
+  return BatchPlan{kernel, walks, paths,
+                   tile_size(ix.device, std::max<u64>(n_kmers, 1), cfg, paths)};
 }
 
 // Offsets, tile table and packed chars of a device-resident batch, with the
@@ -3227,7 +3231,7 @@ static void launch_search(const IndexImpl &ix, u64 n_chars, const u64 *d_ends, u
   launch_search_kernel(stream, sv, rv, sc.tile_read, mtk, sc.err, grid, threads, st,
                        persist ? search_attrs(ix.hot.get(), ix.window_bytes, persist)
                                : LaunchAttrs{},
-                       cfg.table_kernel, instrument);
+                       plan.kernel, instrument);
 }
 
 // The index step of one device-resident batch without any host
@@ -3268,7 +3272,7 @@ void enqueue_index_step(const IndexImpl &ix, const char *d_chars, u64 n_chars,
   const bool stream = !(flags & SBWT_PER_KMER_WALK) && ix.view.suffix_group_starts;
   const u32 mtk = (flags & SBWT_MOVE_TO_KEY_KMER) ? 1u : 0u;
   launch_search_kernel(stream, sv, rv, sc.tile_read, mtk, sc.err, grid,
-                       (int)cfg.block_threads, st, LaunchAttrs{}, cfg.table_kernel);
+                       (int)cfg.block_threads, st, LaunchAttrs{}, plan.kernel);
   note_launches(1);
 }
 
@@ -3357,13 +3361,7 @@ void IndexImpl::search_reads_device_pieces(const char *chars, u64 n_chars,
 }
 
 u32 IndexImpl::host_result_bytes(const LaunchConfig &cfg) const {
-  ReadsView probe{};
-  probe.n_kmers_bound = (64ULL << 20) + 64;
-  const SbwtView sv = view_for(cfg.presearch_letters);
-  return walks_kernel_applies(sv, probe, view.suffix_group_starts != nullptr, 0,
-                              resolve_kernel_mode(sv, cfg.table_kernel))
-             ? 4u
-             : 8u;
+  return plan_batch(*this, 64ULL << 20, 0, 64ULL << 20, 0, cfg).walks ? 4u : 8u;
 }
 
 void IndexImpl::search_reads(const char *chars, u64 n_chars, const u64 *read_ends,
@@ -3421,9 +3419,6 @@ void IndexImpl::search_reads(const char *chars, u64 n_chars, const u64 *read_end
   const bool pinned_chars = is_host_pinned(chars);
   const bool pinned_in = pinned_chars && is_host_pinned(read_ends);
   const bool pinned = pinned_in && is_host_pinned(results);
-  const SbwtView sv_host = view_for(cfg.presearch_letters);
-  const bool stream_host = !(flags & SBWT_PER_KMER_WALK) && view.suffix_group_starts;
-  const u32 mtk_host = (flags & SBWT_MOVE_TO_KEY_KMER) ? 1u : 0u;
   std::unique_ptr<HostSlices> pend;  // the chunk whose 32-bit results are in flight
   auto drain = [&]() {
     if (!pend) return;
@@ -3452,11 +3447,8 @@ void IndexImpl::search_reads(const char *chars, u64 n_chars, const u64 *read_end
     const int b = (int)(i & 1);
     cudaStream_t st = ws.streams[b];
     const u64 nc = prev - c0, nr = r1 - r0;
-    ReadsView probe{};
-    probe.n_kmers_bound = reads_bound(nc, nr);
-    const bool narrow = !pinned && walks_kernel_applies(sv_host, probe, stream_host, mtk_host,
-                                                        resolve_kernel_mode(sv_host,
-                                                                            cfg.table_kernel));
+    const BatchPlan plan = plan_batch(*this, nc, nr, nk, flags, cfg);
+    const bool narrow = !pinned && plan.walks;
     ws.chars[b].ensure(nc + 16);
     ws.ends[b].ensure(nr * 8);
     if (narrow)
@@ -3487,7 +3479,6 @@ void IndexImpl::search_reads(const char *chars, u64 n_chars, const u64 *read_end
     }
     SBWT_CUDA(cudaMemcpyAsync(ws.ends[b].get(), read_ends + r0, nr * 8,
                               cudaMemcpyHostToDevice, st));
-    const BatchPlan plan = plan_batch(*this, nc, nr, nk, flags, cfg);
     launch_prepare(device, k, ws.chars[b].get<char>(), nc, ws.ends[b].get<u64>(), nr, c0, sc, plan,
                    st);
     if (narrow) {

@@ -3,6 +3,8 @@
 
 #include <cuda_runtime.h>
 
+#include <functional>
+
 #include "common.hpp"
 #include "device_layout.hpp"
 
@@ -114,7 +116,12 @@ void enqueue_index_step(const IndexImpl &ix, const char *d_chars, u64 n_chars,
                         u64 out_capacity, u64 max_kmers, u32 flags, const LaunchConfig &cfg,
                         cudaStream_t st);
 u64 index_tile_size(const IndexImpl &ix, u64 max_kmers, const LaunchConfig &cfg);
-LaunchConfig &default_launch_config();
+
+// The process-wide launch configuration: a copy, and a change to it, both under
+// one lock.  A call takes one copy when it starts, so that a change made by
+// another thread meanwhile applies to the next call as a whole.
+LaunchConfig default_launch_config();
+void change_launch_config(const std::function<void(LaunchConfig &)> &change);
 
 }  // namespace sbwt
 

@@ -837,7 +837,7 @@ int sbwt_autotune(const sbwt_index_t *index, const char *d_chars, uint64_t n_cha
     cudaEvent_t e0, e1;
     SBWT_CUDA(cudaEventCreate(&e0));
     SBWT_CUDA(cudaEventCreate(&e1));
-    LaunchConfig saved = default_launch_config();
+    const LaunchConfig saved = default_launch_config();
     double best = 1e30;
     LaunchConfig best_cfg = saved;
     bool have_ref = false;
@@ -870,8 +870,7 @@ int sbwt_autotune(const sbwt_index_t *index, const char *d_chars, uint64_t n_cha
           c.tile = tile;
           c.blocks_per_sm = bt == 128 ? 2 * bps : bps;  // the same threads per SM
           c.block_threads = bt;
-          default_launch_config() = c;
-          u64 n = 0;
+          u64 n = 0;  // (the process-wide configuration stays as it is meanwhile)
           ix.search_reads(d_chars, nc, d_read_ends, nr, out.get<u64>(), nk, &n,
                           SBWT_DEVICE_POINTERS, st, c);  // warm
           SBWT_CUDA(cudaEventRecord(e0, st));
@@ -888,7 +887,6 @@ int sbwt_autotune(const sbwt_index_t *index, const char *d_chars, uint64_t n_cha
             h_ref = h_out;
             have_ref = true;
           } else if (h_out != h_ref) {
-            default_launch_config() = saved;
             throw Error(SBWT_E_CUDA, "autotune: a configuration changed the results");
           }
           if (ms / 3 < best) {
@@ -899,7 +897,7 @@ int sbwt_autotune(const sbwt_index_t *index, const char *d_chars, uint64_t n_cha
         }
       }
     }
-    default_launch_config() = best_cfg;
+    change_launch_config([&](LaunchConfig &c) { c = best_cfg; });
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     cudaStreamDestroy(st);

@@ -188,3 +188,75 @@ def test_concurrent_pseudoalign_on_one_handle():
     assert single[0] == oc.pseudoalign(b[4], b[2], b[3], 0.7)
     idx.close()
     ci.close()
+
+
+def test_searches_stay_exact_while_another_thread_changes_the_configuration():
+    """A call takes one copy of the launch configuration: the packing of the
+    chars and the kernel that reads it agree although kernel, tile, piece size
+    and block size change meanwhile and the autotuner sweeps."""
+    import ctypes as C
+    import torch
+    g = T.gen_genomes(79, 3, 20000, 1, 0.02, 0.02, 0.0)
+    path = str(TMP / "toggle.sbwt")
+    T.build_sbwt(g, 31, path)
+    idx = S.SbwtIndex.open(path)
+    chars, ends = mixed_reads(g, 300, 2000)
+    exp = oracle_results(oracle_index(path, 8), chars, ends)
+    d_chars = torch.from_numpy(chars.copy()).cuda()
+    d_ends = torch.from_numpy(ends.view(np.int64).copy()).cuda()
+    torch.cuda.synchronize()
+    stop, errors = threading.Event(), []
+
+    def change():
+        rng = np.random.default_rng(1)
+        while not stop.is_set():
+            S.set_table_kernel(int(rng.choice([0, 1, 2, 6, 7, 11, 17])))
+            S.set_launch_config(0, 8, int(rng.choice([0, 16, 48, 200])),
+                                int(rng.choice([0, 9000, 40000])))
+            S.set_block_threads(int(rng.choice([128, 256])))
+
+    def on_device(stream):
+        out = torch.full((len(exp) + 1,), -7, dtype=torch.int64, device="cuda")
+        torch.cuda.synchronize()
+        for i in range(150):
+            idx.search_reads(d_chars, d_ends, out=out, stream=stream.cuda_stream)
+            got = out.cpu().numpy()
+            if not np.array_equal(got[:-1].view(np.uint64), exp) or got[-1] != -7:
+                errors.append(f"device pointers, call {i}")
+                return
+
+    def on_host():
+        for i in range(150):
+            if not np.array_equal(idx.search_reads(chars, ends), exp):
+                errors.append(f"host pointers, call {i}")
+                return
+
+    def sweep():
+        p, b, t, ms = C.c_uint32(), C.c_uint32(), C.c_uint64(), C.c_double()
+        S.check(S.lib().sbwt_autotune(idx._h, d_chars.data_ptr(), d_chars.numel(),
+                                      d_ends.data_ptr(), d_ends.numel(), 1 << 20, C.byref(p),
+                                      C.byref(b), C.byref(t), C.byref(ms)))
+
+    def guard(f, *args):
+        try:
+            f(*args)
+        except Exception as e:  # reported below
+            errors.append(f"{f.__name__}: {e!r}")
+
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    changer = threading.Thread(target=guard, args=(change,))
+    work = [threading.Thread(target=guard, args=a) for a in
+            ((on_device, streams[0]), (on_device, streams[1]), (on_host,), (sweep,))]
+    try:
+        for t in [changer, *work]:
+            t.start()
+        for t in work:
+            t.join()
+    finally:
+        stop.set()
+        changer.join()
+        S.set_table_kernel()
+        S.set_launch_config()
+        S.set_block_threads()
+    assert not errors, errors
+    idx.close()
