@@ -41,6 +41,7 @@
 
 #include "index_internal.hpp"
 #include "rank_blocks.cuh"
+#include "table_budget.hpp"
 
 namespace sbwt {
 
@@ -180,7 +181,7 @@ unsigned grid_of(uint64_t n) {
 }  // namespace
 
 // Labels of all nodes; `prev` and the two arrays of n Back records are scratch,
-// key and alive lie in the one of the two that is returned last.
+// key and alive come to lie in one of the two arrays.
 template <class I>
 static void recover_labels(const SbwtView &s, u64 n, u32 k, I *prev, Back<I> *a, Back<I> *b,
                            u64 **key, u8 **alive) {
@@ -216,13 +217,16 @@ static void recover_labels(const SbwtView &s, u64 n, u32 k, I *prev, Back<I> *a,
 
 // Builds the table from the index's rank blocks.  Returns false (and builds
 // nothing) when k > 31, when the vectors' set bits are not one per node (no
-// SBWT), or when the table would not fit in kKmerTableMaxBytes or a quarter of
-// the free device memory.
+// SBWT), or when the table would not fit in kKmerTableMaxBytes or
+// kmer_table_budget of the free device memory.
 bool IndexImpl::build_kmer_table() {
   DeviceGuard g(device);
   drop_kmer_table();
   if (k > 31 || k < 2 || c_map[4] != num_bits) return false;
   const u64 n = num_bits;
+  size_t free_b = 0, total_b = 0;
+  SBWT_CUDA(cudaMemGetInfo(&free_b, &total_b));
+  const u64 budget = kmer_table_budget(free_b, n);
   // one allocation: two arrays of 16-byte records, and the predecessors
   const bool narrow = n < (1ULL << 32) - 1;
   const u64 rec_bytes = (n * 16 + 4096 + 255) / 256 * 256;
@@ -257,11 +261,9 @@ bool IndexImpl::build_kmer_table() {
   SBWT_CUDA(cudaMemcpy(&n_kmers, d_n.get(), 8, cudaMemcpyDeviceToHost));
   u64 slots = 2;
   while (slots < 2 * n_kmers) slots <<= 1;
-  size_t free_b = 0, total_b = 0;
-  SBWT_CUDA(cudaMemGetInfo(&free_b, &total_b));
   const u64 filter_words = std::max<u64>((n_kmers * kFilterBitsPerKmer + 63) / 64, 1);
   if (slots > (1ULL << 32) || slots * 16 > kKmerTableMaxBytes ||
-      slots * 16 + filter_words * 8 > free_b / 4)
+      slots * 16 + filter_words * 8 > budget)
     return false;
   // the path cover first: the table's values hold its positions.  An index
   // that cannot have it (or no memory for it) keeps the table alone.
@@ -274,7 +276,15 @@ bool IndexImpl::build_kmer_table() {
     pos = nullptr;
     drop_path_cover();
   }
-  kmer_table.resize(slots * 16);
+  try {
+    kmer_table.resize(slots * 16);
+    kmer_filter.resize(filter_words * 8);
+  } catch (const Error &e) {  // no room beside the temporaries (see kmer_table_budget)
+    if (e.code != SBWT_E_OOM) throw;
+    cudaGetLastError();
+    drop_kmer_table();
+    return false;
+  }
   SBWT_CUDA(cudaMemset(kmer_table.get(), 0xFF, slots * 16));
   table_insert_kernel<<<grid_of(n), 256>>>(key, alive, n, pos, kmer_table.get<u64>(), slots - 1,
                                            d_n.get<uint32_t>() + 2);
@@ -282,11 +292,9 @@ bool IndexImpl::build_kmer_table() {
   uint32_t e = 0;
   SBWT_CUDA(cudaMemcpy(&e, d_n.get<uint32_t>() + 2, 4, cudaMemcpyDeviceToHost));
   if (e) {
-    kmer_table.release();
-    drop_path_cover();
+    drop_kmer_table();
     throw Error(SBWT_E_FORMAT, "an SBWT k-mer occurs twice");
   }
-  kmer_filter.resize(filter_words * 8);
   SBWT_CUDA(cudaMemset(kmer_filter.get(), 0, filter_words * 8));
   filter_insert_kernel<<<grid_of(n), 256>>>(key, alive, n, kmer_filter.get<unsigned long long>(),
                                             filter_words);
