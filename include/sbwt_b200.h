@@ -389,7 +389,8 @@ int sbwt_write_color_results(const char *out_prefix, int format,
 /* ------------------------------------------------------------------------ */
 /* Process-wide launch configuration used by the search calls (0 = default):
  * presearch depth (<= the handle's), 256-thread blocks per SM, k-mer slots
- * per work tile, chars per chunk of the host-pointer pipeline. */
+ * per work tile (more than 65,536 run as 65,536), chars per chunk of the
+ * host-pointer pipeline.  A call takes one copy of it when it starts. */
 int sbwt_set_launch_config(uint32_t presearch_letters, uint32_t blocks_per_sm,
                            uint64_t tile, uint64_t chunk_chars);
 /* Length of the read search's absent-prefix probe (0 = automatic,

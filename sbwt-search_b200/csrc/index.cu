@@ -368,7 +368,7 @@ __device__ __forceinline__ void write_rows(const PrepareJob &j, uint64_t r0, uin
 
 // First launch: a block per kScanTile reads sums its k-mers and checks its
 // read ends (without `split`, the one block of the batch finishes it here), the blocks after
-// them pack the chars.  C: u32 for batches of fewer than 2^32 chars.
+// them pack the chars.  C: u32 for batches whose reads_bound is below 2^32.
 // A batch whose read ends fail the check (err bit 4) gets a total of 0 and
 // all-zero k-mer offsets: the launches queued after it then do nothing (no
 // host round trip is needed before them).
@@ -3072,8 +3072,19 @@ static uint32_t probe_length(u64 num_bits, u32 k, const LaunchConfig &cfg) {
   return L < k ? L : 0;
 }
 
-// More than every chunk position, slot and read number of a batch.
-static u64 reads_bound(u64 n_chars, u64 n_reads) { return std::max<u64>(n_chars, n_reads) + 64; }
+// The most k-mer slots of a tile.  A larger tile that the caller sets would
+// leave most lanes without work and runs as this one.
+constexpr u64 kMaxTile = 1ULL << 16;
+constexpr u64 kMaxAutoTile = 128;
+static u64 tile_max(const LaunchConfig &cfg) {
+  return cfg.tile ? std::min<u64>(cfg.tile, kMaxTile) : kMaxAutoTile;
+}
+
+// More than every chunk position, slot (a tile past the last one included) and
+// read number of a batch: below 2^32 the kernels compute with 32-bit ones.
+static u64 reads_bound(u64 n_chars, u64 n_reads, const LaunchConfig &cfg) {
+  return std::max<u64>(n_chars, n_reads) + 64 + tile_max(cfg);
+}
 
 // Whether a read search of this index with this (resolved) kernel runs the
 // walks kernel or one with its conditions.
@@ -3090,7 +3101,7 @@ static bool walks_kernel_applies(const IndexImpl &ix, u64 n_kmers_bound, u32 fla
 // with tiles of 16 / 32 / 64 / 128 slots: 63 / 74 / 90 / 124 us on 2.4 M
 // k-mers, - / 92 / 95 / 96 us on 12 M, - / 2.93 / 2.83 / 2.97 ms on 420 M.
 static u64 tile_size(int device, u64 n_kmers, const LaunchConfig &cfg, bool paths) {
-  if (cfg.tile) return cfg.tile;
+  if (cfg.tile) return tile_max(cfg);
   if (paths) {
     const u64 tile = n_kmers / ((u64)sm_count(device) * 4096);
     return (std::min<u64>(std::max<u64>(tile, 16), 64) + 15) & ~15ULL;
@@ -3101,7 +3112,7 @@ static u64 tile_size(int device, u64 n_kmers, const LaunchConfig &cfg, bool path
   // results (fewer pages and DRAM rows at a time; 10 % faster than 577 on the
   // 100 Mbp workload); a multiple of 16 slots: the walks kernels store
   // groups of up to 16 staged results
-  return (std::min<u64>(std::max<u64>(tile, 16), 128) + 15) & ~15ULL;
+  return (std::min<u64>(std::max<u64>(tile, 16), kMaxAutoTile) + 15) & ~15ULL;
 }
 
 // What a batch's preparation and search have to agree on.
@@ -3110,14 +3121,16 @@ struct BatchPlan {
   bool walks;  // it has the walks kernel's conditions: can write 32-bit results
   bool paths;  // it is search_paths_kernel: chars packed as entries
   u64 tile;    // k-mer slots per tile
+  u64 bound;   // reads_bound
 };
 static BatchPlan plan_batch(const IndexImpl &ix, u64 n_chars, u64 n_reads, u64 n_kmers, u32 flags,
                             const LaunchConfig &cfg) {
   const u32 kernel = resolve_kernel_mode(ix.view, cfg.table_kernel);
-  const bool walks = walks_kernel_applies(ix, reads_bound(n_chars, n_reads), flags, kernel);
+  const u64 bound = reads_bound(n_chars, n_reads, cfg);
+  const bool walks = walks_kernel_applies(ix, bound, flags, kernel);
   const bool paths = walks && kernel == kPathsKernel;
   return BatchPlan{kernel, walks, paths,
-                   tile_size(ix.device, std::max<u64>(n_kmers, 1), cfg, paths)};
+                   tile_size(ix.device, std::max<u64>(n_kmers, 1), cfg, paths), bound};
 }
 
 // Offsets, tile table and packed chars of a device-resident batch, with the
@@ -3162,7 +3175,7 @@ static void launch_prepare(int device, u32 k, const char *d_chars, u64 n_chars,
     j.halves = reinterpret_cast<uint2 *>(sc.packed);
     pack_blocks = (u64)grid_for(device, (2 * (n_words + 2) + 3) / 4, 256, 8);
   }
-  const bool wide = n_chars >= (1ULL << 32) - 64, aligned = ((uintptr_t)d_chars & 15) == 0;
+  const bool wide = plan.bound >= (1ULL << 32), aligned = ((uintptr_t)d_chars & 15) == 0;
   auto *const kernel = wide ? (aligned ? prepare_kernel<u64, true> : prepare_kernel<u64, false>)
                             : (aligned ? prepare_kernel<u32, true> : prepare_kernel<u32, false>);
   kernel<<<(unsigned)(j.n_blocks + pack_blocks), kScanThreads, 0, st>>>(j);
@@ -3195,7 +3208,7 @@ static void launch_search(const IndexImpl &ix, u64 n_chars, const u64 *d_ends, u
   if (n_reads == 0 || n_kmers == 0) return;
   ReadsView rv{};
   rv.out32 = d_out32;
-  rv.n_kmers_bound = reads_bound(n_chars, n_reads);
+  rv.n_kmers_bound = plan.bound;
   rv.packed = sc.packed;
   rv.entries = reinterpret_cast<const PathEntry *>(sc.packed);
   rv.invalid = sc.invalid;
@@ -3251,7 +3264,7 @@ void enqueue_index_step(const IndexImpl &ix, const char *d_chars, u64 n_chars,
   const BatchPlan plan = plan_batch(ix, n_chars, n_reads, max_kmers, flags, cfg);
   launch_prepare(ix.device, ix.k, d_chars, n_chars, d_ends, n_reads, 0, sc, plan, st);
   ReadsView rv{};
-  rv.n_kmers_bound = reads_bound(n_chars, n_reads);
+  rv.n_kmers_bound = plan.bound;
   rv.packed = sc.packed;
   rv.entries = reinterpret_cast<const PathEntry *>(sc.packed);
   rv.invalid = sc.invalid;
@@ -3375,7 +3388,8 @@ void IndexImpl::search_reads(const char *chars, u64 n_chars, const u64 *read_end
     // bits: a batch of 2^32 or more chars on an index they serve runs as
     // consecutive launches of at most 2^31 chars each (whole reads).
     if (num_bits < kNarrowLimit && n_reads &&
-        (n_chars + 64 >= (1ULL << 32) || (cfg.chunk_chars && n_chars > cfg.chunk_chars))) {
+        (reads_bound(n_chars, 0, cfg) >= (1ULL << 32) ||
+         (cfg.chunk_chars && n_chars > cfg.chunk_chars))) {
       search_reads_device_pieces(chars, n_chars, read_ends, n_reads, results, capacity,
                                  n_results, flags, user_stream, cfg);
       return;

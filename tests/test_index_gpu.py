@@ -429,3 +429,29 @@ def test_device_pointers_bad_read_ends(kernel):
     finally:
         S.set_table_kernel(DEFAULT_TABLE_KERNEL)
     idx.close()
+
+
+@pytest.mark.parametrize("kernel", [0, 1, 2, 6, 7, 11, 17])
+def test_tiles_of_any_size(kernel):
+    """A tile that the caller sets has no upper limit: sizes past 16 and 32 bits
+    give the oracle's results, from host and device pointers."""
+    import torch
+    g, path, sb = synthetic(41, 3, 5000, 31, 2, 0.02)
+    idx = S.SbwtIndex.open(path)
+    chars, ends = mixed_reads(g, 47, 1500, median=90, sigma=0.8, len_min=0, len_max=500,
+                              sub=0.01, n_rate=0.01)
+    exp = oracle_results(oracle_index(path, 8), chars, ends)
+    d_chars = torch.from_numpy(chars.copy()).cuda()
+    d_ends = torch.from_numpy(ends.view(np.int64).copy()).cuda()
+    S.set_table_kernel(kernel)
+    try:
+        for tile in (65535, 65536, 65537, 1 << 31, (1 << 32) - 1, 1 << 32, (1 << 63) + 5):
+            S.set_launch_config(tile=tile)
+            assert np.array_equal(idx.search_reads(chars, ends), exp), tile
+            out = torch.full((len(exp) + 1,), -7, dtype=torch.int64, device="cuda")
+            assert idx.search_reads(d_chars, d_ends, out=out) == len(exp)
+            got = out.cpu().numpy()
+            assert np.array_equal(got[:-1].view(np.uint64), exp) and got[-1] == -7, tile
+    finally:
+        S.set_table_kernel(DEFAULT_TABLE_KERNEL)
+        S.set_launch_config()
