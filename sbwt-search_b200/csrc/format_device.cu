@@ -220,10 +220,25 @@ __global__ void __launch_bounds__(kScanThreads) scan_apply_kernel(uint64_t *v, u
 
 // ---- ascii in tiles of tokens ------------------------------------------------
 constexpr uint32_t kTileThreads = 256, kTokens = 8, kTile = kTileThreads * kTokens;
-// Bytes of a tile that shared memory holds (16 per token); a tile with more
-// (thousands of empty reads, or tokens of 16 and more digits) is written
-// straight to its place.
+// Bytes of a tile that shared memory holds (16 per token).  A tile with more
+// (tokens of 16 and more digits), or with thousands of empty reads, which one
+// block would count one after the other, is a big one: it is filled with '\n' by
+// many blocks, and its tokens go straight to their places.
 constexpr uint32_t kTileBytes = 16 * kTile;
+// Empty reads from which on a tile is a big one.  1 M reads of which one in 10
+// (30) has 2 ids: 102 (183) us without this line, 120 (110) us at 8192.
+constexpr uint32_t kBigEmpty = 16384;
+
+// What read r, one of the empty reads between the tokens a - 1 and a, adds to a
+// count of them, mod 2^32: the last one its end, the first one its start taken
+// away, so that thousands of empty reads in a row are two additions.
+__device__ __forceinline__ uint32_t empty_share(const uint64_t *off, uint64_t n_reads, uint64_t r) {
+  const uint64_t a = off[r];
+  uint32_t share = 0;
+  if (r + 1 == n_reads || off[r + 2] != a) share += (uint32_t)r + 1;
+  if (r == 0 || off[r - 1] != a) share -= (uint32_t)r;
+  return share;
+}
 
 // One thread per read: first_read[t] = the first read r with off[r] - off[0]
 // >= t * kTile (t <= n / kTile), the empty reads of each tile, and the bit of
@@ -246,23 +261,23 @@ __global__ void tile_lines_kernel(const uint64_t *off, uint64_t n_reads, uint64_
        r0 += step) {
     const uint64_t r = r0 + lane;
     uint64_t a = 0;
-    bool none = false;
+    uint32_t share = 0;
     if (r <= n_reads) {
       a = min(off[r] - base, n);
       const uint64_t before = r ? min(off[r - 1] - base, n) : 0;
       for (uint64_t t = r ? before / kTile + 1 : 0; t <= a / kTile; ++t) first_read[t] = r;
       if (r && a > before) atomicOr(ends + (a - 1) / 32, 1u << ((a - 1) & 31));
-      none = r < n_reads && min(off[r + 1] - base, n) == a;
+      if (r < n_reads && off[r + 1] == off[r]) share = empty_share(off, n_reads, r);
     }
-    const unsigned m = __ballot_sync(FULL, none);
+    const unsigned m = __ballot_sync(FULL, share != 0);
     if (!m) continue;
     const uint64_t t = a / kTile;
     // neighbours are in the same tile nearly always: one add for them
     const int lead = __ffs(m) - 1;
     const uint64_t t0 = __shfl_sync(FULL, t, lead);
-    const unsigned same = __ballot_sync(FULL, none && t == t0);
-    if ((int)lane == lead) atomicAdd(empty + t0, __popc(same));
-    if (none && t != t0) atomicAdd(empty + t, 1u);
+    const uint32_t sum = __reduce_add_sync(FULL, t == t0 ? share : 0);
+    if ((int)lane == lead && sum) atomicAdd(empty + t0, sum);
+    if (t != t0 && share) atomicAdd(empty + t, share);
   }
 }
 
@@ -293,15 +308,17 @@ __device__ __forceinline__ void load_tokens(const V *tok, uint64_t s0, uint64_t 
 }
 
 // bytes[t]: the tile's tokens and terminators plus its empty reads; *flags
-// gets bit 0 when some tile has more bytes than shared memory holds, bit 1
-// when some tile has empty reads.  kSumTiles tiles per block, all their loads in
-// flight.
+// gets bit 0 when some tile has empty reads, and counts the big tiles from bit 1
+// on; big[i]: the i-th of them, empty[t]: its i (kNotBig for the others).
+// kSumTiles tiles per block, all their loads in flight.
+constexpr uint32_t kNotBig = ~0u;
 constexpr uint32_t kSumTiles = 2;
 constexpr uint64_t kFewTiles = 4 * kTileThreads;
 template <class V>
 __global__ void __launch_bounds__(kTileThreads) tile_bytes_kernel(const V *tok, uint64_t max_n,
                                                                   uint64_t tiles,
-                                                                  const uint32_t *empty,
+                                                                  uint32_t *empty,
+                                                                  uint32_t *big,
                                                                   uint64_t *bytes,
                                                                   uint64_t *flags) {
   const uint64_t n = min(flags[1], max_n);  // tile_lines_kernel's status
@@ -326,12 +343,18 @@ __global__ void __launch_bounds__(kTileThreads) tile_bytes_kernel(const V *tok, 
   }
   __syncthreads();
   if (threadIdx.x < kSumTiles && t0 + threadIdx.x < tiles) {
-    const uint32_t e = empty[t0 + threadIdx.x];
+    const uint64_t tile = t0 + threadIdx.x;
+    const uint32_t e = empty[tile];
     uint64_t t = e;
     for (uint32_t w = 0; w < kTileThreads / 32; ++w) t += sums[threadIdx.x][w];
-    bytes[t0 + threadIdx.x] = t;
-    if (e || t > kTileBytes)
-      atomicOr((unsigned long long *)flags, (e ? 2ULL : 0ULL) | (t > kTileBytes ? 1ULL : 0ULL));
+    bytes[tile] = t;
+    if (e) atomicOr((unsigned long long *)flags, 1ULL);
+    uint32_t at = kNotBig;
+    if (t > kTileBytes || e >= kBigEmpty) {
+      at = (uint32_t)(atomicAdd((unsigned long long *)flags, 2ULL) >> 1);
+      big[at] = (uint32_t)tile;
+    }
+    empty[tile] = at;
   }
   if (tiles > kFewTiles) return;
   // few tiles: the last block to get here turns the bytes into offsets
@@ -363,6 +386,40 @@ __device__ __forceinline__ void put_bytes(uint32_t *buf, uint32_t o, uint64_t w)
   if (u2) atomicOr(buf + (o >> 2) + 2, u2);
 }
 
+// e '\n' from o on in the zeroed buf.  A few by their thread, more by its whole
+// warp (all lanes call it): whole words by plain stores, as no other token or
+// line reaches into them.
+__device__ __forceinline__ void put_newlines(uint32_t *buf, uint32_t o, uint32_t e) {
+  constexpr uint32_t kFew = 16, kLines = 0x0A0A0A0Au;
+  if (e <= kFew)
+    for (uint32_t i = o; i < o + e; ++i) atomicOr(buf + (i >> 2), (uint32_t)'\n' << (8 * (i & 3)));
+  for (unsigned m = __ballot_sync(FULL, e > kFew); m; m &= m - 1) {
+    const uint32_t a = __shfl_sync(FULL, o, __ffs(m) - 1);
+    const uint32_t b = a + __shfl_sync(FULL, e, __ffs(m) - 1), lane = threadIdx.x & 31;
+    for (uint32_t w = (a + 3) / 4 + lane; w < b / 4; w += 32) buf[w] = kLines;
+    if (lane == 0 && (a & 3)) atomicOr(buf + a / 4, kLines << (8 * (a & 3)));
+    if (lane == 1 && (b & 3)) atomicOr(buf + b / 4, kLines >> (8 * (4 - (b & 3))));
+  }
+}
+
+// f(off[r], off[r + 1]) of the reads [r0, r1) by the whole block, eight
+// reads' loads in flight per thread.
+template <class F>
+__device__ __forceinline__ void each_read(const uint64_t *off, uint64_t r0, uint64_t r1, F f) {
+  for (uint64_t r = r0 + threadIdx.x; r < r1; r += 8 * kTileThreads) {
+    uint64_t a[8], b[8];
+#pragma unroll
+    for (uint32_t u = 0; u < 8; ++u) {
+      const uint64_t x = min(r + u * kTileThreads, r1 - 1);
+      a[u] = __ldg(off + x);
+      b[u] = __ldg(off + x + 1);
+    }
+#pragma unroll
+    for (uint32_t u = 0; u < 8; ++u)
+      if (r + u * kTileThreads < r1) f(a[u], b[u]);
+  }
+}
+
 // extra[i] = the empty reads before the token of slot i of the tile.  Slot n (in
 // the last tile) stands for the end: it has no token, only the empty reads
 // after the last one.  By the whole block; the caller waits for the counts.
@@ -373,10 +430,9 @@ __device__ __forceinline__ void count_extras(const uint64_t *off, uint64_t n_rea
   for (uint32_t i = threadIdx.x; i < kTile; i += kTileThreads) extra[i] = 0;
   __syncthreads();
   const uint64_t r_hi = s0 + kTile <= n ? first_read[tile + 1] : n_reads;
-  for (uint64_t r = first_read[tile] + threadIdx.x; r < r_hi; r += kTileThreads) {
-    const uint64_t a = min(off[r] - base, n);
-    if (min(off[r + 1] - base, n) == a && a - s0 < kTile) atomicAdd(&extra[a - s0], 1u);
-  }
+  each_read(off, first_read[tile], r_hi, [&](uint64_t a, uint64_t b) {
+    if (a == b && a - base - s0 < kTile) atomicAdd(&extra[a - base - s0], 1u);
+  });
 }
 
 struct TileShared {
@@ -422,9 +478,11 @@ __device__ __forceinline__ void write_tile(TileShared &sh, const V (&v)[kTokens]
   for (uint32_t w = 0; w < kTileThreads / 32; ++w) o += w < wid ? sh.sums[w] : 0;
 #pragma unroll
   for (uint32_t q = 0; q < kTokens; ++q) {
-    if (EXTRAS)
-      for (uint32_t e = extra[kTokens * tid + q]; e; --e, ++o)
-        atomicOr(buf + (o >> 2), (uint32_t)'\n' << (8 * (o & 3)));
+    if (EXTRAS) {
+      const uint32_t e = extra[kTokens * tid + q];
+      put_newlines(buf, o, e);
+      o += e;
+    }
     if (!len[q]) continue;
     const uint32_t term = (bits >> q) & 1u ? '\n' : ' ', end = o + len[q];
     if (is_marker(v[q])) {
@@ -483,9 +541,9 @@ __device__ __forceinline__ void write_tile(TileShared &sh, const V (&v)[kTokens]
 template <class V, bool EXTRAS>
 __global__ void __launch_bounds__(kTileThreads, 5)
     tile_ascii_kernel(const V *tok, uint64_t n, const uint64_t *off, uint64_t n_reads,
-                      const uint64_t *first_read, const uint32_t *ends,
-                      const uint64_t *tile_off, uint8_t *out, const uint64_t *status,
-                      uint64_t out_cap) {
+                      const uint64_t *first_read, const uint32_t *big_of,
+                      const uint32_t *ends, const uint64_t *tile_off, uint8_t *out,
+                      const uint64_t *status, uint64_t out_cap) {
   __shared__ TileShared sh;
   __shared__ uint32_t extra[EXTRAS ? kTile : 1];
   if (status) {
@@ -499,18 +557,21 @@ __global__ void __launch_bounds__(kTileThreads, 5)
   const uint64_t i0 = s0 + kTokens * threadIdx.x;
   const uint32_t bits = i0 < n ? __ldg(ends + i0 / 32) >> (i0 & 31) : 0;
   const uint64_t b0 = __ldg(tile_off + blockIdx.x), b1 = __ldg(tile_off + blockIdx.x + 1);
-  if (b1 == b0 || b1 - b0 > kTileBytes) return;  // past the end; tile_direct_kernel's
+  if (b1 == b0 || __ldg(big_of + blockIdx.x) != kNotBig) return;  // past the end; a big tile
   if (threadIdx.x < 32) sh.table[threadIdx.x] = kDecLen.entry[threadIdx.x];
   if (EXTRAS) count_extras(off, n_reads, n, first_read, blockIdx.x, extra);
   write_tile<V, EXTRAS>(sh, v, (uint32_t)min(n - s0, (uint64_t)kTile), bits, extra,
                         (uint32_t)(b1 - b0), out + b0);
 }
 
-// A small output (out_cap <= kSmallBytes) in one launch and one block: the
-// total, then, if it fits, the tiles one after the other.  result: the total,
-// and 1 when the block did its work (not when a tile is more than shared
-// memory holds).
+// A small output in one launch and one block: the total, then, if it fits, the
+// tiles one after the other.  result: the total, 1 when the block did its work
+// (not when a tile is big or the tokens are more than the block takes), and the
+// number of tokens.
+// More reads than kSmallReads, or fewer for each of several tiles, are faster by
+// many blocks, as this one looks at all of them for every tile.
 constexpr uint64_t kSmallBytes = kTileBytes * 3 / 2;
+constexpr uint64_t kSmallReads = 32768;
 template <class V>
 __global__ void __launch_bounds__(kTileThreads)
     small_ascii_kernel(const V *tok, const uint64_t *off, uint64_t n_reads, uint8_t *out,
@@ -521,12 +582,15 @@ __global__ void __launch_bounds__(kTileThreads)
   const uint64_t base = off[0], n = off[n_reads] - base;
   tok += base;
   if (tid < 32) sh.table[tid] = kDecLen.entry[tid];
-  if (tid == 0) result[1] = 0;
-  if (n > kSmallBytes / 2 || n_reads > kSmallBytes) return;  // at least 2 and 1 bytes each
+  if (tid == 0) {
+    result[1] = 0;
+    result[2] = n;
+  }
+  if (n > kSmallBytes / 2 || (n / kTile + 1) * n_reads > kSmallReads) return;
   __syncthreads();
   uint32_t mine = 0;  // a total of at most 21 kSmallBytes
   for (uint64_t i = tid; i < n; i += kTileThreads) mine += token_len(sh.table, tok[i]) + 1;
-  for (uint64_t r = tid; r < n_reads; r += kTileThreads) mine += off[r] == off[r + 1];
+  each_read(off, 0, n_reads, [&](uint64_t a, uint64_t b) { mine += a == b; });
   uint64_t total;
   block_exclusive(mine, &total);
   if (tid == 0) {
@@ -541,11 +605,12 @@ __global__ void __launch_bounds__(kTileThreads)
     V v[kTokens];
     load_tokens(tok, s0, n, v);
     __syncthreads();
-    for (uint64_t r = tid; r < n_reads; r += kTileThreads) {
-      const uint64_t a = off[r] - base, b = off[r + 1] - base;
+    each_read(off, 0, n_reads, [&](uint64_t a, uint64_t b) {
+      a -= base;
+      b -= base;
       if (a == b && a - s0 < kTile) atomicAdd(&extra[a - s0], 1u);
       if (a < b && b - 1 - s0 < kTile) atomicOr(&ends[(b - 1 - s0) / 32], 1u << ((b - 1) & 31));
-    }
+    });
     __syncthreads();
     mine = 0;
 #pragma unroll
@@ -566,54 +631,94 @@ __global__ void __launch_bounds__(kTileThreads)
   }
 }
 
-// The tiles that shared memory does not hold (thousands of empty reads, or
-// tokens of 16 and more digits): every token straight to its place, then the
-// lines of empty reads by the whole block.
+// ---- big tiles: any number of empty reads, tokens of any length ---------------
+// extra[i * kTile + s]: the empty reads before slot s of big tile i (zeroed by
+// big_fill_kernel).  One thread per read; big_of[t]: tile t's i.
+__global__ void big_empties_kernel(const uint64_t *off, uint64_t n_reads, const uint32_t *big_of,
+                                   uint32_t *extra) {
+  const uint64_t step = (uint64_t)gridDim.x * blockDim.x, base = off[0];
+  for (uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; r < n_reads; r += step) {
+    if (off[r + 1] != off[r]) continue;
+    const uint32_t share = empty_share(off, n_reads, r);
+    const uint64_t a = off[r] - base;
+    const uint32_t i = share ? __ldg(big_of + a / kTile) : kNotBig;
+    if (i != kNotBig) atomicAdd(extra + (uint64_t)i * kTile + a % kTile, share);
+  }
+}
+
+// '\n' into all bytes of the big tiles, 0 into extra.
+__global__ void big_fill_kernel(const uint32_t *big, uint64_t n_big, const uint64_t *tile_off,
+                                uint8_t *out, uint32_t *extra) {
+  for (uint64_t i = blockIdx.y; i < n_big; i += gridDim.y) {
+    for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < kTile; s += gridDim.x * blockDim.x)
+      extra[i * kTile + s] = 0;
+    uint8_t *const dst = out + tile_off[big[i]];
+    const uint64_t shift = (uintptr_t)dst & 15;
+    const uint64_t stop = shift + (tile_off[big[i] + 1] - tile_off[big[i]]);
+    uint8_t *const line = dst - shift;
+    const uint64_t step = 16ULL * gridDim.x * blockDim.x;
+    for (uint64_t p = 16 * (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x); p < stop; p += step) {
+      if (p >= shift && p + 16 <= stop) {
+        *reinterpret_cast<uint4 *>(line + p) =
+            make_uint4(0x0A0A0A0Au, 0x0A0A0A0Au, 0x0A0A0A0Au, 0x0A0A0A0Au);
+      } else {
+        for (uint64_t b = max(p, shift); b < min(p + 16, stop); ++b) line[b] = '\n';
+      }
+    }
+  }
+}
+
+// One block per big tile: every token straight to its place.  extra: nullptr
+// without empty reads.
 template <class V>
 __global__ void __launch_bounds__(kTileThreads)
-    tile_direct_kernel(const V *tok, uint64_t n, uint64_t tiles, const uint64_t *off,
-                       uint64_t n_reads, const uint64_t *first_read, const uint32_t *ends,
-                       const uint64_t *tile_off, uint8_t *out) {
+    big_tokens_kernel(const V *tok, uint64_t n, const uint32_t *big, uint64_t n_big,
+                      const uint32_t *extra, const uint32_t *ends, const uint64_t *tile_off,
+                      uint8_t *out) {
   __shared__ uint64_t table[32], starts[kTile];
-  __shared__ uint32_t extra[kTile];
   const uint32_t tid = threadIdx.x;
   if (tid < 32) table[tid] = kDecLen.entry[tid];
-  for (uint64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-    if (tile_off[tile + 1] - tile_off[tile] <= kTileBytes) continue;
-    const uint64_t s0 = tile * kTile;
-    uint8_t *const dst = out + tile_off[tile];
+  for (uint64_t i = blockIdx.x; i < n_big; i += gridDim.x) {
+    const uint64_t s0 = big[i] * (uint64_t)kTile;
+    const uint32_t left = (uint32_t)min(n - s0, (uint64_t)kTile);
     V v[kTokens];
     load_tokens(tok, s0, n, v);
-    const uint64_t i0 = s0 + kTokens * tid;
-    const uint32_t bits = i0 < n ? ends[i0 / 32] >> (i0 & 31) : 0;
-    count_extras(off, n_reads, n, first_read, tile, extra);
     __syncthreads();
     uint64_t mine = 0, total;
-    uint32_t len[kTokens];
+    uint32_t len[kTokens], before[kTokens];
 #pragma unroll
     for (uint32_t q = 0; q < kTokens; ++q) {
-      len[q] = i0 + q < n ? token_len(table, v[q]) : 0;
-      mine += extra[kTokens * tid + q] + (len[q] ? len[q] + 1 : 0);
+      const uint32_t sl = kTokens * tid + q;
+      len[q] = sl < left ? token_len(table, v[q]) + 1 : 0;
+      before[q] = extra ? __ldg(extra + i * kTile + sl) : 0;
+      mine += before[q] + len[q];
     }
     uint64_t at = block_exclusive(mine, &total);
 #pragma unroll
     for (uint32_t q = 0; q < kTokens; ++q) {
-      starts[kTokens * tid + q] = at;
-      at += extra[kTokens * tid + q];
-      if (!len[q]) continue;
-      if (is_marker(v[q])) {
-        dst[at] = '-';
-        dst[at + 1] = (uint64_t)v[q] == SBWT_NOT_FOUND ? '1' : '2';
-      } else {
-        uint64_t x = (uint64_t)v[q];
-        for (uint32_t i = len[q]; i-- > 0; x /= 10) dst[at + i] = (uint8_t)('0' + x % 10);
-      }
-      at += len[q];
-      dst[at++] = (bits >> q) & 1u ? '\n' : ' ';
+      starts[kTokens * tid + q] = at + before[q];
+      at += before[q] + len[q];
     }
     __syncthreads();
-    for (uint32_t sl = 0; sl < kTile; ++sl)
-      for (uint64_t e = tid; e < extra[sl]; e += kTileThreads) dst[starts[sl] + e] = '\n';
+    uint8_t *const dst = out + tile_off[big[i]];
+    for (uint32_t sl = tid; sl < left; sl += kTileThreads) {  // neighbours by neighbours
+      const V x = tok[s0 + sl];
+      uint8_t *const p = dst + starts[sl];
+      const uint32_t m = token_len(table, x);
+      if (is_marker(x)) {
+        p[0] = '-';
+        p[1] = (uint64_t)x == SBWT_NOT_FOUND ? '1' : '2';
+      } else {
+        uint64_t y = (uint64_t)x;
+        uint32_t d = m;
+        for (; y >> 32; y /= 100000000u) {  // eight digits at a time
+          uint32_t z = (uint32_t)(y % 100000000u);
+          for (uint32_t e = 0; e < 8; ++e, z /= 10) p[--d] = (uint8_t)('0' + z % 10);
+        }
+        for (uint32_t z = (uint32_t)y; d; z /= 10) p[--d] = (uint8_t)('0' + z % 10);
+      }
+      p[m] = (ends[(s0 + sl) / 32] >> (sl & 31)) & 1u ? '\n' : ' ';
+    }
     __syncthreads();
   }
 }
@@ -638,7 +743,7 @@ __global__ void __launch_bounds__(kScanThreads) scan_one_kernel(uint64_t *v, uin
 }
 
 struct FormatWorkspace {
-  DeviceBuffer kmer_off, tile_read, tile_bytes, line_bits, tops, in_a, in_b, out;
+  DeviceBuffer kmer_off, tile_read, tile_bytes, line_bits, extra, tops, in_a, in_b, out;
   cudaStream_t stream = nullptr;
   u64 *host = nullptr;  // pinned: up to four counts
   ~FormatWorkspace() {
@@ -688,23 +793,44 @@ unsigned warp_grid(u64 items) {
   return (unsigned)std::min<u64>(std::max<u64>((items + 7) / 8, 1), 148 * 64);
 }
 
-// The whole of format_tokens in one launch when the output's capacity is small
-// (a few reads): false when that did not do (what it wrote is then written again).
+// The whole of format_tokens in one launch for a small output: false when that
+// did not do (what it wrote is then written again); the number of tokens is in
+// ws.host[2] either way.
 // 100 reads of 2 color ids: 34 us a call against 47 us with a launch per step.
 template <class V>
 bool format_small(const V *tok, const uint64_t *off, u64 n_reads, uint8_t *out, u64 out_cap,
                   u64 *need, FormatWorkspace &ws, cudaStream_t st) {
-  if (out_cap == 0 || out_cap > kSmallBytes) return false;
-  ws.tile_bytes.ensure(16);
+  ws.tile_bytes.ensure(24);
   uint64_t *result = ws.tile_bytes.get<uint64_t>();
   small_ascii_kernel<V><<<1, kTileThreads, 0, st>>>(tok, off, n_reads, out, out_cap, result);
   SBWT_CUDA(cudaGetLastError());
-  SBWT_CUDA(cudaMemcpyAsync(ws.host, result, 16, cudaMemcpyDeviceToHost, st));
+  SBWT_CUDA(cudaMemcpyAsync(ws.host, result, 24, cudaMemcpyDeviceToHost, st));
   SBWT_CUDA(cudaStreamSynchronize(st));
   if (!ws.host[1]) return false;
   *need = ws.host[0];
   if (*need > out_cap) throw Error(SBWT_E_CAPACITY, "output capacity too small");
   return true;
+}
+
+// The big tiles, big[0, n_big), of format_tokens.  1 M reads without a token: 76
+// us a call; 970 us with one block for all of a tile, 166 us with a warp per read
+// and no tiles.
+template <class V>
+void format_big(const V *tok, u64 n, const uint64_t *off, u64 n_reads, bool empties,
+                const uint32_t *big, u64 n_big, const uint32_t *big_of, const uint32_t *ends,
+                const uint64_t *tile_off, uint8_t *out, FormatWorkspace &ws, cudaStream_t st) {
+  uint32_t *extra = nullptr;
+  if (empties) {
+    ws.extra.ensure(n_big * kTile * 4);
+    extra = ws.extra.get<uint32_t>();
+    big_fill_kernel<<<dim3(32, (unsigned)std::min<u64>(n_big, 148 * 4)), 256, 0, st>>>(
+        big, n_big, tile_off, out, extra);
+    big_empties_kernel<<<(unsigned)std::min<u64>(n_reads / 256 + 1, 148 * 16), 256, 0, st>>>(
+        off, n_reads, big_of, extra);
+  }
+  big_tokens_kernel<V><<<(unsigned)std::min<u64>(n_big, 148 * 16), kTileThreads, 0, st>>>(
+      tok, n, big, n_big, extra, ends, tile_off, out);
+  SBWT_CUDA(cudaGetLastError());
 }
 
 // The tokens tok[off[0], off[n_reads]) in lines (reads) of off as ascii, at
@@ -716,21 +842,22 @@ u64 format_tokens(const V *tok, u64 max_n, const uint64_t *off, u64 n_reads, uin
                   u64 out_cap, u64 *need, FormatWorkspace &ws, cudaStream_t st) {
   u64 tiles = max_n / kTile + 1;
   const u64 words = tiles * (kTile / 32);
-  ws.tile_read.ensure(tiles * 8);
+  ws.tile_read.ensure(tiles * 12);           // first reads, big tiles
   ws.tile_bytes.ensure((tiles + 5) * 8);     // offsets, total, status
   ws.line_bits.ensure((tiles + words) * 4);  // empty reads of the tiles, end bits
   uint64_t *first = ws.tile_read.get<uint64_t>(), *bytes = ws.tile_bytes.get<uint64_t>();
   uint32_t *empty = ws.line_bits.get<uint32_t>(), *ends = empty + tiles;
+  uint32_t *big = reinterpret_cast<uint32_t *>(first + tiles);
   SBWT_CUDA(cudaMemsetAsync(empty, 0, (tiles + words) * 4, st));
   tile_lines_kernel<<<(unsigned)std::min<u64>(n_reads / 256 + 1, 148 * 16), 256, 0, st>>>(
       off, n_reads, max_n, first, empty, ends, bytes + tiles + 1);
   tile_bytes_kernel<V><<<(unsigned)((tiles + kSumTiles - 1) / kSumTiles), kTileThreads, 0, st>>>(
-      tok, max_n, tiles, empty, bytes, bytes + tiles + 1);
+      tok, max_n, tiles, empty, big, bytes, bytes + tiles + 1);
   const uint64_t *const status = bytes + tiles + 1;
   const bool few = tiles <= kFewTiles;  // written before the host knows the count
   if (few)
     tile_ascii_kernel<V, true><<<(unsigned)tiles, kTileThreads, 0, st>>>(
-        tok, max_n, off, n_reads, first, ends, bytes, out, status, out_cap);
+        tok, max_n, off, n_reads, first, empty, ends, bytes, out, status, out_cap);
   const u64 total = scan_inplace(bytes, tiles, ws, st, 4, few);
   const u64 flags = ws.host[1], n = ws.host[2], base = ws.host[3];
   if (n > max_n) return format_tokens(tok, n, off, n_reads, out, out_cap, need, ws, st);
@@ -739,31 +866,33 @@ u64 format_tokens(const V *tok, u64 max_n, const uint64_t *off, u64 n_reads, uin
   tok += base;
   tiles = n / kTile + 1;
   if (!few) {
-    auto *const kernel = flags & 2 ? tile_ascii_kernel<V, true> : tile_ascii_kernel<V, false>;
-    kernel<<<(unsigned)tiles, kTileThreads, 0, st>>>(tok, n, off, n_reads, first, ends, bytes,
-                                                     out, nullptr, 0);
+    auto *const kernel = flags & 1 ? tile_ascii_kernel<V, true> : tile_ascii_kernel<V, false>;
+    kernel<<<(unsigned)tiles, kTileThreads, 0, st>>>(tok, n, off, n_reads, first, empty, ends,
+                                                     bytes, out, nullptr, 0);
   }
-  if (flags & 1)
-    tile_direct_kernel<V><<<(unsigned)std::min<u64>(tiles, 148 * 16), kTileThreads, 0, st>>>(
-        tok, n, tiles, off, n_reads, first, ends, bytes, out);
   SBWT_CUDA(cudaGetLastError());
+  if (flags >> 1)
+    format_big(tok, n, off, n_reads, flags & 1, big, flags >> 1, empty, ends, bytes, out, ws, st);
   return total;
 }
 
 // The ascii of the tokens tok[off[0], off[n_reads]).  Their count is only known
-// on the device: a small output is one launch, a medium one takes the
-// capacity's bound on the count (two bytes a token) for its tiles, and from
-// kBoundBytes on the count is read back first (a wait of ~10 us, against tiles
-// and end bits for several times the tokens).
-constexpr u64 kBoundBytes = 64ULL << 20;
+// on the device: a small capacity is one launch and a medium one bounds the
+// count (two bytes a token) for the tiles.  From kBoundBytes on the count is
+// read back first (a wait of ~10 us, against tiles and end bits for many times
+// the tokens), by the small output's launch unless there are too many reads for
+// it (100 reads of 2 color ids into 16 MB: 72 us by the bound, 41 us so).
+constexpr u64 kBoundBytes = 4ULL << 20;
 template <class V>
 u64 format_ascii(const V *tok, const uint64_t *off, u64 n_reads, uint8_t *out, u64 out_cap,
                  u64 *need, FormatWorkspace &ws, cudaStream_t st) {
-  u64 total = 0;
-  if (format_small(tok, off, n_reads, out, out_cap, need ? need : &total, ws, st))
-    return ws.host[0];
-  u64 max_n = out_cap / 2;
-  if (out_cap == 0 || out_cap > kBoundBytes) {
+  u64 total = 0, max_n = out_cap / 2;
+  const bool bound = out_cap > 0 && out_cap <= kBoundBytes;
+  if (n_reads <= kSmallReads && (!bound || out_cap <= kSmallBytes)) {
+    if (format_small(tok, off, n_reads, out, out_cap, need ? need : &total, ws, st))
+      return ws.host[0];
+    max_n = ws.host[2];
+  } else if (!bound) {
     SBWT_CUDA(cudaMemcpyAsync(ws.host, off, 8, cudaMemcpyDeviceToHost, st));
     SBWT_CUDA(cudaMemcpyAsync(ws.host + 1, off + n_reads, 8, cudaMemcpyDeviceToHost, st));
     SBWT_CUDA(cudaStreamSynchronize(st));

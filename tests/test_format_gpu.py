@@ -173,3 +173,93 @@ def test_ascii_tiles_match_host_writer(n_tokens, empty, kind):
         h = out.cpu().numpy()
         assert h[shift:shift + len(exp)].tobytes() == exp
         assert (h[:shift] == 7).all() and (h[shift + len(exp):] == 7).all()
+
+
+def _ascii_call(kind, vals, lines, cap, shift=0, k=5):
+    """Lines of the given lengths through device pointers: (code, bytes needed,
+    output with 16 bytes around it)."""
+    import torch
+    L, nb = S.lib(), C.c_uint64()
+    d_v = torch.from_numpy(np.append(vals, vals.dtype.type(0)).view(
+        np.int64 if vals.itemsize == 8 else np.int32)).cuda()
+    out = torch.full((16 + shift + cap + 16,), 7, dtype=torch.uint8, device="cuda")
+    if kind == "colors":
+        d_o = torch.from_numpy(np.concatenate([[0], np.cumsum(lines)]).astype(np.int64)).cuda()
+        torch.cuda.synchronize()
+        rc = L.sbwt_format_color_results(d_v.data_ptr(), d_o.data_ptr(), len(lines), 100, 0,
+                                         out.data_ptr() + 16 + shift, cap, C.byref(nb),
+                                         S.DEVICE_POINTERS, 0, None)
+    else:
+        d_e = torch.from_numpy(np.cumsum(np.where(lines > 0, lines + k - 1, 1))).cuda()
+        torch.cuda.synchronize()
+        rc = L.sbwt_format_index_results(d_v.data_ptr(), d_e.data_ptr(), len(lines), k, 0,
+                                         out.data_ptr() + 16 + shift, cap, C.byref(nb),
+                                         S.DEVICE_POINTERS, 0, None)
+    return rc, nb.value, out.cpu().numpy()
+
+
+def _ascii_oracle(kind, vals, lines, name, k=5):
+    if kind == "colors":
+        offs = np.concatenate([[0], np.cumsum(lines)]).astype(np.uint64)
+        return host_color_bytes(vals, offs, 100, 0, name)
+    ends = np.cumsum(np.where(lines > 0, lines + k - 1, 1)).astype(np.uint64)
+    return host_index_bytes(vals, ends, k, 0, name)
+
+
+@pytest.mark.parametrize("kind", ["index", "index_wide", "colors"])
+@pytest.mark.parametrize("n_tokens,empty,where", [
+    (0, 8192, "first"), (0, 8193, "first"), (0, 300_000, "first"), (1, 300_000, "first"),
+    (1, 300_000, "last"), (2048, 40_000, "first"), (2048, 40_000, "last"),
+    (6000, 200_000, "between"), (6000, 60_000, "spread"), (70_000, 1_000_000, "spread"),
+    (5000, 0, "none")])
+def test_ascii_of_mostly_empty_reads(n_tokens, empty, where, kind):
+    """Batches of which few reads have a token: tiles with more lines than shared
+    memory holds, whose empty reads lie before, after and between the tokens, in
+    one stretch or many; exact and large capacities, and one byte too few."""
+    rng = np.random.default_rng(n_tokens + empty)
+    n_lines = min(n_tokens, max(1, n_tokens // 3))
+    cuts = np.sort(rng.choice(np.arange(1, max(n_tokens, 2)), max(n_lines - 1, 0), replace=False))
+    sizes = np.diff(np.concatenate([[0], cuts, [n_tokens]])) if n_tokens else np.zeros(0, np.int64)
+    at = {"first": 0, "last": len(sizes), "between": len(sizes) // 2}.get(where, 0)
+    lines = np.insert(sizes, at, np.zeros(empty, np.int64))
+    if where == "spread":
+        lines = np.zeros(len(sizes) + empty, np.int64)
+        lines[np.sort(rng.choice(len(lines), len(sizes), replace=False))] = sizes
+    top = {"index": 1 << 32, "index_wide": 1 << 63, "colors": 1 << 32}[kind]
+    vals = _edge_values(rng, n_tokens, top)
+    if kind == "index_wide":  # 16 digits and more: tiles are big without empty reads too
+        vals = np.maximum(vals, np.uint64(10 ** 16))
+    if kind == "colors":
+        vals = vals.astype(np.uint32)
+    else:
+        vals[rng.random(n_tokens) < 0.1] = O.NOT_FOUND
+    exp = _ascii_oracle(kind, vals, lines, "mostly_empty")
+    for cap, shift in ((len(exp), 0), (len(exp), 5), (len(exp) + (40 << 20), 11)):
+        rc, need, out = _ascii_call(kind, vals, lines, cap, shift)
+        assert rc == S.OK and need == len(exp)
+        lo = 16 + shift
+        assert out[lo:lo + need].tobytes() == exp
+        assert (out[:lo] == 7).all() and (out[lo + need:] == 7).all()
+    rc, need, out = _ascii_call(kind, vals, lines, len(exp) - 1)
+    assert rc == S.E_CAPACITY and need == len(exp) and (out == 7).all()
+
+
+@pytest.mark.parametrize("kind", ["index", "colors"])
+@pytest.mark.parametrize("empty", [0, 300_000])
+@pytest.mark.parametrize("top", [1 << 8, 1 << 32])
+def test_ascii_of_a_large_batch(top, empty, kind):
+    """More tiles than are written before the host knows their count, by a
+    capacity that bounds the count (short tokens) and by one from which on it is
+    read back."""
+    rng = np.random.default_rng(empty + 1)
+    sizes = rng.integers(1, 200, 26_000)
+    lines = np.insert(sizes, rng.integers(0, len(sizes), empty), 0)
+    vals = _edge_values(rng, int(sizes.sum()), top)
+    if kind == "colors":
+        vals = vals.astype(np.uint32)
+    exp = _ascii_oracle(kind, vals, lines, "large")
+    assert len(vals) > 1100 * 2048 and (len(exp) > 16 << 20) == (top > 1 << 8)
+    rc, need, out = _ascii_call(kind, vals, lines, len(exp), 3)
+    assert rc == S.OK and need == len(exp)
+    assert out[19:19 + need].tobytes() == exp
+    assert (out[:19] == 7).all() and (out[19 + need:] == 7).all()
