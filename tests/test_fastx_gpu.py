@@ -182,3 +182,14 @@ def test_fastq_record_after_fasta(before, tmp_path):
     start; the largest has more groups than one block sums up."""
     text = b"".join(b">%d\nAC\n" % i for i in range(before)) + b"@q\nACGT\n+\n@III\n"
     assert check_same(text, tmp_path) == before + 1
+
+
+@pytest.mark.parametrize("first", [b"@", b">", b"+", b"I"])
+@pytest.mark.parametrize("per", [1, 3, 4, 17, 40])
+def test_fix_up_of_long_records(per, first, tmp_path):
+    """Records of 4 to 82 lines, most of them entered inside by a group of 1024
+    lines: the line on which its first guess and the truth meet lies among the
+    group's first eight lines, in one of the runs of 32 after them, or nowhere."""
+    n = 12_000 // (2 + 2 * per)
+    for shift in (1, 2, 5):
+        assert check_same(_records(n, shift, per, first), tmp_path) == n
