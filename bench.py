@@ -817,6 +817,7 @@ KERNELS = {0: "search_reads_kernel", 1: "search_table_kernel", 2: "search_walks_
 DEFAULT_KERNEL_MODE = 7
 KMERS_KERNEL_MAX_BYTES = 256 << 20  # without a cover, mode 7 picks the k-mers kernel up to this
 PATHS_KERNEL_MAX_NODES = 192 << 24  # an index with its k-mer table has its path cover below this
+PATHS_KERNEL_MIN_RATIO = 128  # possible k-mers for each of the index's from which on it always runs
 
 
 def search_kernel_name(idx, mode: int) -> str:
@@ -827,7 +828,8 @@ def search_kernel_name(idx, mode: int) -> str:
     if not table:
         return KERNELS[0]
     if mode == 7:
-        if idx.num_bits < PATHS_KERNEL_MAX_NODES:
+        if idx.num_bits < PATHS_KERNEL_MAX_NODES and \
+                4 ** idx.k >= PATHS_KERNEL_MIN_RATIO * idx.num_bits:
             return "search_paths_kernel"
         mode = 11 if 0 < idx.filter_bytes() and table + idx.filter_bytes() <= \
             KMERS_KERNEL_MAX_BYTES else 17

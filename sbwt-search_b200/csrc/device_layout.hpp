@@ -66,6 +66,7 @@ struct SbwtView {
   uint64_t node_mask;
   const uint32_t *path_node;    // node at each position of the path cover, or nullptr
   const PathEntry *path_entry;  // chars and breaks of the positions
+  uint32_t path_len;            // k-mers (positions) of the cover
   const uint64_t *lmer_filter;  // Bloom filter of the k-mers' L-mers, or nullptr
   uint32_t lmer_words;          // 64-bit words of lmer_filter
   uint32_t lmer_len;            // L (0: no filter)

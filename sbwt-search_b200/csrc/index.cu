@@ -2448,8 +2448,18 @@ static bool walks_kernel_applies(const SbwtView &sv, const ReadsView &rv, bool s
 
 // Mode 7 (automatic, the default) runs search_paths_kernel on an index with a
 // path cover (every narrow index with suffix groups whose cover fits the
-// device: it is faster than the two below at every size measured, see its
-// comment), else the k-mers kernel or the walks kernel.
+// device) unless k is so short that most k-mers branch and a run is a few k-mers
+// long: with 4^k / k-mers below 8 (no L-mer filter), or below 128 and a small
+// table, where independent lookups are the cheaper ones; else the k-mers kernel
+// or the walks kernel.  300 k reads of random / half random / 5 % / 0.5 % / 0 %
+// substituted chars, us: paths against the k-mers kernel on 2 M nodes at 9 (k =
+// 12) 1276 / 1017 / 1010 / 648 / 539 against 544 / 584 / 606 / 642 / 653, at 34
+// (k = 13) 820 / 613 / 687 / 377 / 302 against 507 / 577 / 603 / 649 / 654, at 135
+// (k = 14) 554 / 431 / 536 / 293 / 228 against 492 / 573 / 597 / 641 / 652, all
+// faster from k = 15 on; against the walks kernel with a 256 MiB table at 8 (k =
+// 13) 1316 / 1118 / 1152 / 858 / 758 against 1270 / 1182 / 1183 / 1046 / 935; 1 M
+// reads with a 2 GiB table at 4.5 (k = 14) 6.0 / 5.2 / 5.3 / 3.9 / 3.4 against 4.6
+// / 3.7 / 3.7 / 3.5 / 3.1 ms.
 // The k-mers kernel (modes 6, 11) has the walks kernel's conditions.  Mode 7
 // picks it (without a cover), with 2 k-mers per lane (mode 11: 51
 // registers, 5 blocks per SM; faster than 4 per lane at 3 blocks), when the
@@ -2466,9 +2476,12 @@ constexpr u64 kKmersKernelMaxBytes = 256ULL << 20;
 constexpr uint32_t kPathsKernel = 100;  // what mode 7 resolves to, not a mode of its own
 static uint32_t resolve_kernel_mode(const SbwtView &sv, uint32_t kernel_mode) {
   if (kernel_mode != 7) return kernel_mode;
-  if (sv.path_node) return kPathsKernel;
   const u64 bytes = (sv.kmer_table_mask + 1) * 16 + sv.filter_words * 8;
-  return sv.kmer_table && sv.kmer_filter && bytes <= kKmersKernelMaxBytes ? 11u : 17u;
+  const bool small = sv.kmer_table && sv.kmer_filter && bytes <= kKmersKernelMaxBytes;
+  // (a cover is of an index of k <= 31)
+  if (sv.path_node && sv.lmer_filter && (!small || (1ULL << (2 * sv.k)) / 128 >= sv.path_len))
+    return kPathsKernel;
+  return small ? 11u : 17u;
 }
 
 // kernel_mode: resolved (BatchPlan::kernel).

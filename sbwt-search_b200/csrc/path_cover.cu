@@ -30,7 +30,7 @@
 // (shorter than a few hundred k-mers) become paths of one k-mer each.
 //
 // L-mer filter: a blocked Bloom filter of every L-mer inside the SBWT's
-// k-mers, L = ceil(log4 k-mers) + 2.  An L-mer it rejects proves absent all
+// k-mers (L: see lmer_length).  An L-mer it rejects proves absent all
 // k - L + 1 k-mers that hold it, so the k-mers around a read error cost two
 // or three probes instead of a table lookup each.  Only the last L-mer of
 // each k-mer is inserted, and all L-mers of the k-mers without a k-mer before
@@ -310,12 +310,19 @@ unsigned grid_of(uint64_t n) {
 }
 
 // Length of the filter's L-mers: short enough that an absent one rules out
-// many k-mers, long enough that a random one is absent (about 4^-2).
+// many k-mers, long enough that a random one is absent.  With l = ceil(log4
+// k-mers): l + 2 (a random one is present at most once in 16) from k = l + 5
+// on, else l + 1, or l where k is l + 1 (an L-mer of all k chars rules out one
+// k-mer).  300 k random reads on 2 M nodes (l = 11), L = l / l + 1 / l + 2 / l +
+// 3: k = 13 920 / 820 / 1182 / 1192 us, k = 14 753 / 554 / 636 / 1043, k = 16 527
+// / 377 / 376 / 419; 1 M on 69 M nodes (l = 14), k = 15: 3.17 / 3.95 ms.
+// 0, no filter: fewer than 8 possible k-mers for each of the SBWT's.  Most L-mers
+// are in such a graph then, and the read search does not run over its cover.
 uint32_t lmer_length(u64 n_kmers, u32 k) {
   u32 lg = 0;
   while (lg < 32 && (1ULL << (2 * lg)) < n_kmers) ++lg;
-  const u32 L = std::max<u32>(lg + 2, 4);
-  return L + 4 <= k ? L : 0;
+  if ((1ULL << (2 * k)) / 8 < n_kmers) return 0;
+  return k >= lg + 5 ? std::max<u32>(lg + 2, 4) : std::min(lg + 1, k - 1);
 }
 
 }  // namespace
@@ -423,6 +430,7 @@ bool IndexImpl::build_path_cover(const u64 *key, const u8 *alive, u64 n_kmers, u
   SBWT_CUDA(cudaGetLastError());
   view.path_node = path_nodes.get<u32>();
   view.path_entry = path_entries.get<PathEntry>();
+  view.path_len = (u32)n_kmers;
   view.lmer_filter = L ? lmer_filter.get<u64>() : nullptr;
   view.lmer_words = (u32)lm_words;
   view.lmer_len = L;
@@ -435,6 +443,7 @@ void IndexImpl::drop_path_cover() {
   lmer_filter.release();
   view.path_node = nullptr;
   view.path_entry = nullptr;
+  view.path_len = 0;
   view.lmer_filter = nullptr;
   view.lmer_words = 0;
   view.lmer_len = 0;

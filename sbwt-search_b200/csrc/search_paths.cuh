@@ -4,9 +4,9 @@
 
 namespace sbwt {
 
-// Read search of an index with its path cover (the automatic choice where it
-// exists; the conditions of the walks kernel, whose tiles, work queue and
-// -1/-2 rules it shares).  A lane resolves runs of k-mers instead of k-mers:
+// Read search of an index with its path cover and L-mer filter (the automatic
+// choice as resolve_kernel_mode says; the conditions of the walks kernel, whose
+// tiles, work queue and -1/-2 rules it shares).  A lane resolves runs of k-mers instead of k-mers:
 //   P_SEED : the k-mer at pos by one table lookup: its position on the cover;
 //   P_EXT  : the read's next chars against the cover's, 32 at a time: as long
 //            as they agree (and the path does not break) the k-mers are the
@@ -229,11 +229,9 @@ __global__ void __launch_bounds__(256, kPathsBlocksPerSm)
         mode = P_EXT;
         hi = window_at(hi, lo, k);  // the chars after the k-mer
         inv >>= k;
-      } else if (L) {
+      } else {
         mode = P_MISS;
         filt = true;
-      } else {
-        run_n = 1;
       }
     }
     store(kRunsInFlight);
@@ -311,7 +309,7 @@ __global__ void __launch_bounds__(256, kPathsBlocksPerSm)
             apos = pos + run_n + n + k;
             // the k-mer before it has no other edge: absent
             const uint32_t more = __funnelshift_r(e0.branch, e1.branch, off) | (uint32_t)inv;
-            if (L && !((more >> m) & 1u)) mode = P_MISS;
+            if (!((more >> m) & 1u)) mode = P_MISS;
           }
         }
       }

@@ -129,3 +129,58 @@ def test_pipeline_batches_around_a_scan_block():
         k = idx.count_kmers(ends[:n])
         assert np.array_equal(pipe.run(chars[:last], ends[:n]), exp[:k])
     pipe.close()
+
+
+@pytest.mark.parametrize("k", [2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15, 16, 17, 18, 20, 24, 29])
+def test_reads_of_every_k(k):
+    """From graphs that hold every k-mer to ones where a run is long, over the
+    lines between the kernels and the lengths of the filter's L-mers."""
+    import torch
+    g = genomes_of("strains", k)
+    path = TMP / f"cover_reads_{k}.sbwt"
+    T.build_sbwt(g, k, str(path))
+    idx = S.SbwtIndex.open(path)
+    oracle = oracle_index(str(path), min(k, 6))
+    for sub, n_rate, frac in ((0.0, 0.0, 1.0), (0.02, 0.005, 0.7), (0.2, 0.03, 0.5)):
+        chars, ends = mixed_reads(g, 29, 600, median=90, sigma=0.8, sub=sub, n_rate=n_rate,
+                                  frac=frac, len_min=0, len_max=500)
+        exp = oracle_results(oracle, chars, ends)
+        d_chars = torch.from_numpy(chars.copy()).cuda()
+        d_ends = torch.from_numpy(ends.view(np.int64).copy()).cuda()
+        out = torch.full((len(exp) + 4,), -7, dtype=torch.int64, device="cuda")
+        assert idx.search_reads(d_chars, d_ends, out=out) == len(exp)
+        got = out.cpu().numpy()
+        assert np.array_equal(got[:len(exp)].view(np.uint64), exp)
+        assert (got[len(exp):] == -7).all()
+        assert np.array_equal(idx.search_reads(chars, ends), exp)
+
+
+@pytest.mark.parametrize("k", [12, 13, 14, 15])
+def test_short_k_with_a_large_table(k):
+    """A table past the k-mers kernel's limit and 4^k from 2 to 130 times the
+    k-mers: the automatic kernel equals the general one and the table kernel."""
+    import torch
+    rng = np.random.default_rng(31)
+    chars = np.frombuffer(b"ACGT", np.uint8)[rng.integers(0, 4, 4_150_000)]
+    path = TMP / f"cover_large_{k}.sbwt"
+    S.build_index((chars, np.array([len(chars)], np.uint64)), k, path)
+    idx = S.SbwtIndex.open(path)
+    assert idx.set_kmer_table(True) + idx.filter_bytes() > 256 << 20
+    reads = chars[:600_000].copy()
+    for a, rate in ((150_000, 0.01), (300_000, 0.1), (450_000, 0.75)):
+        hit = np.flatnonzero(rng.random(150_000) < rate) + a
+        reads[hit] = np.frombuffer(b"ACGTN", np.uint8)[rng.choice(5, len(hit), p=[.24] * 4 + [.04])]
+    ends = np.sort(rng.choice(np.arange(1, len(reads)), 5000, replace=False))
+    d_reads = torch.from_numpy(reads).cuda()
+    d_ends = torch.from_numpy(np.append(ends, len(reads)).astype(np.int64)).cuda()
+    got = []
+    try:
+        for mode in (-1, 0, 1):
+            S.set_table_kernel(mode)
+            out = torch.full((len(reads) + 1,), -7, dtype=torch.int64, device="cuda")
+            n = idx.search_reads(d_reads, d_ends, out=out)
+            got.append(out.cpu().numpy())
+            assert (got[-1][n:] == -7).all()
+    finally:
+        S.set_table_kernel()
+    assert np.array_equal(got[0], got[1]) and np.array_equal(got[0], got[2])
