@@ -3558,9 +3558,14 @@ void IndexImpl::search_positions(const u64 *bit_seqs, u64 n_words, const u64 *po
   const SbwtView sv = view_for(cfg.presearch_letters);
   const u32 mtk = (flags & SBWT_MOVE_TO_KEY_KMER) ? 1u : 0u;
   const int grid = grid_for(device, n, 256, 4 * cfg.blocks_per_sm);
-  // table kernel mode 0 keeps the presearch and steps
-  const auto kernel = sv.kmer_table && cfg.table_kernel != 0 ? search_positions_table_kernel
-                                                             : search_positions_kernel;
+  // Table kernel mode 0 keeps the presearch and steps, and so does a k that the
+  // presearch covers but for a step.  4 M positions of reads in order / shuffled /
+  // of random chars by the presearch against the table: 61 / 73 / 59 and 109 / 96 /
+  // 110 us with no step (2 M nodes, k = 11), 108 / 108 / 101 and 133 / 127 / 147
+  // with one (8 M nodes, k = 13), 132 / 158 / 120 and 120 / 124 / 132 with two
+  // (9 M nodes, k = 14).
+  const bool table = sv.kmer_table && cfg.table_kernel != 0 && k >= sv.p + 2;
+  const auto kernel = table ? search_positions_table_kernel : search_positions_kernel;
   if (flags & SBWT_DEVICE_POINTERS) {
     kernel<<<grid, 256, 0, st>>>(sv, bit_seqs, n_words * 32, positions, n, results, mtk,
                                  ws.err_dev.get<u32>());

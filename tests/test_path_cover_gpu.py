@@ -184,3 +184,26 @@ def test_short_k_with_a_large_table(k):
     finally:
         S.set_table_kernel()
     assert np.array_equal(got[0], got[1]) and np.array_equal(got[0], got[2])
+
+
+@pytest.mark.parametrize("k", [5, 12, 13, 14])
+@pytest.mark.parametrize("depth", [1, 2, 3, 4, 11, 12, 13, 14])
+def test_positions_of_every_presearch_depth(k, depth):
+    """The positions seam by presearch and steps or by the table, as k and the
+    presearch depth decide."""
+    if depth > k:
+        pytest.skip("deeper than k")
+    g = genomes_of("strains", k)
+    path = TMP / f"cover_depth_{k}.sbwt"
+    T.build_sbwt(g, k, str(path))
+    idx = S.SbwtIndex.open(path, presearch_letters=depth)
+    chars = g.chars[:len(g.chars) // 32 * 32].copy()
+    rng = np.random.default_rng(depth)
+    hit = rng.random(len(chars)) < 0.03
+    chars[hit] = np.frombuffer(b"ACGT", np.uint8)[rng.integers(0, 4, int(hit.sum()))]
+    bits, _ = O.seq_to_bits(chars.tobytes())
+    bits = bits[:len(chars) // 32]
+    pos = np.arange(len(chars) - k + 1, dtype=np.uint64)
+    pos = np.concatenate([pos, rng.permutation(pos)])
+    exp = oracle_index(str(path), min(k, 6)).search_positions(bits, pos)
+    assert np.array_equal(idx.search(bits, pos), exp)
