@@ -49,6 +49,8 @@ struct ColorsJob {
   const uint64_t *not_found;  // per read or nullptr
   const uint64_t *invalid;    // per read or nullptr
   uint64_t n_reads;
+  const uint64_t *list;     // the reads to do (n_list of them), nullptr: all
+  uint64_t n_list;
   double tau;
   uint32_t include_not_found, include_invalid;
   // mode 0: passing colors.  Of the row words of a (read, tile), those with a
@@ -235,11 +237,13 @@ __global__ void __launch_bounds__(32 * kColorWarps, P <= 8 ? 8 : (P <= 16 ? 6 : 
   stage[lane] = 0;
   __syncwarp();
   const uint64_t warps = (uint64_t)gridDim.x * kColorWarps;
-  const uint64_t n_items = job.n_reads * T;
+  const bool listed = P > kPlanes[0] && job.list;
+  const uint64_t n_items = (listed ? job.n_list : job.n_reads) * T;
   const uint64_t n_vals_end = job.offs[job.n_reads];
   for (uint64_t item = blockIdx.x * (uint64_t)kColorWarps + wid; item < n_items; item += warps) {
-    const uint64_t r = T == 1 ? item : item / T;
-    const uint32_t wbase = (uint32_t)(item - r * T) * 32;
+    const uint64_t at = T == 1 ? item : item / T;
+    const uint64_t r = listed ? __ldg(job.list + at) : at;
+    const uint32_t tile = (uint32_t)(item - at * T), wbase = 32 * tile;
     uint64_t o0 = job.offs[r], o1 = job.offs[r + 1];
     if (o1 < o0 || o1 > n_vals_end || ((o1 - o0) >> P)) {
       if (lane == 0) atomicOr(err, o1 < o0 || o1 > n_vals_end ? kErrOffsets : kErrLong);
@@ -382,7 +386,7 @@ __global__ void __launch_bounds__(32 * kColorWarps, P <= 8 ? 8 : (P <= 16 ? 6 : 
       if (ge) job.pass_bits[r * cv.row_words + wbase + __popc(mask & below)] = ge;
       const uint32_t passing = __reduce_add_sync(FULL, (uint32_t)__popcll(ge));
       if (lane == 0) {
-        job.word_mask[item] = mask;
+        job.word_mask[r * T + tile] = mask;
         if (T == 1)
           job.pass_count[r] = passing;
         else if (passing)
@@ -589,24 +593,38 @@ static void enqueue_scan_counts(const uint32_t *d_cnt, uint64_t n, uint64_t *d_o
   SBWT_CUDA(cudaGetLastError());
 }
 
-// out[0] = max over reads of offs[r + 1] - offs[r]; out[1] = 1 when some
-// offset decreases.  out is zeroed before the launch.
-__global__ void max_span_kernel(const uint64_t *offs, uint64_t n_reads,
-                                unsigned long long *out) {
+// The reads of at least `shortest` k-mers into list, their number into out[2];
+// out[0] = the longest read's k-mers; out[1] = 1 when some offset decreases.  out
+// is zeroed before the launch.
+__global__ void long_reads_kernel(const uint64_t *offs, uint64_t n_reads, uint64_t shortest,
+                                  uint64_t *list, unsigned long long *out) {
+  const uint32_t lane = threadIdx.x & 31;
   unsigned long long m = 0, bad = 0;
   const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; r < n_reads; r += step) {
-    const uint64_t a = offs[r], b = offs[r + 1];
-    if (b < a)
-      bad = 1;
-    else
-      m = max(m, (unsigned long long)(b - a));
+  for (uint64_t r0 = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) & ~31ULL; r0 < n_reads;
+       r0 += step) {
+    const uint64_t r = r0 + lane;
+    uint64_t span = 0;
+    if (r < n_reads) {
+      const uint64_t a = offs[r], b = offs[r + 1];
+      if (b < a)
+        bad = 1;
+      else
+        span = b - a;
+    }
+    m = max(m, (unsigned long long)span);
+    const uint32_t found = __ballot_sync(0xFFFFFFFFu, span >= shortest);
+    if (!found) continue;
+    unsigned long long at = 0;
+    if (lane == 0) at = atomicAdd(out + 2, (unsigned long long)__popc(found));
+    at = __shfl_sync(0xFFFFFFFFu, at, 0);
+    if ((found >> lane) & 1u) list[at + __popc(found & ((1u << lane) - 1u))] = r;
   }
   for (int o = 16; o; o >>= 1) {
     m = max(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
     bad |= __shfl_xor_sync(0xFFFFFFFFu, bad, o);
   }
-  if ((threadIdx.x & 31) == 0) {
+  if (lane == 0) {
     if (m) atomicMax(out, m);
     if (bad) atomicOr(out + 1, bad);
   }
@@ -709,7 +727,7 @@ bool ColorsImpl::set_node_table(bool enable) {
 
 struct ColorsWorkspace {
   int device = -1;
-  DeviceBuffer vals, offs, nf, inv, pass_bits, pass_count, ids_off, ids, counts, status, span;
+  DeviceBuffer vals, offs, nf, inv, pass_bits, pass_count, ids_off, ids, counts, status, span, list;
   cudaStream_t stream = nullptr;
   u64 *status_host = nullptr;  // pinned: the error bits, the id count
   uint32_t *err() { return status.get<uint32_t>(); }
@@ -744,13 +762,14 @@ static int planes_for(u64 max_kmers) {
 
 // Runs the colors kernel on device-resident arrays.  mode 0 -> passing words
 // + counts; mode 1 -> counts.  A read of 2^planes or more k-mers sets kErrLong
-// in *d_err.  d_word_mask: n_reads x tiles.
+// in *d_err.  d_word_mask: n_reads x tiles.  d_list: if set, the n_list reads
+// that are done (after a launch over all of them, with more planes).
 // One B200, 1 M reads of 120 k-mers: 2000 colors 8.31 -> 3.20 ms.
 void ColorsImpl::launch(const u64 *d_vals, const u64 *d_offs, const u64 *d_nf,
                         const u64 *d_inv, u64 n_reads, int planes, double tau,
                         u32 flags, int mode, u64 *d_pass_bits, uint32_t *d_word_mask,
                         uint32_t *d_pass_count, uint32_t *d_counts, uint32_t *d_err,
-                        cudaStream_t st) const {
+                        cudaStream_t st, const u64 *d_list, u64 n_list) const {
   if (n_reads == 0) return;
   ColorsJob job{};
   job.vals = d_vals;
@@ -758,10 +777,12 @@ void ColorsImpl::launch(const u64 *d_vals, const u64 *d_offs, const u64 *d_nf,
   job.not_found = d_nf;
   job.invalid = d_inv;
   job.n_reads = n_reads;
+  job.list = d_list;
+  job.n_list = n_list;
   job.tau = tau;
   job.include_not_found = (flags & SBWT_INCLUDE_NOT_FOUND) ? 1 : 0;
   job.include_invalid = (flags & SBWT_INCLUDE_INVALID) ? 1 : 0;
-  if (mode == 0 && view.tiles > 1)  // tiles of a read add their passing counts
+  if (mode == 0 && view.tiles > 1 && !d_list)  // tiles of a read add their passing counts
     SBWT_CUDA(cudaMemsetAsync(d_pass_count, 0, n_reads * 4, st));
   job.pass_bits = d_pass_bits;
   job.word_mask = d_word_mask;
@@ -769,7 +790,7 @@ void ColorsImpl::launch(const u64 *d_vals, const u64 *d_offs, const u64 *d_nf,
   job.counts = d_counts;
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-  const u64 items = n_reads * view.tiles;
+  const u64 items = (d_list ? n_list : n_reads) * view.tiles;
   const u64 blocks = std::min<u64>((items + kColorWarps - 1) / kColorWarps, (u64)sms * 32);
   const bool direct = view.node_rec != nullptr;
   auto go = [&](auto kernel) {
@@ -826,19 +847,22 @@ static u64 max_span(const u64 *offs, u64 n_reads) {
   return m;
 }
 
-// Longest read of device-resident offsets (one small reduction, 16 bytes back).
-static u64 device_max_span(ColorsWorkspace &ws, const u64 *d_offs, u64 n_reads,
-                           cudaStream_t st) {
-  ws.span.ensure(16);
-  SBWT_CUDA(cudaMemsetAsync(ws.span.get(), 0, 16, st));
+// The reads of device-resident offsets that the planes of short reads leave out,
+// into ws.list (their number to *n_list); returns the longest one's k-mers.
+static u64 list_long_reads(ColorsWorkspace &ws, const u64 *d_offs, u64 n_reads, cudaStream_t st,
+                           u64 *n_list) {
+  ws.span.ensure(24);
+  ws.list.ensure(n_reads * 8);
+  SBWT_CUDA(cudaMemsetAsync(ws.span.get(), 0, 24, st));
   const u64 blocks = std::min<u64>((n_reads + 255) / 256, 148 * 8);
-  max_span_kernel<<<(unsigned)std::max<u64>(blocks, 1), 256, 0, st>>>(
-      d_offs, n_reads, ws.span.get<unsigned long long>());
+  long_reads_kernel<<<(unsigned)std::max<u64>(blocks, 1), 256, 0, st>>>(
+      d_offs, n_reads, 1ULL << kPlanes[0], ws.list.get<u64>(), ws.span.get<unsigned long long>());
   SBWT_CUDA(cudaGetLastError());
-  unsigned long long h[2] = {0, 0};
-  SBWT_CUDA(cudaMemcpyAsync(h, ws.span.get(), 16, cudaMemcpyDeviceToHost, st));
+  unsigned long long h[3] = {0, 0, 0};
+  SBWT_CUDA(cudaMemcpyAsync(h, ws.span.get(), 24, cudaMemcpyDeviceToHost, st));
   SBWT_CUDA(cudaStreamSynchronize(st));
   if (h[1]) throw Error(SBWT_E_INVALID, "offsets must be non-decreasing");
+  *n_list = h[2];
   return h[0];
 }
 
@@ -852,21 +876,26 @@ static bool wait_status(ColorsWorkspace &ws, cudaStream_t st) {
   SBWT_CUDA(cudaMemsetAsync(ws.status.get(), 0, 8, st));
   SBWT_CUDA(cudaStreamSynchronize(st));
   if (e & kErrOffsets) throw Error(SBWT_E_INVALID, "offsets must be non-decreasing");
-  if (e & kErrLong) return true;
-  throw Error(SBWT_E_INVALID, "an SBWT index is not a key k-mer of this color index");
+  if (e & kErrNode)
+    throw Error(SBWT_E_INVALID, "an SBWT index is not a key k-mer of this color index");
+  return true;
 }
 
 // Device-resident batches: `run` with the planes of short reads first (the
-// longest read is only known on the device), again with the planes they need
-// when some read is longer; each time the status is read back once.
+// longest read is only known on the device), which leaves the longer ones out,
+// then over those alone with the planes they need; each time the status is read
+// back once.
+// 2000 colors, 200 k reads of 120 k-mers and one of 300: 0.85 ms, 1.63 ms with all
+// of them done again; 100 k reads of about 270: 0.97 against 1.52 ms.
 template <class F>
 static void run_planes(ColorsWorkspace &ws, const u64 *d_offs, u64 n_reads, cudaStream_t st,
                        F &&run) {
-  run(kPlanes[0]);
-  if (wait_status(ws, st)) {
-    run(planes_for(device_max_span(ws, d_offs, n_reads, st)));
-    wait_status(ws, st);
-  }
+  run(kPlanes[0], nullptr, 0);
+  if (!wait_status(ws, st)) return;
+  u64 n_list = 0;
+  const int planes = planes_for(list_long_reads(ws, d_offs, n_reads, st, &n_list));
+  run(planes, ws.list.get<u64>(), n_list);
+  wait_status(ws, st);
 }
 
 void ColorsImpl::counts(const u64 *vals, const u64 *offs, u64 n_reads, uint32_t *out,
@@ -875,9 +904,9 @@ void ColorsImpl::counts(const u64 *vals, const u64 *offs, u64 n_reads, uint32_t 
   ColorsWorkspace &ws = colors_workspace(device);
   if (n_reads == 0) return;
   if (flags & SBWT_DEVICE_POINTERS) {
-    run_planes(ws, offs, n_reads, user_stream, [&](int planes) {
+    run_planes(ws, offs, n_reads, user_stream, [&](int planes, const u64 *list, u64 n_list) {
       launch(vals, offs, nullptr, nullptr, n_reads, planes, 0.0, 0, 1, nullptr, nullptr, nullptr,
-             out, ws.err(), user_stream);
+             out, ws.err(), user_stream, list, n_list);
     });
     return;
   }
@@ -925,9 +954,9 @@ void ColorsImpl::pseudoalign(const u64 *vals, const u64 *offs, const u64 *nf,
   const u64 *d_nf = flags & SBWT_INCLUDE_NOT_FOUND ? nf : nullptr;
   const u64 *d_inv = flags & SBWT_INCLUDE_INVALID ? inv : nullptr;
   if (dev) {
-    run_planes(ws, offs, n_reads, st, [&](int planes) {
+    run_planes(ws, offs, n_reads, st, [&](int planes, const u64 *list, u64 n_list) {
       launch(vals, offs, d_nf, d_inv, n_reads, planes, tau, flags, 0, d_bits, d_mask, d_count,
-             nullptr, ws.err(), st);
+             nullptr, ws.err(), st, list, n_list);
       enqueue_scan_counts(d_count, n_reads, ids_offsets, ws.total(), st);
       emit_ids(d_bits, d_mask, ids_offsets, n_reads, ids, capacity, st);
     });

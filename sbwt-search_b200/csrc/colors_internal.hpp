@@ -65,7 +65,8 @@ struct ColorsImpl {
   void launch(const u64 *d_vals, const u64 *d_offs, const u64 *d_nf, const u64 *d_inv,
               u64 n_reads, int planes, double tau, u32 flags, int mode, u64 *d_pass_bits,
               uint32_t *d_word_mask, uint32_t *d_pass_count, uint32_t *d_counts,
-              uint32_t *d_err, cudaStream_t st) const;
+              uint32_t *d_err, cudaStream_t st, const u64 *d_list = nullptr,
+              u64 n_list = 0) const;
   void emit_ids(const u64 *d_pass_bits, const uint32_t *d_word_mask, const u64 *d_ids_off,
                 u64 n_reads, uint32_t *d_ids, u64 capacity, cudaStream_t st) const;
 

@@ -77,3 +77,54 @@ def test_decreasing_device_offsets_are_an_error():
         rc = S.lib().sbwt_color_counts(ci._h, vals.data_ptr(), d.data_ptr(), 3, out.data_ptr(),
                                        S.DEVICE_POINTERS, None)
         assert rc == S.E_INVALID
+
+
+@pytest.mark.parametrize("n_colors", [40, 2100])
+@pytest.mark.parametrize("share", [0.001, 0.3, 1.0])
+def test_long_reads_among_short_ones(n_colors, share):
+    """Device batches whose longer reads take a second launch: none but one, some
+    and all of them long, in any order; a value past the index in a read of
+    either kind is an error, and the next call is right."""
+    import torch
+    g = T.gen_genomes(37, n_colors, 150, 5, 0.01, 0.04, 0.0)
+    sp, cp = TMP / f"cl_{n_colors}.sbwt", TMP / f"cl_{n_colors}.tcolors"
+    T.build_colored(g, 31, str(sp), str(cp))
+    idx, ci = S.SbwtIndex.open(sp), S.ColorIndex.open(cp)
+    nodes = idx.search_reads(g.chars, np.cumsum(g.lens).astype(np.uint64))
+    rng = np.random.default_rng(n_colors)
+    spans = rng.integers(0, 130, 2000)
+    at = rng.choice(2000, max(1, int(2000 * share)), replace=False)
+    spans[at] = rng.integers(256, 400, len(at))
+    is_short = np.flatnonzero((spans > 0) & (spans < 256))
+    bad_reads = [int(at[0])] + [int(r) for r in is_short[:1]]
+    flat = np.concatenate([np.resize(nodes[int(rng.integers(0, len(nodes))):], n) for n in spans])
+    offs = np.concatenate([[0], np.cumsum(spans)]).astype(np.uint64)
+    oc = O.OracleColors(O.ColorsFile.read(cp))
+    zero = np.zeros(len(spans), np.uint64)
+    rows, exp = oc.pseudoalign([flat[offs[r]:offs[r + 1]] for r in range(2000)], zero, zero, 0.6,
+                               want_counts=True)
+    n_ids = sum(map(len, rows))
+    d_offs = torch.from_numpy(offs.view(np.int64).copy()).cuda()
+    for bad in (None, *bad_reads, None):
+        vals = flat.copy()
+        if bad is not None:
+            vals[offs[bad]] = 1 << 40
+        d_vals = torch.from_numpy(vals.view(np.int64).copy()).cuda()
+        io = torch.zeros(len(spans) + 1, dtype=torch.int64, device="cuda")
+        ids = torch.full((n_ids + 1,), -7, dtype=torch.int32, device="cuda")
+        counts = torch.full((2000 * n_colors + 1,), -7, dtype=torch.int32, device="cuda")
+        torch.cuda.synchronize()
+        rc = S.lib().sbwt_pseudoalign(ci._h, d_vals.data_ptr(), d_offs.data_ptr(), None, None, 2000,
+                                      C.c_double(0.6), S.DEVICE_POINTERS, ids.data_ptr(), n_ids,
+                                      io.data_ptr(), None)
+        rc2 = S.lib().sbwt_color_counts(ci._h, d_vals.data_ptr(), d_offs.data_ptr(), 2000,
+                                        counts.data_ptr(), S.DEVICE_POINTERS, None)
+        if bad is not None:
+            assert rc == S.E_INVALID and rc2 == S.E_INVALID
+            continue
+        assert rc == S.OK and rc2 == S.OK
+        h = ids.cpu().numpy()
+        assert h[:n_ids].tolist() == sum(rows, []) and h[n_ids] == -7
+        assert np.array_equal(np.diff(io.cpu().numpy()), [len(r) for r in rows])
+        h = counts.cpu().numpy()
+        assert np.array_equal(h[:-1].astype(np.uint64).reshape(exp.shape), exp) and h[-1] == -7
