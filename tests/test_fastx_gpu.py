@@ -193,3 +193,48 @@ def test_fix_up_of_long_records(per, first, tmp_path):
     n = 12_000 // (2 + 2 * per)
     for shift in (1, 2, 5):
         assert check_same(_records(n, shift, per, first), tmp_path) == n
+
+
+@pytest.mark.parametrize("kind", ["fastq", "short lines", "long lines"])
+@pytest.mark.parametrize("lead", [0, 5])
+def test_large_text(kind, lead, tmp_path):
+    """Texts past the sizes of one block's scan of the newline counts (33 MB) and
+    of the copy's smallest range (9.7 M output chars): reads of 0 to 400 chars,
+    10 M lines of one or two chars, and lines of up to 3 MB, with text and output
+    on and off a 16-byte boundary."""
+    import torch
+    rng = np.random.default_rng(len(kind))
+    seq = np.frombuffer(b"ACGTN", np.uint8)[rng.integers(0, 5, 4 << 20)].tobytes()
+    if kind == "fastq":
+        at, n = rng.integers(0, len(seq) - 400, 120_000), rng.integers(0, 401, 120_000)
+        text = b"".join(b"@%d\n%s\n+\n%s\n" % (i, seq[a:a + m], b"I" * m)
+                        for i, (a, m) in enumerate(zip(at, n)))
+    elif kind == "short lines":
+        lines = np.full((10_500_000, 3), ord("\n"), np.uint8)
+        lines[:, 0] = np.frombuffer(b"ACGT", np.uint8)[rng.integers(0, 4, len(lines))]
+        two = rng.random(len(lines)) < 0.3
+        lines[two, 1] = ord("G")
+        lines[rng.integers(0, len(lines), 1000), 0] = ord(">")
+        keep = np.ones(lines.shape, bool)
+        keep[~two, 2] = False
+        text = b">x\n" + lines[keep].tobytes() + b">y\nA"
+    else:
+        text = b"".join(b">%d\n%s\n" % (i, seq[a:a + m]) for i, (a, m) in enumerate(
+            zip(rng.integers(0, 1 << 20, 30), rng.integers(0, 3_000_000, 30))))
+    assert len(text) > 22_000_000
+    hc, he = host_fastx(text, tmp_path / "in.fx")
+    assert len(hc) > 10_000_000
+    d_text = torch.from_numpy(np.frombuffer(b"\n" * lead + text, np.uint8).copy()).cuda()
+    d_chars = torch.full((lead + len(hc) + 16,), 7, dtype=torch.uint8, device="cuda")
+    d_ends = torch.full((len(he) + 1,), -7, dtype=torch.int64, device="cuda")
+    nc, nr = C.c_uint64(), C.c_uint64()
+    torch.cuda.synchronize()
+    S.check(S.lib().sbwt_fastx_parse(d_text.data_ptr() + lead, len(text),
+                                     d_chars.data_ptr() + lead, len(hc), d_ends.data_ptr(),
+                                     len(he), C.byref(nc), C.byref(nr), S.DEVICE_POINTERS, 0, None))
+    assert (nc.value, nr.value) == (len(hc), len(he))
+    h = d_chars.cpu().numpy()
+    assert h[lead:lead + len(hc)].tobytes() == hc
+    assert (h[:lead] == 7).all() and (h[lead + len(hc):] == 7).all()
+    e = d_ends.cpu().numpy()
+    assert np.array_equal(e[:-1].view(np.uint64), he) and e[-1] == -7

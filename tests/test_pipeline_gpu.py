@@ -145,3 +145,28 @@ def test_server_admits_slots_by_free_device_memory():
     assert got == exp
     assert 1 <= srv.slots()["open"] <= 4
     srv.close()
+
+
+@pytest.mark.parametrize("n_colors", [150, 2100])
+def test_more_ids_than_the_staging_holds(n_colors):
+    """A batch that passes more than 64 ids per read of the pipeline's size, whose
+    ids the host takes from the passing words (one color tile and two), then
+    batches that fit on the same pipeline: nothing of the large one is left."""
+    g, sp, cp = colored(9, n_colors, 200, 1)
+    idx, ci = S.SbwtIndex.open(sp), S.ColorIndex.open(cp)
+    p = S.Pipeline(idx, ci, 1 << 16, 8, tau=0.05)
+    oc = O.OracleColors(O.ColorsFile.read(cp))
+    chars, ends = T.gen_reads(3, g, 8, 1.0, 120, 0.0, 20, 400, 0.0, 0.0)
+    noise = np.full(len(chars), ord("A"), np.uint8)
+    for source, n in ((chars, 8), (noise, 8), (chars, 8), (chars, 1), (noise, 1)):
+        e = ends[:n]
+        c = source[:int(e[-1])]
+        res = idx.search_reads(c, e)
+        per = np.split(res, np.cumsum([max(0, len(r) - 30) for r in T.split_reads(c, e)])[:-1])
+        found = [x[x < O.INVALID] for x in per]
+        exp = oc.pseudoalign(found, [0] * n, [0] * n, 0.05)
+        assert source is noise or n < 8 or sum(map(len, exp)) > 8 * 64
+        assert p.run(c, e) == exp
+        ids, offs = p.run(c, e, raw=True)
+        assert len(ids) == sum(map(len, exp)) == int(offs[-1])
+    p.close()
