@@ -225,9 +225,9 @@ constexpr uint32_t kTileThreads = 256, kTokens = 8, kTile = kTileThreads * kToke
 // block would count one after the other, is a big one: it is filled with '\n' by
 // many blocks, and its tokens go straight to their places.
 constexpr uint32_t kTileBytes = 16 * kTile;
-// Empty reads from which on a tile is a big one.  1 M reads of which one in 10
-// (30) has 2 ids: 102 (183) us without this line, 120 (110) us at 8192.
-constexpr uint32_t kBigEmpty = 16384;
+// Empty reads from which on a tile is a big one.  1 M reads of which one in 20
+// has 2 ids (19,000 of them a tile): 94 us here, 112 us at 16384.
+constexpr uint32_t kBigEmpty = 24576;
 
 // What read r, one of the empty reads between the tokens a - 1 and a, adds to a
 // count of them, mod 2^32: the last one its end, the first one its start taken
@@ -309,9 +309,9 @@ __device__ __forceinline__ void load_tokens(const V *tok, uint64_t s0, uint64_t 
 
 // bytes[t]: the tile's tokens and terminators plus its empty reads; *flags
 // gets bit 0 when some tile has empty reads, and counts the big tiles from bit 1
-// on; big[i]: the i-th of them, empty[t]: its i (kNotBig for the others).
-// kSumTiles tiles per block, all their loads in flight.
-constexpr uint32_t kNotBig = ~0u;
+// on; big[i]: the i-th of them, whose empty[t] becomes kBig | i (a store for every
+// tile took 7 % longer).  kSumTiles tiles per block, all their loads in flight.
+constexpr uint32_t kBig = 1u << 31;
 constexpr uint32_t kSumTiles = 2;
 constexpr uint64_t kFewTiles = 4 * kTileThreads;
 template <class V>
@@ -349,12 +349,11 @@ __global__ void __launch_bounds__(kTileThreads) tile_bytes_kernel(const V *tok, 
     for (uint32_t w = 0; w < kTileThreads / 32; ++w) t += sums[threadIdx.x][w];
     bytes[tile] = t;
     if (e) atomicOr((unsigned long long *)flags, 1ULL);
-    uint32_t at = kNotBig;
     if (t > kTileBytes || e >= kBigEmpty) {
-      at = (uint32_t)(atomicAdd((unsigned long long *)flags, 2ULL) >> 1);
+      const uint32_t at = (uint32_t)(atomicAdd((unsigned long long *)flags, 2ULL) >> 1);
       big[at] = (uint32_t)tile;
+      empty[tile] = kBig | at;
     }
-    empty[tile] = at;
   }
   if (tiles > kFewTiles) return;
   // few tiles: the last block to get here turns the bytes into offsets
@@ -386,37 +385,42 @@ __device__ __forceinline__ void put_bytes(uint32_t *buf, uint32_t o, uint64_t w)
   if (u2) atomicOr(buf + (o >> 2) + 2, u2);
 }
 
-// e '\n' from o on in the zeroed buf.  A few by their thread, more by its whole
-// warp (all lanes call it): whole words by plain stores, as no other token or
-// line reaches into them.
-__device__ __forceinline__ void put_newlines(uint32_t *buf, uint32_t o, uint32_t e) {
-  constexpr uint32_t kFew = 16, kLines = 0x0A0A0A0Au;
-  if (e <= kFew)
-    for (uint32_t i = o; i < o + e; ++i) atomicOr(buf + (i >> 2), (uint32_t)'\n' << (8 * (i & 3)));
-  for (unsigned m = __ballot_sync(FULL, e > kFew); m; m &= m - 1) {
-    const uint32_t a = __shfl_sync(FULL, o, __ffs(m) - 1);
-    const uint32_t b = a + __shfl_sync(FULL, e, __ffs(m) - 1), lane = threadIdx.x & 31;
-    for (uint32_t w = (a + 3) / 4 + lane; w < b / 4; w += 32) buf[w] = kLines;
-    if (lane == 0 && (a & 3)) atomicOr(buf + a / 4, kLines << (8 * (a & 3)));
-    if (lane == 1 && (b & 3)) atomicOr(buf + b / 4, kLines >> (8 * (4 - (b & 3))));
+// e '\n' from o on in the zeroed buf.  A few by their thread; where a thread of
+// the warp has more (many: the same for all its lanes, which all call it), those
+// by the whole warp: whole words by plain stores, as no other token or line
+// reaches into them.
+constexpr uint32_t kFewLines = 64;
+__device__ __forceinline__ void put_newlines(uint32_t *buf, uint32_t o, uint32_t e, bool many) {
+  constexpr uint32_t kLines = 0x0A0A0A0Au;
+  if (many) {
+    for (unsigned m = __ballot_sync(FULL, e > kFewLines); m; m &= m - 1) {
+      const uint32_t a = __shfl_sync(FULL, o, __ffs(m) - 1);
+      const uint32_t b = a + __shfl_sync(FULL, e, __ffs(m) - 1), lane = threadIdx.x & 31;
+      for (uint32_t w = (a + 3) / 4 + lane; w < b / 4; w += 32) buf[w] = kLines;
+      if (lane == 0 && (a & 3)) atomicOr(buf + a / 4, kLines << (8 * (a & 3)));
+      if (lane == 1 && (b & 3)) atomicOr(buf + b / 4, kLines >> (8 * (4 - (b & 3))));
+    }
+    if (e > kFewLines) return;
   }
+  for (; e; --e, ++o) atomicOr(buf + (o >> 2), (uint32_t)'\n' << (8 * (o & 3)));
 }
 
-// f(off[r], off[r + 1]) of the reads [r0, r1) by the whole block, eight
-// reads' loads in flight per thread.
+// f(off[r], off[r + 1]) of all reads by the whole block, eight reads' loads in
+// flight per thread.
 template <class F>
-__device__ __forceinline__ void each_read(const uint64_t *off, uint64_t r0, uint64_t r1, F f) {
-  for (uint64_t r = r0 + threadIdx.x; r < r1; r += 8 * kTileThreads) {
-    uint64_t a[8], b[8];
+__device__ __forceinline__ void each_read(const uint64_t *off, uint64_t n_reads, F f) {
+  constexpr uint32_t U = 8;
+  for (uint64_t r = threadIdx.x; r < n_reads; r += U * kTileThreads) {
+    uint64_t a[U], b[U];
 #pragma unroll
-    for (uint32_t u = 0; u < 8; ++u) {
-      const uint64_t x = min(r + u * kTileThreads, r1 - 1);
+    for (uint32_t u = 0; u < U; ++u) {
+      const uint64_t x = min(r + u * kTileThreads, n_reads - 1);
       a[u] = __ldg(off + x);
       b[u] = __ldg(off + x + 1);
     }
 #pragma unroll
-    for (uint32_t u = 0; u < 8; ++u)
-      if (r + u * kTileThreads < r1) f(a[u], b[u]);
+    for (uint32_t u = 0; u < U; ++u)
+      if (r + u * kTileThreads < n_reads) f(a[u], b[u]);
   }
 }
 
@@ -430,9 +434,10 @@ __device__ __forceinline__ void count_extras(const uint64_t *off, uint64_t n_rea
   for (uint32_t i = threadIdx.x; i < kTile; i += kTileThreads) extra[i] = 0;
   __syncthreads();
   const uint64_t r_hi = s0 + kTile <= n ? first_read[tile + 1] : n_reads;
-  each_read(off, first_read[tile], r_hi, [&](uint64_t a, uint64_t b) {
-    if (a == b && a - base - s0 < kTile) atomicAdd(&extra[a - base - s0], 1u);
-  });
+  for (uint64_t r = first_read[tile] + threadIdx.x; r < r_hi; r += kTileThreads) {
+    const uint64_t a = off[r] - base;
+    if (off[r + 1] - base == a && a - s0 < kTile) atomicAdd(&extra[a - s0], 1u);
+  }
 }
 
 struct TileShared {
@@ -458,13 +463,17 @@ __device__ __forceinline__ void write_tile(TileShared &sh, const V (&v)[kTokens]
   for (uint32_t i = tid; 16 * i < stop; i += kTileThreads)
     reinterpret_cast<uint4 *>(buf)[i] = make_uint4(0, 0, 0, 0);
   __syncthreads();
-  uint32_t len[kTokens], mine = 0;
+  uint32_t len[kTokens], mine = 0, most = 0;
 #pragma unroll
   for (uint32_t q = 0; q < kTokens; ++q) {
     len[q] = kTokens * tid + q < left ? token_len(sh.table, v[q]) + 1 : 0;
     mine += len[q];
-    if (EXTRAS) mine += extra[kTokens * tid + q];
+    if (EXTRAS) {
+      mine += extra[kTokens * tid + q];
+      most = max(most, extra[kTokens * tid + q]);
+    }
   }
+  const bool many = EXTRAS && __any_sync(FULL, most > kFewLines);
   uint32_t x = mine;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
@@ -480,7 +489,7 @@ __device__ __forceinline__ void write_tile(TileShared &sh, const V (&v)[kTokens]
   for (uint32_t q = 0; q < kTokens; ++q) {
     if (EXTRAS) {
       const uint32_t e = extra[kTokens * tid + q];
-      put_newlines(buf, o, e);
+      put_newlines(buf, o, e, many);
       o += e;
     }
     if (!len[q]) continue;
@@ -541,7 +550,7 @@ __device__ __forceinline__ void write_tile(TileShared &sh, const V (&v)[kTokens]
 template <class V, bool EXTRAS>
 __global__ void __launch_bounds__(kTileThreads, 5)
     tile_ascii_kernel(const V *tok, uint64_t n, const uint64_t *off, uint64_t n_reads,
-                      const uint64_t *first_read, const uint32_t *big_of,
+                      const uint64_t *first_read, const uint32_t *empty,
                       const uint32_t *ends, const uint64_t *tile_off, uint8_t *out,
                       const uint64_t *status, uint64_t out_cap) {
   __shared__ TileShared sh;
@@ -557,7 +566,9 @@ __global__ void __launch_bounds__(kTileThreads, 5)
   const uint64_t i0 = s0 + kTokens * threadIdx.x;
   const uint32_t bits = i0 < n ? __ldg(ends + i0 / 32) >> (i0 & 31) : 0;
   const uint64_t b0 = __ldg(tile_off + blockIdx.x), b1 = __ldg(tile_off + blockIdx.x + 1);
-  if (b1 == b0 || __ldg(big_of + blockIdx.x) != kNotBig) return;  // past the end; a big tile
+  if (b1 == b0) return;  // past the end
+  // a big tile (without empty reads only by its bytes)
+  if (EXTRAS ? __ldg(empty + blockIdx.x) >= kBig : b1 - b0 > kTileBytes) return;
   if (threadIdx.x < 32) sh.table[threadIdx.x] = kDecLen.entry[threadIdx.x];
   if (EXTRAS) count_extras(off, n_reads, n, first_read, blockIdx.x, extra);
   write_tile<V, EXTRAS>(sh, v, (uint32_t)min(n - s0, (uint64_t)kTile), bits, extra,
@@ -590,7 +601,7 @@ __global__ void __launch_bounds__(kTileThreads)
   __syncthreads();
   uint32_t mine = 0;  // a total of at most 21 kSmallBytes
   for (uint64_t i = tid; i < n; i += kTileThreads) mine += token_len(sh.table, tok[i]) + 1;
-  each_read(off, 0, n_reads, [&](uint64_t a, uint64_t b) { mine += a == b; });
+  each_read(off, n_reads, [&](uint64_t a, uint64_t b) { mine += a == b; });
   uint64_t total;
   block_exclusive(mine, &total);
   if (tid == 0) {
@@ -605,7 +616,7 @@ __global__ void __launch_bounds__(kTileThreads)
     V v[kTokens];
     load_tokens(tok, s0, n, v);
     __syncthreads();
-    each_read(off, 0, n_reads, [&](uint64_t a, uint64_t b) {
+    each_read(off, n_reads, [&](uint64_t a, uint64_t b) {
       a -= base;
       b -= base;
       if (a == b && a - s0 < kTile) atomicAdd(&extra[a - s0], 1u);
@@ -633,16 +644,16 @@ __global__ void __launch_bounds__(kTileThreads)
 
 // ---- big tiles: any number of empty reads, tokens of any length ---------------
 // extra[i * kTile + s]: the empty reads before slot s of big tile i (zeroed by
-// big_fill_kernel).  One thread per read; big_of[t]: tile t's i.
-__global__ void big_empties_kernel(const uint64_t *off, uint64_t n_reads, const uint32_t *big_of,
+// big_fill_kernel).  One thread per read; empty: tile_bytes_kernel's.
+__global__ void big_empties_kernel(const uint64_t *off, uint64_t n_reads, const uint32_t *empty,
                                    uint32_t *extra) {
   const uint64_t step = (uint64_t)gridDim.x * blockDim.x, base = off[0];
   for (uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; r < n_reads; r += step) {
     if (off[r + 1] != off[r]) continue;
     const uint32_t share = empty_share(off, n_reads, r);
     const uint64_t a = off[r] - base;
-    const uint32_t i = share ? __ldg(big_of + a / kTile) : kNotBig;
-    if (i != kNotBig) atomicAdd(extra + (uint64_t)i * kTile + a % kTile, share);
+    const uint32_t i = share ? __ldg(empty + a / kTile) : 0;
+    if (i & kBig) atomicAdd(extra + (uint64_t)(i & ~kBig) * kTile + a % kTile, share);
   }
 }
 
@@ -817,7 +828,7 @@ bool format_small(const V *tok, const uint64_t *off, u64 n_reads, uint8_t *out, 
 // and no tiles.
 template <class V>
 void format_big(const V *tok, u64 n, const uint64_t *off, u64 n_reads, bool empties,
-                const uint32_t *big, u64 n_big, const uint32_t *big_of, const uint32_t *ends,
+                const uint32_t *big, u64 n_big, const uint32_t *empty, const uint32_t *ends,
                 const uint64_t *tile_off, uint8_t *out, FormatWorkspace &ws, cudaStream_t st) {
   uint32_t *extra = nullptr;
   if (empties) {
@@ -826,7 +837,7 @@ void format_big(const V *tok, u64 n, const uint64_t *off, u64 n_reads, bool empt
     big_fill_kernel<<<dim3(32, (unsigned)std::min<u64>(n_big, 148 * 4)), 256, 0, st>>>(
         big, n_big, tile_off, out, extra);
     big_empties_kernel<<<(unsigned)std::min<u64>(n_reads / 256 + 1, 148 * 16), 256, 0, st>>>(
-        off, n_reads, big_of, extra);
+        off, n_reads, empty, extra);
   }
   big_tokens_kernel<V><<<(unsigned)std::min<u64>(n_big, 148 * 16), kTileThreads, 0, st>>>(
       tok, n, big, n_big, extra, ends, tile_off, out);
@@ -877,18 +888,20 @@ u64 format_tokens(const V *tok, u64 max_n, const uint64_t *off, u64 n_reads, uin
 }
 
 // The ascii of the tokens tok[off[0], off[n_reads]).  Their count is only known
-// on the device: a small capacity is one launch and a medium one bounds the
-// count (two bytes a token) for the tiles.  From kBoundBytes on the count is
-// read back first (a wait of ~10 us, against tiles and end bits for many times
-// the tokens), by the small output's launch unless there are too many reads for
-// it (100 reads of 2 color ids into 16 MB: 72 us by the bound, 41 us so).
-constexpr u64 kBoundBytes = 4ULL << 20;
+// on the device: a small capacity is one launch, a medium one bounds the count
+// (two bytes a token) for the tiles, and from `most` on the count is read back
+// first (a wait of ~10 us, against tiles and end bits for many times the tokens).
+// A few reads may well fill little of their room, so there `most` is smaller,
+// and the launch for small outputs brings the count back (100 reads of 2 color
+// ids into 16 / 64 MB: 75 / 87 us by the bound, 41 us so).
 template <class V>
 u64 format_ascii(const V *tok, const uint64_t *off, u64 n_reads, uint8_t *out, u64 out_cap,
                  u64 *need, FormatWorkspace &ws, cudaStream_t st) {
   u64 total = 0, max_n = out_cap / 2;
-  const bool bound = out_cap > 0 && out_cap <= kBoundBytes;
-  if (n_reads <= kSmallReads && (!bound || out_cap <= kSmallBytes)) {
+  const bool few = n_reads <= kSmallReads;
+  const u64 most = few ? 4ULL << 20 : 64ULL << 20;
+  const bool bound = out_cap > 0 && out_cap <= most;
+  if (few && (!bound || out_cap <= kSmallBytes)) {
     if (format_small(tok, off, n_reads, out, out_cap, need ? need : &total, ws, st))
       return ws.host[0];
     max_n = ws.host[2];
