@@ -411,8 +411,9 @@ int sbwt_set_probe_length(uint32_t probe_len);
  *       stream steps, all loads of a lane independent);
  *   7 = automatic, the default: the paths kernel (one table lookup per run
  *       of consecutive k-mers, the rest of the run read along a cover of the
- *       graph's edges by paths) on an index with its path cover; without one
- *       11 when the table and filter take at most 256 MiB, else 17;
+ *       graph's edges by paths) on an index with its path cover, from 4^k =
+ *       128 times its k-mers on (8 times when the table and filter take more
+ *       than 256 MiB); else 11 when these take at most 256 MiB, else 17;
  *   8, 9 = the walks kernel without the filter and the staged stores, 1 or 2
  *       walks per lane; 10 = the same with 1 walk and the filter in front of
  *       the table, one k-mer at a time; 11, 12 = the k-mers kernel with 2 or

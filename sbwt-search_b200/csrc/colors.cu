@@ -219,10 +219,10 @@ __device__ __forceinline__ uint64_t counter_bytes(const uint64_t (&p)[P], int q)
 // MODE 0: passing color words + count per read; MODE 1: full counts.  P: the
 // counter planes; a read of 2^P or more k-mers sets kErrLong and is left out.
 //
-// What bounds it: instructions, ~1,500 per read of 120 k-mers with 2000
-// colors, and the rows (11 KB a read) from L2.  Planes in shared memory with
-// one ripple per row took ~7,200 instructions (8.3 ms for 1 M reads of the
-// 2000-strain workload; see the figures at launch_colors).
+// What bounds it: instructions, 2,325 warp instructions per read of 120 k-mers
+// with 2000 colors (ALU pipe 74 %), beside the rows (11 KB a read, 8.5 KB of them
+// from DRAM).  Planes in shared memory with one ripple per row took 7,324 (8.3 ms
+// for 1 M reads; now 3.2 ms, see ColorsImpl::launch).
 template <int MODE, bool DIRECT, int P>
 __global__ void __launch_bounds__(32 * kColorWarps, P <= 8 ? 8 : (P <= 16 ? 6 : 3))
     colors_kernel(ColorsView cv, ColorsJob job, uint32_t *err) {

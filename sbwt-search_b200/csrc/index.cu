@@ -581,8 +581,8 @@ struct ReadsView {
   const uint64_t *n_kmers_dev;  // if set, the k-mer total is read from here
   unsigned long long *queue;    // work-queue counter (tiles handed out), zeroed
   uint64_t n_kmers_bound;       // > every chunk position, slot and read number
-  uint32_t *out32;  // walks kernel only: 32-bit results here instead of `out`
-                    // (node, 0xFFFFFFFF not found, 0xFFFFFFFE invalid)
+  uint32_t *out32;  // if set, 32-bit results here instead of `out` (node, 0xFFFFFFFF not
+                    // found, 0xFFFFFFFE invalid); see walks_kernel_applies
 };
 
 __device__ __forceinline__ bool invalid_at(const uint32_t *inv, uint64_t i) {
@@ -2428,7 +2428,7 @@ static void launch_one_wave(void (*kernel)(KArgs...), int grid, int threads, cud
 // kernel_mode: 0 = the general kernel; 1 = the table kernel; 2..5 = the
 // walks kernel with (walks per lane, blocks per SM) = (1, 5), (2, 4), (2, 3),
 // (4, 2) (the table kernel when the index has no k-mer filter); 6 = the
-// k-mers kernel; 7 = 11 when the table and filter are small, else 17; 8, 9 =
+// k-mers kernel; 7 = search_paths_kernel, 11 or 17 (resolve_kernel_mode); 8, 9 =
 // the walks kernel without filter and staging, 1 or 2 walks per lane; 10 =
 // the same with the filter in front of the table, one k-mer at a time; 11,
 // 12 = the k-mers kernel with 2 or 8 k-mers per lane (6: 4); 13, 14 = the
@@ -2437,8 +2437,8 @@ static void launch_one_wave(void (*kernel)(KArgs...), int grid, int threads, cud
 // 16, 17 = 13 staging 8 or 16 slots per store group; 18 = 14 staging 16;
 // 19 = 6 without the filter.
 // Results never depend on it.
-// Whether launch_search_kernel runs the walks kernel (the only one that can
-// write 32-bit results, ReadsView::out32).
+// Whether launch_search_kernel runs the walks, k-mers or paths kernel (those that
+// can write 32-bit results, ReadsView::out32).
 static bool walks_kernel_applies(const SbwtView &sv, const ReadsView &rv, bool stream,
                                  uint32_t mtk, uint32_t kernel_mode) {
   const bool narrow = sv.num_bits < kNarrowLimit && rv.n_kmers_bound < (1ULL << 32);
@@ -3320,7 +3320,7 @@ static ReadsScratch scratch_for(Workspace &ws, int b, u64 n_chars, u64 n_reads,
   ws.packed[b].ensure((n_words + 2) * 16);  // words, or interleaved entries
   ws.invalid[b].ensure((n_words + 2) * 4);
   ws.block_sums[b].ensure(((n_reads + kScanTile - 1) / kScanTile + 1) * 8);
-  ws.total[b].ensure(8);
+  if (b) ws.total[b].ensure(8);  // slot 0's lies beside the error word
   ws.tile_read[b].ensure((n_kmers_max / tile_min + 2) * 8);
   ws.queue[b].ensure(8);
   return ReadsScratch{ws.kmer_off[b].get<u64>(), ws.packed[b].get<u64>(),

@@ -23,8 +23,8 @@ constexpr u64 kFilterBitsPerKmer = 10;
 constexpr u64 kLmerFilterBits = 8;
 
 // Read search kernel of an index with a k-mer table by default
-// (LaunchConfig::table_kernel): automatic (the k-mers kernel for small
-// tables, else the table kernel).
+// (LaunchConfig::table_kernel): automatic (the paths kernel where its runs are
+// long, else the k-mers kernel for small tables or the walks kernel).
 constexpr uint32_t kDefaultTableKernel = 7;
 
 struct LaunchConfig {
@@ -37,7 +37,7 @@ struct LaunchConfig {
   uint32_t probe_len = 0;          // absent-prefix probe length (0 = auto, ~0u = off)
   uint32_t l2_window = 0;          // persisting L2 window over the index's hot data
   uint32_t table_kernel = kDefaultTableKernel;  // read search kernel with a k-mer table
-                                               // (0 general, 1 table, 2-4 walks)
+                                               // (modes: launch_search_kernel)
 };
 
 struct IndexImpl {
