@@ -76,6 +76,7 @@ def lib():
         L.sbwt_count_kmers.restype = u64
         L.sbwt_search_reads.argtypes = [vp, vp, u64, vp, u64, vp, u64,
                                         C.POINTER(u64), u32, vp]
+        L.sbwt_search_reads_noalloc.argtypes = L.sbwt_search_reads.argtypes
         L.sbwt_set_launch_config.argtypes = [u32, u32, u64, u64]
         L.sbwt_set_probe_length.argtypes = [u32]
         L.sbwt_set_l2_window.argtypes = [C.c_int]

@@ -1,5 +1,7 @@
 """Read search over the path cover (the automatic kernel of an index with its
 k-mer table): equal to the oracle on the graphs and reads where runs end."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -153,6 +155,19 @@ def test_reads_of_every_k(k):
         assert np.array_equal(got[:len(exp)].view(np.uint64), exp)
         assert (got[len(exp):] == -7).all()
         assert np.array_equal(idx.search_reads(chars, ends), exp)
+        n = C.c_uint64()
+        out.fill_(-7)
+        S.check(S.lib().sbwt_search_reads_noalloc(
+            idx._h, d_chars.data_ptr(), d_chars.numel(), d_ends.data_ptr(), d_ends.numel(),
+            out.data_ptr(), out.numel(), C.byref(n), 0, None))
+        got = out.cpu().numpy()
+        assert n.value == len(exp) and np.array_equal(got[:len(exp)].view(np.uint64), exp)
+        assert (got[len(exp):] == -7).all()
+        pipe = S.Pipeline(idx, None, len(chars), len(ends))
+        for m in (600, 3, 600):
+            last = int(ends[m - 1])
+            assert np.array_equal(pipe.run(chars[:last], ends[:m]), exp[:idx.count_kmers(ends[:m])])
+        pipe.close()
 
 
 @pytest.mark.parametrize("k", [12, 13, 14, 15])
