@@ -220,24 +220,20 @@ __global__ void __launch_bounds__(kScanThreads) scan_apply_kernel(uint64_t *v, u
 
 // ---- ascii in tiles of tokens ------------------------------------------------
 constexpr uint32_t kTileThreads = 256, kTokens = 8, kTile = kTileThreads * kTokens;
-// Bytes of a tile that shared memory holds (16 per token).  A tile with more
-// (tokens of 16 and more digits), or with thousands of empty reads, which one
-// block would count one after the other, is a big one: it is filled with '\n' by
-// many blocks, and its tokens go straight to their places.
+// Bytes of a tile that shared memory holds (16 per token).  A tile with more (tens
+// of thousands of empty reads, or tokens of 16 and more digits) is a big one: it is
+// filled with '\n' by many blocks, and its tokens go straight to their places.
 constexpr uint32_t kTileBytes = 16 * kTile;
-// Empty reads from which on a tile is a big one.  1 M reads of which one in 20
-// has 2 ids (19,000 of them a tile): 94 us here, 112 us at 16384.
-constexpr uint32_t kBigEmpty = 24576;
 
-// What read r, one of the empty reads between the tokens a - 1 and a, adds to a
-// count of them, mod 2^32: the last one its end, the first one its start taken
-// away, so that thousands of empty reads in a row are two additions.
-__device__ __forceinline__ uint32_t empty_share(const uint64_t *off, uint64_t n_reads, uint64_t r) {
-  const uint64_t a = off[r];
-  uint32_t share = 0;
-  if (r + 1 == n_reads || off[r + 2] != a) share += (uint32_t)r + 1;
-  if (r == 0 || off[r - 1] != a) share -= (uint32_t)r;
-  return share;
+// What read r adds to a count of the empty reads in front of a token, mod 2^32: the
+// last one of a stretch its end, the first one its start taken away, so that
+// thousands of empty reads in a row are two additions.  before, a, b, after:
+// off[r - 1] to off[r + 2], where they exist (all loaded at once).
+__device__ __forceinline__ uint32_t empty_share(uint64_t r, uint64_t n_reads, uint64_t before,
+                                                uint64_t a, uint64_t b, uint64_t after) {
+  if (a != b) return 0;
+  return (r + 1 == n_reads || after != a ? (uint32_t)r + 1 : 0u) -
+         (r == 0 || before != a ? (uint32_t)r : 0u);
 }
 
 // One thread per read: first_read[t] = the first read r with off[r] - off[0]
@@ -263,11 +259,13 @@ __global__ void tile_lines_kernel(const uint64_t *off, uint64_t n_reads, uint64_
     uint64_t a = 0;
     uint32_t share = 0;
     if (r <= n_reads) {
-      a = min(off[r] - base, n);
-      const uint64_t before = r ? min(off[r - 1] - base, n) : 0;
+      const uint64_t o_before = r ? off[r - 1] : base, o = off[r];
+      const uint64_t o_end = off[min(r + 1, n_reads)], o_after = off[min(r + 2, n_reads)];
+      a = min(o - base, n);
+      const uint64_t before = min(o_before - base, n);
       for (uint64_t t = r ? before / kTile + 1 : 0; t <= a / kTile; ++t) first_read[t] = r;
       if (r && a > before) atomicOr(ends + (a - 1) / 32, 1u << ((a - 1) & 31));
-      if (r < n_reads && off[r + 1] == off[r]) share = empty_share(off, n_reads, r);
+      if (r < n_reads) share = empty_share(r, n_reads, o_before, o, o_end, o_after);
     }
     const unsigned m = __ballot_sync(FULL, share != 0);
     if (!m) continue;
@@ -349,7 +347,7 @@ __global__ void __launch_bounds__(kTileThreads) tile_bytes_kernel(const V *tok, 
     for (uint32_t w = 0; w < kTileThreads / 32; ++w) t += sums[threadIdx.x][w];
     bytes[tile] = t;
     if (e) atomicOr((unsigned long long *)flags, 1ULL);
-    if (t > kTileBytes || e >= kBigEmpty) {
+    if (t > kTileBytes) {
       const uint32_t at = (uint32_t)(atomicAdd((unsigned long long *)flags, 2ULL) >> 1);
       big[at] = (uint32_t)tile;
       empty[tile] = kBig | at;
@@ -385,31 +383,28 @@ __device__ __forceinline__ void put_bytes(uint32_t *buf, uint32_t o, uint64_t w)
   if (u2) atomicOr(buf + (o >> 2) + 2, u2);
 }
 
-// e '\n' from o on in the zeroed buf.  A few by their thread; where a thread of
-// the warp has more (many: the same for all its lanes, which all call it), those
-// by the whole warp: whole words by plain stores, as no other token or line
-// reaches into them.
+// The stretches of more than kFewLines '\n' (e from o on, in the zeroed buf) of a
+// warp's threads, by the whole warp: whole words by plain stores, as no other
+// token or line reaches into them.  (Kept out of write_tile's token loop, which
+// it made 7 % longer for tiles with short stretches alone.)
 constexpr uint32_t kFewLines = 64;
-__device__ __forceinline__ void put_newlines(uint32_t *buf, uint32_t o, uint32_t e, bool many) {
+__device__ __forceinline__ void put_newlines(uint32_t *buf, uint32_t o, uint32_t e) {
   constexpr uint32_t kLines = 0x0A0A0A0Au;
-  if (many) {
-    for (unsigned m = __ballot_sync(FULL, e > kFewLines); m; m &= m - 1) {
-      const uint32_t a = __shfl_sync(FULL, o, __ffs(m) - 1);
-      const uint32_t b = a + __shfl_sync(FULL, e, __ffs(m) - 1), lane = threadIdx.x & 31;
-      for (uint32_t w = (a + 3) / 4 + lane; w < b / 4; w += 32) buf[w] = kLines;
-      if (lane == 0 && (a & 3)) atomicOr(buf + a / 4, kLines << (8 * (a & 3)));
-      if (lane == 1 && (b & 3)) atomicOr(buf + b / 4, kLines >> (8 * (4 - (b & 3))));
-    }
-    if (e > kFewLines) return;
+  const uint32_t lane = threadIdx.x & 31;
+  for (unsigned m = __ballot_sync(FULL, e > kFewLines); m; m &= m - 1) {
+    const uint32_t a = __shfl_sync(FULL, o, __ffs(m) - 1);
+    const uint32_t b = a + __shfl_sync(FULL, e, __ffs(m) - 1);
+    for (uint32_t w = (a + 3) / 4 + lane; w < b / 4; w += 32) buf[w] = kLines;
+    if (lane == 0 && (a & 3)) atomicOr(buf + a / 4, kLines << (8 * (a & 3)));
+    if (lane == 1 && (b & 3)) atomicOr(buf + b / 4, kLines >> (8 * (4 - (b & 3))));
   }
-  for (; e; --e, ++o) atomicOr(buf + (o >> 2), (uint32_t)'\n' << (8 * (o & 3)));
 }
 
-// f(off[r], off[r + 1]) of all reads by the whole block, eight reads' loads in
+// f(off[r], off[r + 1]) of all reads by the whole block, four reads' loads in
 // flight per thread.
 template <class F>
 __device__ __forceinline__ void each_read(const uint64_t *off, uint64_t n_reads, F f) {
-  constexpr uint32_t U = 8;
+  constexpr uint32_t U = 4;
   for (uint64_t r = threadIdx.x; r < n_reads; r += U * kTileThreads) {
     uint64_t a[U], b[U];
 #pragma unroll
@@ -485,12 +480,25 @@ __device__ __forceinline__ void write_tile(TileShared &sh, const V (&v)[kTokens]
   uint32_t o = shift + x - mine;
 #pragma unroll
   for (uint32_t w = 0; w < kTileThreads / 32; ++w) o += w < wid ? sh.sums[w] : 0;
+  if (EXTRAS && many) {
+    uint32_t at = o;
+#pragma unroll
+    for (uint32_t q = 0; q < kTokens; ++q) {
+      const uint32_t e = extra[kTokens * tid + q];
+      put_newlines(buf, at, e);
+      at += e + len[q];
+    }
+  }
+  const uint32_t alone = many ? kFewLines : ~0u;
 #pragma unroll
   for (uint32_t q = 0; q < kTokens; ++q) {
     if (EXTRAS) {
-      const uint32_t e = extra[kTokens * tid + q];
-      put_newlines(buf, o, e, many);
-      o += e;
+      uint32_t e = extra[kTokens * tid + q];
+      if (e > alone) {
+        o += e;
+        e = 0;
+      }
+      for (; e; --e, ++o) atomicOr(buf + (o >> 2), (uint32_t)'\n' << (8 * (o & 3)));
     }
     if (!len[q]) continue;
     const uint32_t term = (bits >> q) & 1u ? '\n' : ' ', end = o + len[q];
@@ -550,9 +558,9 @@ __device__ __forceinline__ void write_tile(TileShared &sh, const V (&v)[kTokens]
 template <class V, bool EXTRAS>
 __global__ void __launch_bounds__(kTileThreads, 5)
     tile_ascii_kernel(const V *tok, uint64_t n, const uint64_t *off, uint64_t n_reads,
-                      const uint64_t *first_read, const uint32_t *empty,
-                      const uint32_t *ends, const uint64_t *tile_off, uint8_t *out,
-                      const uint64_t *status, uint64_t out_cap) {
+                      const uint64_t *first_read, const uint32_t *ends,
+                      const uint64_t *tile_off, uint8_t *out, const uint64_t *status,
+                      uint64_t out_cap) {
   __shared__ TileShared sh;
   __shared__ uint32_t extra[EXTRAS ? kTile : 1];
   if (status) {
@@ -566,9 +574,7 @@ __global__ void __launch_bounds__(kTileThreads, 5)
   const uint64_t i0 = s0 + kTokens * threadIdx.x;
   const uint32_t bits = i0 < n ? __ldg(ends + i0 / 32) >> (i0 & 31) : 0;
   const uint64_t b0 = __ldg(tile_off + blockIdx.x), b1 = __ldg(tile_off + blockIdx.x + 1);
-  if (b1 == b0) return;  // past the end
-  // a big tile (without empty reads only by its bytes)
-  if (EXTRAS ? __ldg(empty + blockIdx.x) >= kBig : b1 - b0 > kTileBytes) return;
+  if (b1 == b0 || b1 - b0 > kTileBytes) return;  // past the end; a big tile
   if (threadIdx.x < 32) sh.table[threadIdx.x] = kDecLen.entry[threadIdx.x];
   if (EXTRAS) count_extras(off, n_reads, n, first_read, blockIdx.x, extra);
   write_tile<V, EXTRAS>(sh, v, (uint32_t)min(n - s0, (uint64_t)kTile), bits, extra,
@@ -649,9 +655,9 @@ __global__ void big_empties_kernel(const uint64_t *off, uint64_t n_reads, const 
                                    uint32_t *extra) {
   const uint64_t step = (uint64_t)gridDim.x * blockDim.x, base = off[0];
   for (uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; r < n_reads; r += step) {
-    if (off[r + 1] != off[r]) continue;
-    const uint32_t share = empty_share(off, n_reads, r);
-    const uint64_t a = off[r] - base;
+    const uint64_t o = off[r], a = o - base;
+    const uint32_t share = empty_share(r, n_reads, r ? off[r - 1] : o, o, off[r + 1],
+                                       off[min(r + 2, n_reads)]);
     const uint32_t i = share ? __ldg(empty + a / kTile) : 0;
     if (i & kBig) atomicAdd(extra + (uint64_t)(i & ~kBig) * kTile + a % kTile, share);
   }
@@ -868,7 +874,7 @@ u64 format_tokens(const V *tok, u64 max_n, const uint64_t *off, u64 n_reads, uin
   const bool few = tiles <= kFewTiles;  // written before the host knows the count
   if (few)
     tile_ascii_kernel<V, true><<<(unsigned)tiles, kTileThreads, 0, st>>>(
-        tok, max_n, off, n_reads, first, empty, ends, bytes, out, status, out_cap);
+        tok, max_n, off, n_reads, first, ends, bytes, out, status, out_cap);
   const u64 total = scan_inplace(bytes, tiles, ws, st, 4, few);
   const u64 flags = ws.host[1], n = ws.host[2], base = ws.host[3];
   if (n > max_n) return format_tokens(tok, n, off, n_reads, out, out_cap, need, ws, st);
@@ -878,8 +884,8 @@ u64 format_tokens(const V *tok, u64 max_n, const uint64_t *off, u64 n_reads, uin
   tiles = n / kTile + 1;
   if (!few) {
     auto *const kernel = flags & 1 ? tile_ascii_kernel<V, true> : tile_ascii_kernel<V, false>;
-    kernel<<<(unsigned)tiles, kTileThreads, 0, st>>>(tok, n, off, n_reads, first, empty, ends,
-                                                     bytes, out, nullptr, 0);
+    kernel<<<(unsigned)tiles, kTileThreads, 0, st>>>(tok, n, off, n_reads, first, ends, bytes,
+                                                     out, nullptr, 0);
   }
   SBWT_CUDA(cudaGetLastError());
   if (flags >> 1)
